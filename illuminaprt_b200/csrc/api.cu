@@ -58,7 +58,7 @@ int ensure_raw_tris(ilg_ctx *ctx)
     if (ctx->raw_ready) return ILG_OK;
     const uint32_t n = ctx->stats.n_tris;
     CK(ctx->raw_tris.reserve(3ull * n));
-    CK(build_raw_tris(ctx->bb.prim_of, ctx->idx.ptr, ctx->pos.ptr, n, ctx->raw_tris.ptr, ctx->stream));
+    CK(build_raw_tris(ctx->bb.tris, ctx->idx.ptr, ctx->pos.ptr, n, ctx->raw_tris.ptr, ctx->stream));
     ctx->raw_ready = true;
     return ILG_OK;
 }
@@ -495,8 +495,8 @@ int ilg_save(ilg_ctx *ctx, const char *path)
     h.n_leaf_tris = ctx->stats.n_leaf_tris;
     h.max_depth = ctx->stats.max_depth;
     h.has_mat = ctx->has_mat ? 1u : 0u;
-    h.node_bytes = sizeof(Node8);
-    h.tri_bytes = sizeof(Tri);
+    h.node_bytes = sizeof(FileNode8);
+    h.tri_bytes = sizeof(FileTri);
     std::vector<float> pos(3ull * h.n_verts);
     std::vector<uint32_t> idx(3ull * h.n_tris), mat(h.has_mat ? h.n_tris : 0), prim(h.n_leaf_tris);
     std::vector<Node8> nodes(h.n_nodes);
@@ -506,11 +506,17 @@ int ilg_save(ilg_ctx *ctx, const char *path)
     if (h.has_mat) CK(cudaMemcpyAsync(mat.data(), ctx->mat.ptr, 4ull * h.n_tris, cudaMemcpyDeviceToHost, st));
     CK(cudaMemcpyAsync(nodes.data(), ctx->bb.nodes, sizeof(Node8) * h.n_nodes, cudaMemcpyDeviceToHost, st));
     CK(cudaMemcpyAsync(tris.data(), ctx->bb.tris, sizeof(Tri) * h.n_leaf_tris, cudaMemcpyDeviceToHost, st));
-    CK(cudaMemcpyAsync(prim.data(), ctx->bb.prim_of, 4ull * h.n_leaf_tris, cudaMemcpyDeviceToHost, st));
     CK(cudaStreamSynchronize(st));
+    std::vector<FileNode8> fnodes(h.n_nodes);
+    for (uint32_t i = 0; i < h.n_nodes; i++) fnodes[i] = to_file(nodes[i]);
+    std::vector<FileTri> ftris(h.n_leaf_tris);
+    for (uint32_t i = 0; i < h.n_leaf_tris; i++) {
+        ftris[i] = FileTri{tris[i].a, tris[i].b, tris[i].c};
+        prim[i] = tris[i].id.x;
+    }
     const std::pair<const void *, size_t> parts[6] = {
         {pos.data(), 12ull * h.n_verts}, {idx.data(), 12ull * h.n_tris}, {mat.data(), 4ull * mat.size()},
-        {nodes.data(), sizeof(Node8) * nodes.size()}, {tris.data(), sizeof(Tri) * tris.size()},
+        {fnodes.data(), sizeof(FileNode8) * fnodes.size()}, {ftris.data(), sizeof(FileTri) * ftris.size()},
         {prim.data(), 4ull * prim.size()}};
     uint64_t sum = 0xCBF29CE484222325ull;
     for (auto &q : parts) {
@@ -541,21 +547,21 @@ int ilg_load(ilg_ctx *ctx, const char *path)
     if (fread(&h, sizeof(h), 1, f) != 1) return bad("short header");
     if (memcmp(h.magic, "ILGBVH8", 8) != 0) return bad("not a scene file");
     if (h.version != kSceneFileVersion || h.header_bytes != sizeof(h)) return bad("unsupported version");
-    if (h.node_bytes != sizeof(Node8) || h.tri_bytes != sizeof(Tri)) return bad("record sizes differ");
+    if (h.node_bytes != sizeof(FileNode8) || h.tri_bytes != sizeof(FileTri)) return bad("record sizes differ");
     if (h.n_verts == 0 || h.n_tris == 0 || h.n_tris > (1u << 30) || h.n_leaf_tris != h.n_tris || h.n_nodes == 0 ||
         h.n_nodes > h.n_tris + 1u || h.has_mat > 1u)
         return bad("inconsistent counts");
     const uint64_t expect = 12ull * h.n_verts + 12ull * h.n_tris + (h.has_mat ? 4ull * h.n_tris : 0ull) +
-                            sizeof(Node8) * (uint64_t)h.n_nodes + sizeof(Tri) * (uint64_t)h.n_leaf_tris +
+                            sizeof(FileNode8) * (uint64_t)h.n_nodes + sizeof(FileTri) * (uint64_t)h.n_leaf_tris +
                             4ull * h.n_leaf_tris;
     if (h.payload_bytes != expect) return bad("payload size differs from the counts");
     std::vector<float> pos(3ull * h.n_verts);
     std::vector<uint32_t> idx(3ull * h.n_tris), mat(h.has_mat ? h.n_tris : 0), prim(h.n_leaf_tris);
-    std::vector<Node8> nodes(h.n_nodes);
-    std::vector<Tri> tris(h.n_leaf_tris);
+    std::vector<FileNode8> fnodes(h.n_nodes);
+    std::vector<FileTri> ftris(h.n_leaf_tris);
     const std::pair<void *, size_t> parts[6] = {
         {pos.data(), 12ull * h.n_verts}, {idx.data(), 12ull * h.n_tris}, {mat.data(), 4ull * mat.size()},
-        {nodes.data(), sizeof(Node8) * nodes.size()}, {tris.data(), sizeof(Tri) * tris.size()},
+        {fnodes.data(), sizeof(FileNode8) * fnodes.size()}, {ftris.data(), sizeof(FileTri) * ftris.size()},
         {prim.data(), 4ull * prim.size()}};
     uint64_t sum = 0xCBF29CE484222325ull, stored = 0;
     for (auto &q : parts) {
@@ -565,6 +571,9 @@ int ilg_load(ilg_ctx *ctx, const char *path)
     if (fread(&stored, sizeof(stored), 1, f) != 1) return bad("truncated checksum");
     fclose(f);
     if (stored != sum) return fail(ctx, ILG_EINVAL, "ilg_load: %s: checksum mismatch", path);
+    std::vector<Node8> nodes(h.n_nodes);
+    for (uint32_t i = 0; i < h.n_nodes; i++)
+        if (!from_file(fnodes[i], nodes[i])) return fail(ctx, ILG_EINVAL, "ilg_load: %s: bad node record", path);
     // record -> triangle map: a permutation of the triangles (the renderer indexes with it)
     {
         std::vector<unsigned char> seen(h.n_tris, 0);
@@ -573,19 +582,19 @@ int ilg_load(ilg_ctx *ctx, const char *path)
             seen[p] = 1;
         }
     }
+    std::vector<Tri> tris(h.n_leaf_tris);
+    for (uint32_t i = 0; i < h.n_leaf_tris; i++)
+        tris[i] = Tri{ftris[i].a, ftris[i].b, ftris[i].c, uint4{prim[i], 0u, 0u, 0u}};
     int rc = ilg_set_mesh(ctx, pos.data(), h.n_verts, idx.data(), h.n_tris, h.has_mat ? mat.data() : nullptr);
     if (rc) return rc;
     CK(cudaSetDevice(ctx->device));
     cudaStream_t st = ctx->stream;
     CK(ctx->bb.nodes_b.reserve(h.n_nodes));
     CK(ctx->bb.tris_b.reserve(h.n_leaf_tris));
-    CK(ctx->bb.prim_of_b.reserve(h.n_leaf_tris));
     ctx->bb.nodes = ctx->bb.nodes_b.ptr;
     ctx->bb.tris = ctx->bb.tris_b.ptr;
-    ctx->bb.prim_of = ctx->bb.prim_of_b.ptr;
     CK(cudaMemcpyAsync(ctx->bb.nodes, nodes.data(), sizeof(Node8) * h.n_nodes, cudaMemcpyHostToDevice, st));
     CK(cudaMemcpyAsync(ctx->bb.tris, tris.data(), sizeof(Tri) * h.n_leaf_tris, cudaMemcpyHostToDevice, st));
-    CK(cudaMemcpyAsync(ctx->bb.prim_of, prim.data(), 4ull * h.n_leaf_tris, cudaMemcpyHostToDevice, st));
     CK(cudaStreamSynchronize(st));
     ctx->stats.n_tris = h.n_tris;
     ctx->stats.n_nodes = h.n_nodes;
@@ -946,15 +955,14 @@ static int prepare_scene(ilg_ctx *runner, ilg_ctx *ctx, const ilg_camera_frame &
         return fail(runner, ILG_ESTATE, "ilg_render: mesh lights were set for an earlier mesh (call ilg_set_lights again)");
     const uint32_t n = ctx->n_tris;
     if (ctx->attr_dirty) {
-        CK2(runner, ctx->tri_attr.reserve(n));
         CK2(runner, ctx->light_of_prim.reserve(n));
-        CK2(runner, build_tri_attr(ctx->bb.prim_of, n, ctx->mat.ptr, ctx->light_range.ptr, ctx->n_lights,
-                                   ctx->light_of_prim.ptr, ctx->tri_attr.ptr, st));
+        CK2(runner, build_tri_attr(ctx->bb.tris, n, ctx->mat.ptr, ctx->light_range.ptr, ctx->n_lights,
+                                   ctx->light_of_prim.ptr, st));
         ctx->attr_dirty = false;
     }
     S = SceneRec{};
     S.nodes = ctx->bb.nodes; S.tris = ctx->bb.tris; S.n_nodes = ctx->stats.n_nodes; S.n_tris = ctx->stats.n_tris;
-    S.tri_attr = ctx->tri_attr.ptr; S.mats = ctx->mats.ptr; S.n_mats = ctx->n_mats;
+    S.mats = ctx->mats.ptr; S.n_mats = ctx->n_mats;
     S.lights = ctx->lights.ptr; S.n_lights = ctx->n_lights;
     S.sky = make_float3(sky[0], sky[1], sky[2]);
     S.inf_escape = ctx->inf_escape;

@@ -600,7 +600,7 @@ __global__ void k_collapse(const Work *__restrict__ in, const uint32_t *__restri
                            const float4 *__restrict__ tlo, const float4 *__restrict__ thi,
                            const float *__restrict__ pos, const uint32_t *__restrict__ idx, Node8 *__restrict__ nodes,
                            uint32_t *__restrict__ node_count, uint32_t node_cap, Tri *__restrict__ tris,
-                           uint32_t *__restrict__ prim_of, uint32_t *__restrict__ tri_count, uint32_t tri_cap,
+                           uint32_t *__restrict__ tri_count, uint32_t tri_cap,
                            float min_step, uint32_t *__restrict__ err)
 {
     uint32_t w = blockIdx.x * blockDim.x + threadIdx.x;
@@ -697,8 +697,9 @@ __global__ void k_collapse(const Work *__restrict__ in, const uint32_t *__restri
     // origin one step below the union so that floor() never goes negative
     float3 org = make_float3(plo.x - sx, plo.y - sy, plo.z - sz);
 
-    uint8_t meta[8], qlx[8], qly[8], qlz[8], qhx[8], qhy[8], qhz[8];
-    for (int s = 0; s < 8; s++) meta[s] = qlx[s] = qly[s] = qlz[s] = qhx[s] = qhy[s] = qhz[s] = 0;
+    uint8_t qlx[8], qly[8], qlz[8], qhx[8], qhy[8], qhz[8];
+    for (int s = 0; s < 8; s++) qlx[s] = qly[s] = qlz[s] = qhx[s] = qhy[s] = qhz[s] = 0;
+    uint32_t slots = 0;
 
     // internal children in slot order -> contiguous child nodes
     uint32_t imask = 0;
@@ -723,7 +724,7 @@ __global__ void k_collapse(const Work *__restrict__ in, const uint32_t *__restri
         qhy[s] = (uint8_t)fmin(fmax(hy, 0.0), 255.0);
         qhz[s] = (uint8_t)fmin(fmax(hz, 0.0), 255.0);
         if (imask & (1u << s)) {
-            meta[s] = (uint8_t)kMetaInternal;
+            slots |= 8u << (4 * s);
             uint32_t ci = child_base + __popc(imask & ((1u << s) - 1u));
             uint32_t slot = atomicAdd(out_count, 1u);
             if (slot >= out_cap) { atomicOr(err, 8u); continue; }
@@ -731,7 +732,7 @@ __global__ void k_collapse(const Work *__restrict__ in, const uint32_t *__restri
         } else {
             int pos_of[kLeafMax];
             const int nt = leaf_tris(ch[k], child, pos_of);
-            meta[s] = (uint8_t)((nt << 5) | tri_off);
+            slots |= ((1u << nt) - 1u) << (4 * s);
             for (int q = 0; q < nt; q++) {
                 uint32_t t = sorted_tri[pos_of[q]];
                 uint32_t a = idx[3 * t], b = idx[3 * t + 1], c = idx[3 * t + 2];
@@ -747,8 +748,8 @@ __global__ void k_collapse(const Work *__restrict__ in, const uint32_t *__restri
                 tr.a = make_float4(v0x, v0y, v0z, nx);
                 tr.b = make_float4(e1x, e1y, e1z, ny);
                 tr.c = make_float4(e2x, e2y, e2z, nz);
+                tr.id = make_uint4(t, 0u, 0u, 0u);
                 tris[tri_base + tri_off + q] = tr;
-                prim_of[tri_base + tri_off + q] = t;
             }
             tri_off += nt;
         }
@@ -758,13 +759,12 @@ __global__ void k_collapse(const Work *__restrict__ in, const uint32_t *__restri
         return (uint32_t)b[0] | ((uint32_t)b[1] << 8) | ((uint32_t)b[2] << 16) | ((uint32_t)b[3] << 24);
     };
     Node8 nd;
-    nd.q[0] = make_uint4(__float_as_uint(org.x), __float_as_uint(org.y), __float_as_uint(org.z),
-                         (uint32_t)(ex + 127) | ((uint32_t)(ey + 127) << 8) | ((uint32_t)(ez + 127) << 16) |
-                             (imask << 24));
-    nd.q[1] = make_uint4(child_base, tri_base, pack4(meta), pack4(meta + 4));
+    nd.q[0] = make_uint4(__float_as_uint(org.x), __float_as_uint(org.y), __float_as_uint(org.z), child_base);
+    nd.q[1] = make_uint4((uint32_t)(ex + 127) << 23, (uint32_t)(ey + 127) << 23, (uint32_t)(ez + 127) << 23, tri_base);
     nd.q[2] = make_uint4(pack4(qlx), pack4(qlx + 4), pack4(qhx), pack4(qhx + 4));
     nd.q[3] = make_uint4(pack4(qly), pack4(qly + 4), pack4(qhy), pack4(qhy + 4));
     nd.q[4] = make_uint4(pack4(qlz), pack4(qlz + 4), pack4(qhz), pack4(qhz + 4));
+    nd.q[5] = make_uint4(slots, 0u, 0u, 0u);
     nodes[job.node] = nd;
 }
 
@@ -850,7 +850,7 @@ int bvh_build(BuildBuffers &B, const float *d_pos, uint32_t n_verts, const uint3
         ILG_CK(cudaMemsetAsync(cout, 0, sizeof(uint32_t), st));
         k_collapse<<<div_up(host_in, 64), 64, 0, st>>>(qin, cin, qout, cout, queue_cap, B.child, B.cnt, B.dpd, B.nlo,
                                                         B.nhi, B.vals_alt, B.tlo, B.thi, d_pos, d_idx, B.nodes,
-                                                        B.counters + 0, node_cap, B.tris, B.prim_of, B.counters + 1,
+                                                        B.counters + 0, node_cap, B.tris, B.counters + 1,
                                                         tri_cap, min_step, B.err);
         ILG_CK(cudaGetLastError());
         ILG_CK(cudaMemcpyAsync(&host_in, cout, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));

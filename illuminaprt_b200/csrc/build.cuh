@@ -46,7 +46,6 @@ struct BuildBuffers {
     // outputs (the built scene)
     DevBuf<Node8> nodes_b;
     DevBuf<Tri> tris_b;
-    DevBuf<uint32_t> prim_of_b;
 
     float4 *tlo, *thi, *nlo, *nhi;
     uint32_t *keys, *keys_alt, *vals, *vals_alt, *arrivals, *cbounds, *counters, *err;
@@ -58,7 +57,6 @@ struct BuildBuffers {
     void *qa_raw, *qb_raw;  // two 8-byte work-item queues
     Node8 *nodes;
     Tri *tris;
-    uint32_t *prim_of;
 
     cudaError_t reserve(size_t n, size_t sort_bytes, size_t node_cap, size_t queue_cap, cudaStream_t)
     {
@@ -70,7 +68,7 @@ struct BuildBuffers {
         ILG_R(child_b, n) ILG_R(range_b, n) ILG_R(parent_int_b, n) ILG_R(parent_leaf_b, n) ILG_R(cnt_b, n)
         ILG_R(cost_b, n) ILG_R(dpc_b, 8 * n) ILG_R(dpd_b, 16 * n)
         ILG_R(sort_tmp_b, sort_bytes) ILG_R(qa_b, queue_cap) ILG_R(qb_b, queue_cap)
-        ILG_R(nodes_b, node_cap) ILG_R(tris_b, n) ILG_R(prim_of_b, n)
+        ILG_R(nodes_b, node_cap) ILG_R(tris_b, n)
 #undef ILG_R
         tlo = tlo_b.ptr; thi = thi_b.ptr; nlo = nlo_b.ptr; nhi = nhi_b.ptr;
         keys = keys_b.ptr; keys_alt = keys_alt_b.ptr; vals = vals_b.ptr; vals_alt = vals_alt_b.ptr;
@@ -78,7 +76,7 @@ struct BuildBuffers {
         child = child_b.ptr; range = range_b.ptr; parent_int = parent_int_b.ptr; parent_leaf = parent_leaf_b.ptr;
         cnt = cnt_b.ptr; cost = cost_b.ptr; dpc = dpc_b.ptr; dpd = dpd_b.ptr;
         sort_tmp = sort_tmp_b.ptr; qa_raw = qa_b.ptr; qb_raw = qb_b.ptr;
-        nodes = nodes_b.ptr; tris = tris_b.ptr; prim_of = prim_of_b.ptr;
+        nodes = nodes_b.ptr; tris = tris_b.ptr;
         return cudaSuccess;
     }
 
@@ -96,7 +94,7 @@ struct BuildBuffers {
     {
         release_scratch();
         cb_b.release(); counters_b.release(); err_b.release();
-        nodes_b.release(); tris_b.release(); prim_of_b.release();
+        nodes_b.release(); tris_b.release();
     }
 };
 

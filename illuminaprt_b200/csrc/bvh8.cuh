@@ -8,35 +8,66 @@
 namespace ilg {
 
 // ---------------------------------------------------------------------------
-// Node record: 80 bytes = 5 x uint4, 16-byte aligned, read with 128-bit loads.
-//   q0: origin.xyz (float bits), w = ex | ey << 8 | ez << 16 | imask << 24
-//       (e* are biased power-of-two exponents of the quantisation step,
-//        imask bit s = slot s holds an internal child)
-//   q1: x = first child node, y = first triangle record,
-//       z = meta[0..3], w = meta[4..7]
+// Node record: 96 bytes, 32-byte aligned, read with three 256-bit loads.
+//   q0: origin.xyz (float bits), w = first child node
+//   q1: quantisation step per axis (float bits of powers of two), w = first
+//       triangle record
 //   q2: x/y = qlo.x[0..7], z/w = qhi.x[0..7]   (one byte per slot)
 //   q3: same for y, q4: same for z
-// meta byte: 0 = empty slot; 0x80 = internal child; otherwise a leaf with
-// count (1..3) in bits 5-6 and the offset of its first triangle from the
-// node's first triangle record (0..23) in bits 0-4.
+//   q5: x = slots word, the rest 0
+// The lanes of a warp visit different nodes, so each of a lane's loads costs
+// L1 a cycle of its own: as five 16-byte loads of an 80-byte record the node
+// fetches kept L1's data pipe 70 % busy; in three loads the record is read in
+// three cycles a lane, and it covers three 32-byte sectors either way.
+// Slots word: one nibble per slot. 0 = empty slot; 8 = internal child;
+// 1, 3 or 7 = a leaf with 1, 2 or 3 triangles (one bit each). The triangles
+// of a node's leaves are stored contiguously in slot order, so the triangle
+// of bit b is record first_triangle + popc(slots & 0x77777777 & ((1 << b) - 1)).
+// The traversal gets a node's hit children and hit triangles from one AND
+// with a mask that has a whole nibble per hit slot.
 // Internal children of a node are stored contiguously in slot order, so the
-// child in slot s is node first_child + popc(imask & ((1 << s) - 1)).
+// child in slot s is node first_child + popc(slots & 0x88888888 & ((8 << 4 s) - 1)).
 // Slots are assigned so that a ray in octant o visits children in
 // descending order of (slot ^ (7 - o)), which approximates front to back.
 // ---------------------------------------------------------------------------
-struct __align__(16) Node8 {
+struct __align__(32) Node8 {
+    uint4 q[6];
+};
+static_assert(sizeof(Node8) == 96, "node record must be 96 bytes");
+
+// Node record of a scene file: 80 bytes.
+//   q0: origin.xyz, w = ex | ey << 8 | ez << 16 | imask << 24 (e* are the
+//       biased exponents of the quantisation steps, imask bit s = slot s holds
+//       an internal child)
+//   q1: x = first child node, y = first triangle record,
+//       z = meta[0..3], w = meta[4..7]
+//   q2..q4: the plane bytes, as above
+// meta byte of a slot: 0 = empty; 0x80 = internal child; otherwise a leaf
+// with count (1..3) in bits 5-6 and the offset of its first triangle from the
+// node's first triangle record (0..23) in bits 0-4.
+struct __align__(16) FileNode8 {
     uint4 q[5];
 };
-static_assert(sizeof(Node8) == 80, "node record must be 80 bytes");
+static_assert(sizeof(FileNode8) == 80, "file node record must be 80 bytes");
 
-// Triangle record: 48 bytes = 3 x float4.
+// Triangle record: 64 bytes, 32-byte aligned, read with two loads.
 //   a = (v0.x, v0.y, v0.z, n.x), b = (e1.xyz, n.y), c = (e2.xyz, n.z)
+//   id = (index in the input mesh, material (low 16 bits) | light (high 16,
+//         0xffff none; written by build_tri_attr before a render), 0, 0)
 // with e1 = v1 - v0, e2 = v2 - v0, n = e1 x e2 evaluated exactly as the
 // reference does (IndexedTriangle.cpp:44-45, :103), one rounding per op.
-struct __align__(16) Tri {
+struct __align__(32) Tri {
+    float4 a, b, c;
+    uint4 id;
+};
+static_assert(sizeof(Tri) == 64, "triangle record must be 64 bytes");
+
+// Triangle record of a scene file: 48 bytes (the input indices follow as an
+// array of their own).
+struct __align__(16) FileTri {
     float4 a, b, c;
 };
-static_assert(sizeof(Tri) == 48, "triangle record must be 48 bytes");
+static_assert(sizeof(FileTri) == 48, "file triangle record must be 48 bytes");
 
 constexpr int kMaxStack = 64;      // traversal stack entries (node groups)
 // triangles per leaf child; measured on a B200 with the treelet-restructured
@@ -44,7 +75,49 @@ constexpr int kMaxStack = 64;      // traversal stack entries (node groups)
 // field, 960x540x16 ms): 1: 6790 / 2254, 25.6; 2: 7100 / 2357, 26.0;
 // 3: 6920 / 2316, 26.7
 constexpr int kLeafMax = 2;
-constexpr uint32_t kMetaInternal = 0x80u;
+constexpr uint32_t kSlotInner = 0x88888888u, kSlotTris = 0x77777777u;
+constexpr uint32_t kMetaInternal = 0x80u;  // scene file
+
+inline FileNode8 to_file(const Node8 &n)
+{
+    FileNode8 f;
+    uint32_t imask = 0, off = 0;
+    uint64_t meta = 0;
+    for (int s = 0; s < 8; s++) {
+        const uint32_t nib = (n.q[5].x >> (4 * s)) & 15u;
+        const uint32_t count = nib == 7u ? 3u : (nib == 3u ? 2u : (nib == 1u ? 1u : 0u));
+        if (nib == 8u) {
+            imask |= 1u << s;
+            meta |= (uint64_t)kMetaInternal << (8 * s);
+        } else if (count) {
+            meta |= (uint64_t)((count << 5) | off) << (8 * s);
+        }
+        off += count;
+    }
+    f.q[0] = uint4{n.q[0].x, n.q[0].y, n.q[0].z,
+                   n.q[1].x >> 23 | (n.q[1].y >> 23) << 8 | (n.q[1].z >> 23) << 16 | imask << 24};
+    f.q[1] = uint4{n.q[0].w, n.q[1].w, (uint32_t)meta, (uint32_t)(meta >> 32)};
+    for (int a = 0; a < 3; a++) f.q[2 + a] = n.q[2 + a];
+    return f;
+}
+
+// False when the record is not one that to_file writes (triangle offsets that
+// do not follow from the counts, or an imask that the slots contradict).
+inline bool from_file(const FileNode8 &f, Node8 &n)
+{
+    uint32_t slots = 0;
+    for (int s = 0; s < 8; s++) {
+        const uint32_t m = ((s < 4 ? f.q[1].z : f.q[1].w) >> (8 * (s & 3))) & 0xffu;
+        slots |= (m == kMetaInternal ? 8u : (1u << ((m >> 5) & 3u)) - 1u) << (4 * s);
+    }
+    const uint32_t e = f.q[0].w;
+    n.q[0] = uint4{f.q[0].x, f.q[0].y, f.q[0].z, f.q[1].x};
+    n.q[1] = uint4{(e & 0xffu) << 23, (e >> 8 & 0xffu) << 23, (e >> 16 & 0xffu) << 23, f.q[1].y};
+    for (int a = 0; a < 3; a++) n.q[2 + a] = f.q[2 + a];
+    n.q[5] = uint4{slots, 0u, 0u, 0u};
+    const FileNode8 back = to_file(n);
+    return back.q[0].w == f.q[0].w && back.q[1].z == f.q[1].z && back.q[1].w == f.q[1].w;
+}
 
 // Lower bound of the reference's triangle window, `t < 1e-5` evaluated in
 // double (IndexedTriangle.cpp:115): for a float t this is t < the smallest
@@ -62,13 +135,13 @@ __device__ __forceinline__ float window_hi(float tmax)
 // with every product and sum rounded separately (no contraction), so that t,
 // beta and gamma are bit-identical to the reference compiled without FMA.
 // `hi` is window_hi(current Max).
-__device__ __forceinline__ bool shirley(const Tri &tr, float ox, float oy, float oz, float dx, float dy,
+__device__ __forceinline__ bool shirley(float4 ta, float4 tb, float4 tc, float ox, float oy, float oz, float dx, float dy,
                                         float dz, float hi, float &t_out, float &b_out, float &g_out)
 {
-    const float nx = tr.a.w, ny = tr.b.w, nz = tr.c.w;
+    const float nx = ta.w, ny = tb.w, nz = tc.w;
     const float den = __fadd_rn(__fadd_rn(__fmul_rn(nx, dx), __fmul_rn(ny, dy)), __fmul_rn(nz, dz));
-    const float rcp = __fdiv_rn(1.0f, den);
-    const float ex = __fsub_rn(tr.a.x, ox), ey = __fsub_rn(tr.a.y, oy), ez = __fsub_rn(tr.a.z, oz);
+    const float rcp = __frcp_rn(den);  // correctly rounded, as the division 1 / den is
+    const float ex = __fsub_rn(ta.x, ox), ey = __fsub_rn(ta.y, oy), ez = __fsub_rn(ta.z, oz);
     const float num = __fadd_rn(__fadd_rn(__fmul_rn(nx, ex), __fmul_rn(ny, ey)), __fmul_rn(nz, ez));
     const float t = __fmul_rn(num, rcp);
     if (t > hi || t < window_lo()) return false;
@@ -77,10 +150,10 @@ __device__ __forceinline__ bool shirley(const Tri &tr, float ox, float oy, float
     const float iy = __fsub_rn(__fmul_rn(dz, ex), __fmul_rn(dx, ez));
     const float iz = __fsub_rn(__fmul_rn(dx, ey), __fmul_rn(dy, ex));
     const float beta =
-        __fmul_rn(__fadd_rn(__fadd_rn(__fmul_rn(ix, tr.c.x), __fmul_rn(iy, tr.c.y)), __fmul_rn(iz, tr.c.z)), -rcp);
+        __fmul_rn(__fadd_rn(__fadd_rn(__fmul_rn(ix, tc.x), __fmul_rn(iy, tc.y)), __fmul_rn(iz, tc.z)), -rcp);
     if (beta < 0.0f) return false;
     const float gamma =
-        __fmul_rn(__fadd_rn(__fadd_rn(__fmul_rn(ix, tr.b.x), __fmul_rn(iy, tr.b.y)), __fmul_rn(iz, tr.b.z)), rcp);
+        __fmul_rn(__fadd_rn(__fadd_rn(__fmul_rn(ix, tb.x), __fmul_rn(iy, tb.y)), __fmul_rn(iz, tb.z)), rcp);
     if (__fadd_rn(beta, gamma) > 1.0f || gamma < 0.0f) return false;
     // A NaN t (origin in the triangle's plane, direction parallel to it)
     // passes the reference's comparisons and poisons its ray.Max; it is
@@ -156,7 +229,7 @@ __device__ __forceinline__ bool watertight(float4 v0, float4 v1, float4 v2, floa
     if (det == 0.f) return false;
     const float Az = __fmul_rn(sh.sz, akz), Bz = __fmul_rn(sh.sz, bkz), Cz = __fmul_rn(sh.sz, ckz);
     const float T = __fadd_rn(__fadd_rn(__fmul_rn(U, Az), __fmul_rn(V, Bz)), __fmul_rn(W, Cz));
-    const float rcp = __fdiv_rn(1.0f, det);
+    const float rcp = __frcp_rn(det);
     const float t = __fmul_rn(T, rcp);
     if (!(t <= hi) || t < window_lo()) return false;
     t_out = t;

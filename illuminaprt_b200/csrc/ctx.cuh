@@ -79,7 +79,7 @@ struct ilg_ctx {
     bool lights_use_mesh = false;    // some light samples the uploaded mesh's triangles
     uint32_t mesh_gen = 0;           // bumped by every ilg_set_mesh / ilg_load
     uint32_t lights_mesh_gen = 0;    // mesh_gen the mesh lights' areas were computed for
-    ilg::DevBuf<uint32_t> tri_attr, light_of_prim;
+    ilg::DevBuf<uint32_t> light_of_prim;
     bool attr_dirty = true;
     // path tracing: wavefront buffers
     ilg::DevBuf<float4> q_o0, q_d0, q_o1, q_d1, beta, s_o, s_d, s_c, accum, accum_direct, accum_albedo;
@@ -142,7 +142,7 @@ struct ilg_ctx {
 
     ilg::SceneView view() const
     {
-        return ilg::SceneView{bb.nodes, bb.tris, bb.prim_of, stats.n_nodes, stats.n_tris};
+        return ilg::SceneView{bb.nodes, bb.tris, stats.n_nodes, stats.n_tris};
     }
 
     int check_device_error()
@@ -171,7 +171,7 @@ struct ilg_ctx {
         post_pixels = post_frames = 0;
         ro.release(); rd.release(); hprim.release(); ht.release(); hu.release(); hv.release(); hocc.release();
         derr.release(); dstats.release();
-        mats.release(); lights.release(); light_range.release(); tri_attr.release(); light_of_prim.release();
+        mats.release(); lights.release(); light_range.release(); light_of_prim.release();
         q_o0.release(); q_d0.release(); q_o1.release(); q_d1.release(); beta.release(); s_o.release();
         s_d.release(); s_c.release(); accum.release(); accum_direct.release(); accum_albedo.release(); q_p0.release(); q_p1.release(); counts.release();
         hit_tri.release(); hit_t.release(); out_dev.release(); path_scene.release(); s_sid.release();

@@ -523,10 +523,10 @@ __global__ void __launch_bounds__(256) k_shade(RenderDev R, int cur, uint32_t de
             if ((depth == 0 || after_specular) && S.inf_escape > 0.f) add = add + beta * S.inf_escape;
             if (tslot != 0xffffffffu && depth >= 2 && !is_black(add)) credit(R, tslot, depth - 1, add);
         } else if (depth <= S.max_depth) {
-            const uint32_t attr = S.tri_attr[ti];
+            const Tri tr = S.tris[ti];
+            const uint32_t attr = tr.id.y;
             const uint32_t mat_id = attr & 0xffffu, light_id = attr >> 16;
             const Mat m = S.mats[mat_id < S.n_mats ? mat_id : 0];
-            const Tri tr = S.tris[ti];
             const float3 ng = normalize3(make_float3(tr.a.w, tr.b.w, tr.c.w));
             const float t = R.hit_t[i];
             const float3 dd = make_float3(d.x, d.y, d.z);
@@ -692,131 +692,98 @@ __global__ void __launch_bounds__(256) k_shadow(RenderDev R)
 }
 
 // ---------------------------------------------------------------------------
-// Persistent forms of k_extend and k_shadow: each warp keeps its lanes busy by
-// fetching a new ray from a device counter whenever kRefillLanes lanes are
-// idle (as k_trace_dyn does for batched queries), so the incoherent bounce
-// and shadow rays do not leave lanes waiting on the longest ray of a warp.
-// Rays of one warp may belong to different scenes of a batch; each lane
-// traverses its own scene's tree.
+// Persistent forms of k_extend and k_shadow over trace_persistent, so the
+// incoherent bounce and shadow rays do not leave lanes waiting on the longest
+// ray of a warp. Rays of one warp may belong to different scenes of a batch;
+// each lane traverses its own scene's tree. Seven blocks an SM (72 registers):
+// measured on the 5.2 M-triangle field at 1920x1080, 4 samples, depth 12: six
+// blocks 16.9 ms, seven 15.7, eight (spilling) 16.3; 18.5 with the previous
+// traversal.
 // ---------------------------------------------------------------------------
-template <bool kAnyHit>
+__device__ __forceinline__ void bind_scene(TraceScene &T, const SceneRec &S)
+{
+    T.nodes = S.nodes;
+    T.tris = S.tris;
+    T.n_nodes = S.n_nodes;
+    T.n_tris = S.n_tris;
+}
+
+// kOne: a render of one scene, whose tree then stays in uniform registers
+// instead of six registers a lane (and two dependent loads a ray).
+template <bool kAnyHit, bool kOne>
 __device__ __forceinline__ void wave_trace_dyn(const RenderDev &R, uint32_t n, uint32_t *next, int cur)
 {
-    const uint32_t lane = threadIdx.x & 31u;
     __shared__ uint2 sstack[kShortStack * kStackColumns];  // launched with kStackColumns threads a block
     uint2 lstack[kMaxStack - kShortStack];
     const SplitStack stack{sstack + threadIdx.x, lstack};
-    RayState r;
-    const Node8 *nodes = nullptr;
-    const Tri *tris = nullptr;
-    uint32_t n_nodes = 0, n_tris = 0;
-    bool active = false, exhausted = false;  // exhausted is warp-uniform
+    TraceScene scene{nullptr, nullptr, 0u, 0u};
+    if (kOne) bind_scene(scene, R.scenes[0]);
     uint32_t id = 0;
-    while (true) {
-        const uint32_t idle = __ballot_sync(0xffffffffu, !active);
-        if (!exhausted && (__popc(idle) >= kRefillLanes || idle == 0xffffffffu)) {
-            const uint32_t leader = __ffs(idle) - 1u;
-            uint32_t base = 0;
-            if (lane == leader) base = atomicAdd(next, (uint32_t)__popc(idle));
-            base = __shfl_sync(0xffffffffu, base, leader);
-            if (base >= n) exhausted = true;
-            if (!active) {
-                const uint32_t k = base + __popc(idle & ((1u << lane) - 1u));
-                if (k < n) {
-                    id = k;
-                    const SceneRec &S = R.scenes[kAnyHit ? R.s_sid[id] : R.path_scene[R.q_path[cur][id]]];
-                    nodes = S.nodes;
-                    tris = S.tris;
-                    n_nodes = S.n_nodes;
-                    n_tris = S.n_tris;
-                    if (kAnyHit) ray_init(r, R.s_o[id], R.s_d[id], n_nodes);
-                    else ray_init(r, R.q_o[cur][id], R.q_d[cur][id], n_nodes);
-                    active = true;
-                }
-            }
-        }
-        if (__ballot_sync(0xffffffffu, active) == 0u) break;
-        if (active && ray_step<kAnyHit, false, false, false, kTrisPerStep, false, SplitStack>(r, stack, nodes, tris,
-                                                                                         n_nodes, n_tris, R.err)) {
+    trace_persistent<kAnyHit, false, false, kRefillLanes>(
+        stack, scene, n, next, R.err, nullptr,
+        [&](uint32_t k, RayState &r, TraceScene &T) {
+            id = k;
+            if (!kOne) bind_scene(T, R.scenes[kAnyHit ? R.s_sid[id] : R.path_scene[R.q_path[cur][id]]]);
+            if (kAnyHit) ray_init(r, R.s_o[id], R.s_d[id], T.n_nodes);
+            else ray_init(r, R.q_o[cur][id], R.q_d[cur][id], T.n_nodes);
+        },
+        [&](const RayState &r) {
             if (kAnyHit) {
                 if (r.best == -1) shadow_unoccluded(R, id);
             } else {
                 R.hit_tri[id] = r.best;
                 R.hit_t[id] = r.best >= 0 ? r.tcur : __int_as_float(0x7f800000);
             }
-            active = false;
-        }
-    }
+        });
 }
 
 // The shadow rays of depth d and the extension rays of depth d + 1 in one
 // persistent launch: both come from k_shade at depth d and neither reads
 // what the other writes (shadow rays add to the pixel sums and training
 // targets, extension rays write hit records), so one traversal loop
-// (ray_step<kMixed>) takes the extension rays first, then the shadow rays:
+// (trace_persistent<kMixed>) takes the extension rays first, then the shadow rays:
 // twice the rays in flight and one launch tail instead of two. `cur` is the
 // queue the extension rays are in.
-__global__ void __launch_bounds__(kStackColumns) k_trace_mixed(RenderDev R, int cur, uint32_t *next)
+template <bool kOne>
+__global__ void __launch_bounds__(kStackColumns, 7) k_trace_mixed(RenderDev R, int cur, uint32_t *next)
 {
-    const uint32_t lane = threadIdx.x & 31u;
     __shared__ uint2 sstack[kShortStack * kStackColumns];  // launched with kStackColumns threads a block
     uint2 lstack[kMaxStack - kShortStack];
     const SplitStack stack{sstack + threadIdx.x, lstack};
     const uint32_t n_ext = min(R.count[cur], R.capacity), n_sh = min(*R.sh_count, R.sh_capacity);
-    const uint32_t n = n_ext + n_sh;
-    RayState r;
-    const Node8 *nodes = nullptr;
-    const Tri *tris = nullptr;
-    uint32_t n_nodes = 0, n_tris = 0;
-    bool active = false, exhausted = false;  // exhausted is warp-uniform
+    TraceScene scene{nullptr, nullptr, 0u, 0u};
+    if (kOne) bind_scene(scene, R.scenes[0]);
     uint32_t id = 0;
-    while (true) {
-        const uint32_t idle = __ballot_sync(0xffffffffu, !active);
-        if (!exhausted && (__popc(idle) >= kRefillLanes || idle == 0xffffffffu)) {
-            const uint32_t leader = __ffs(idle) - 1u;
-            uint32_t base = 0;
-            if (lane == leader) base = atomicAdd(next, (uint32_t)__popc(idle));
-            base = __shfl_sync(0xffffffffu, base, leader);
-            if (base >= n) exhausted = true;
-            if (!active) {
-                const uint32_t k = base + __popc(idle & ((1u << lane) - 1u));
-                if (k < n) {
-                    const bool shadow = k >= n_ext;
-                    id = shadow ? k - n_ext : k;
-                    const SceneRec &S = R.scenes[shadow ? R.s_sid[id] : R.path_scene[R.q_path[cur][id]]];
-                    nodes = S.nodes;
-                    tris = S.tris;
-                    n_nodes = S.n_nodes;
-                    n_tris = S.n_tris;
-                    if (shadow) ray_init(r, R.s_o[id], R.s_d[id], n_nodes);
-                    else ray_init(r, R.q_o[cur][id], R.q_d[cur][id], n_nodes);
-                    r.any = shadow;
-                    active = true;
-                }
-            }
-        }
-        if (__ballot_sync(0xffffffffu, active) == 0u) break;
-        if (active && ray_step<false, false, false, false, kTrisPerStep, true, SplitStack>(r, stack, nodes, tris,
-                                                                                             n_nodes, n_tris, R.err)) {
+    trace_persistent<false, false, true, kRefillLanes>(
+        stack, scene, n_ext + n_sh, next, R.err, nullptr,
+        [&](uint32_t k, RayState &r, TraceScene &T) {
+            const bool shadow = k >= n_ext;
+            id = shadow ? k - n_ext : k;
+            if (!kOne) bind_scene(T, R.scenes[shadow ? R.s_sid[id] : R.path_scene[R.q_path[cur][id]]]);
+            if (shadow) ray_init(r, R.s_o[id], R.s_d[id], T.n_nodes);
+            else ray_init(r, R.q_o[cur][id], R.q_d[cur][id], T.n_nodes);
+            r.any = shadow;
+        },
+        [&](const RayState &r) {
             if (r.any) {
                 if (r.best == -1) shadow_unoccluded(R, id);
             } else {
                 R.hit_tri[id] = r.best;
                 R.hit_t[id] = r.best >= 0 ? r.tcur : __int_as_float(0x7f800000);
             }
-            active = false;
-        }
-    }
+        });
 }
 
-__global__ void __launch_bounds__(kStackColumns) k_extend_dyn(RenderDev R, int cur, uint32_t *next)
+template <bool kOne>
+__global__ void __launch_bounds__(kStackColumns, 7) k_extend_dyn(RenderDev R, int cur, uint32_t *next)
 {
-    wave_trace_dyn<false>(R, min(R.count[cur], R.capacity), next, cur);
+    wave_trace_dyn<false, kOne>(R, min(R.count[cur], R.capacity), next, cur);
 }
 
-__global__ void __launch_bounds__(kStackColumns) k_shadow_dyn(RenderDev R, uint32_t *next)
+template <bool kOne>
+__global__ void __launch_bounds__(kStackColumns, 7) k_shadow_dyn(RenderDev R, uint32_t *next)
 {
-    wave_trace_dyn<true>(R, min(*R.sh_count, R.sh_capacity), next, 0);
+    wave_trace_dyn<true, kOne>(R, min(*R.sh_count, R.sh_capacity), next, 0);
 }
 
 // ---------------------------------------------------------------------------
@@ -826,7 +793,7 @@ __global__ void __launch_bounds__(kStackColumns) k_shadow_dyn(RenderDev R, uint3
 // its path ends; a warp refills once kRefillLanesPersistent of its lanes are
 // idle. The paths of every scene of a batch, of any length, flow through the
 // same kernel with no host round trip and no queue in memory. Closest-hit
-// and shadow rays share one traversal loop (ray_step<kMixed>), so lanes
+// and shadow rays share one traversal loop (ray_tri<kMixed>), so lanes
 // tracing either kind stay on the same code; lanes whose ray finished wait
 // and shade together. The sample sequence, the shading code (light_sample,
 // continue_path) and the traversal are the wavefront's, so every path is the
@@ -928,10 +895,10 @@ __device__ __forceinline__ bool shade_vertex(const RenderDev &R, PathLane &P, co
         return false;
     }
     if (depth > S.max_depth) return false;
-    const uint32_t attr = S.tri_attr[ti];
+    const Tri tr = S.tris[ti];
+    const uint32_t attr = tr.id.y;
     const uint32_t mat_id = attr & 0xffffu, light_id = attr >> 16;
     const Mat m = S.mats[mat_id < S.n_mats ? mat_id : 0];
-    const Tri tr = S.tris[ti];
     const float3 ng = normalize3(make_float3(tr.a.w, tr.b.w, tr.c.w));
     const float t = r.tcur;
     const float3 p = make_float3(o.x + t * d.x, o.y + t * d.y, o.z + t * d.z);
@@ -980,16 +947,8 @@ __global__ void __launch_bounds__(kPersistThreads) k_render_persistent(RenderDev
     bool active = false, exhausted = false;  // exhausted is warp-uniform
     // 0: tracing; 1: closest hit found, waiting to shade; 2: shadow ray done, waiting to be counted
     uint32_t state = 0;
-    const Node8 *nodes = nullptr;
-    const Tri *tris = nullptr;
-    uint32_t n_nodes = 0, n_tris = 0;
-    auto bind_scene = [&]() {
-        const SceneRec &S = R.scenes[P.sid];
-        nodes = S.nodes;
-        tris = S.tris;
-        n_nodes = S.n_nodes;
-        n_tris = S.n_tris;
-    };
+    TraceScene scene{nullptr, nullptr, 0u, 0u};
+    const uint32_t magic = plane_magic(R.n_scenes);
     while (true) {
         const uint32_t idle = __ballot_sync(0xffffffffu, !active);
         if (!exhausted && (__popc(idle) >= kRefillLanesPersistent || idle == 0xffffffffu)) {
@@ -1002,7 +961,7 @@ __global__ void __launch_bounds__(kPersistThreads) k_render_persistent(RenderDev
                 const uint64_t k = base + __popc(idle & ((1u << lane) - 1u));
                 if (k < total) {
                     start_path(R, k, P, r);
-                    bind_scene();
+                    bind_scene(scene, R.scenes[P.sid]);
                     ro = make_float4(r.ox, r.oy, r.oz, r.tmin);
                     rd = make_float4(r.dx, r.dy, r.dz, r.tcur);
                     active = true;
@@ -1012,9 +971,16 @@ __global__ void __launch_bounds__(kPersistThreads) k_render_persistent(RenderDev
         }
         const uint32_t live = __ballot_sync(0xffffffffu, active);
         if (live == 0u) break;
-        if (active && state == 0 &&
-            ray_step<false, false, false, false, kTrisPerStep, true>(r, stack, nodes, tris, n_nodes, n_tris, R.err))
-            state = r.any ? 2u : 1u;
+        const bool trace = active && state == 0u;
+        __syncwarp();
+        if (trace && r.tq_hits == 0u && ray_has_nodes(r)) ray_node(r, stack, scene.nodes, scene.n_nodes, magic, R.err);
+        while (true) {
+            const uint32_t tri = __ballot_sync(0xffffffffu, trace && r.tg_hits != 0u);
+            const uint32_t node = __ballot_sync(0xffffffffu, trace && r.tq_hits == 0u && ray_has_nodes(r));
+            if (tri == 0u || (__popc(tri) < kTriLanes && __popc(node) >= kNodeLanes)) break;
+            if (trace && r.tg_hits) ray_tri<false, false, false, false, true>(r, scene.tris, scene.n_tris, R.err);
+        }
+        if (trace && r.tg_hits == 0u && !ray_has_nodes(r)) state = r.any ? 2u : 1u;
         // Shading and shadow results run for the waiting lanes together, once
         // three quarters of the warp's paths wait or none is tracing, so that
         // this code runs with most lanes converged instead of one lane at a
@@ -1052,13 +1018,13 @@ __global__ void k_resolve(const float4 *__restrict__ accum, uint32_t wh, float s
     out[3 * p + 2] = a.z * scale;
 }
 
-__global__ void k_tri_attr(const uint32_t *__restrict__ prim_of, uint32_t n, const uint32_t *__restrict__ mat_ids,
-                           const uint32_t *__restrict__ light_of_prim, uint32_t *__restrict__ attr)
+__global__ void k_tri_attr(Tri *__restrict__ tris, uint32_t n, const uint32_t *__restrict__ mat_ids,
+                           const uint32_t *__restrict__ light_of_prim)
 {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
-    const uint32_t p = prim_of[i];
-    attr[i] = (mat_ids ? (mat_ids[p] & 0xffffu) : 0u) | (light_of_prim[p] << 16);
+    const uint32_t p = tris[i].id.x;
+    tris[i].id.y = (mat_ids ? (mat_ids[p] & 0xffffu) : 0u) | (light_of_prim[p] << 16);
 }
 
 __global__ void k_light_of_prim(uint32_t *lop, uint32_t n_prims, const uint2 *range, uint32_t n_lights)
@@ -1105,12 +1071,12 @@ cudaError_t triangle_areas(const float *pos, const uint32_t *idx, uint32_t first
     return cudaGetLastError();
 }
 
-cudaError_t build_tri_attr(const uint32_t *prim_of, uint32_t n_tris, const uint32_t *mat_ids,
+cudaError_t build_tri_attr(Tri *tris, uint32_t n_tris, const uint32_t *mat_ids,
                            const uint2 *light_range, uint32_t n_lights, uint32_t *light_of_prim,
-                           uint32_t *attr, cudaStream_t st)
+                           cudaStream_t st)
 {
     k_light_of_prim<<<blocks_for(n_tris, 256), 256, 0, st>>>(light_of_prim, n_tris, light_range, n_lights);
-    k_tri_attr<<<blocks_for(n_tris, 256), 256, 0, st>>>(prim_of, n_tris, mat_ids, light_of_prim, attr);
+    k_tri_attr<<<blocks_for(n_tris, 256), 256, 0, st>>>(tris, n_tris, mat_ids, light_of_prim);
     return cudaGetLastError();
 }
 
@@ -1217,7 +1183,7 @@ cudaError_t render_wave(const RenderDev &R, uint32_t n_paths, uint64_t wave_begi
     const uint32_t last = (R.cache_depth && R.train_tail && cache) ? std::min(R.depth_max, tail) : R.depth_max;
     // persistent traversal: the shadow rays of depth d and the extension rays
     // of depth d + 1 go in one launch (k_trace_mixed)
-    const bool merge = R.persistent && !R.stats;
+    const bool merge = R.persistent && !R.stats, one = R.n_scenes == 1u;
     bool traced = false;  // this depth's extension rays were traced with the previous depth's shadow rays
     for (uint32_t depth = 0; depth <= last; depth++) {
         if (!traced) {
@@ -1229,7 +1195,8 @@ cudaError_t render_wave(const RenderDev &R, uint32_t n_paths, uint64_t wave_begi
                 k_extend<false><<<blocks_for(n_paths, T), T, 0, st>>>(R, cur);
             } else {
                 if ((e = cudaMemsetAsync(R.count + 6, 0, sizeof(uint32_t), st)) != cudaSuccess) return e;
-                k_extend_dyn<<<persistent_blocks(n_paths), kStackColumns, 0, st>>>(R, cur, R.count + 6);
+                (one ? k_extend_dyn<true> : k_extend_dyn<false>)<<<persistent_blocks(n_paths), kStackColumns, 0, st>>>(
+                    R, cur, R.count + 6);
             }
             n_launch++;
         }
@@ -1247,8 +1214,8 @@ cudaError_t render_wave(const RenderDev &R, uint32_t n_paths, uint64_t wave_begi
         }
         if (depth < last && merge) {
             if ((e = cudaMemsetAsync(R.count + 6, 0, sizeof(uint32_t), st)) != cudaSuccess) return e;
-            k_trace_mixed<<<persistent_blocks((uint64_t)n_paths + R.sh_capacity), kStackColumns, 0, st>>>(
-                R, cur ^ 1, R.count + 6);
+            (one ? k_trace_mixed<true> : k_trace_mixed<false>)<<<persistent_blocks((uint64_t)n_paths + R.sh_capacity),
+                                                                 kStackColumns, 0, st>>>(R, cur ^ 1, R.count + 6);
             // the queues the next k_shade appends to, now that they are consumed
             if ((e = cudaMemsetAsync(R.count + cur, 0, sizeof(uint32_t), st)) != cudaSuccess) return e;
             if ((e = cudaMemsetAsync(R.sh_count, 0, sizeof(uint32_t), st)) != cudaSuccess) return e;
@@ -1261,7 +1228,8 @@ cudaError_t render_wave(const RenderDev &R, uint32_t n_paths, uint64_t wave_begi
                 k_shadow<false><<<blocks_for((uint64_t)R.sh_capacity, T), T, 0, st>>>(R);
             } else {
                 if ((e = cudaMemsetAsync(R.count + 7, 0, sizeof(uint32_t), st)) != cudaSuccess) return e;
-                k_shadow_dyn<<<persistent_blocks(R.sh_capacity), kStackColumns, 0, st>>>(R, R.count + 7);
+                (one ? k_shadow_dyn<true> : k_shadow_dyn<false>)<<<persistent_blocks(R.sh_capacity), kStackColumns, 0,
+                                                                   st>>>(R, R.count + 7);
             }
             n_launch++;
         }

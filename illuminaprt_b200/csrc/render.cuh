@@ -36,7 +36,6 @@ struct SceneRec {
     const Node8 *nodes;
     const Tri *tris;
     uint32_t n_nodes, n_tris;
-    const uint32_t *tri_attr;  // per triangle record: material (low 16) | light (high 16, 0xffff none)
     const Mat *mats;
     uint32_t n_mats;
     const Light *lights;
@@ -122,10 +121,11 @@ struct RenderDev {
     uint32_t *s_meta;          // per shadow segment: (slot << 8 | vertex) of a training path, or ~0
 };
 
-// light_range: per light (first triangle, triangle count) in the uploaded mesh
-cudaError_t build_tri_attr(const uint32_t *prim_of, uint32_t n_tris, const uint32_t *mat_ids,
+// Writes the records' material and light ids. light_range: per light (first
+// triangle, triangle count) in the uploaded mesh
+cudaError_t build_tri_attr(Tri *tris, uint32_t n_tris, const uint32_t *mat_ids,
                            const uint2 *light_range, uint32_t n_lights, uint32_t *light_of_prim,
-                           uint32_t *attr, cudaStream_t st);
+                           cudaStream_t st);
 // area[k] = area of uploaded triangle first + k (0.5 |(v1 - v0) x (v2 - v0)|,
 // IndexedTriangle::GetArea, Core/Shape/IndexedTriangle.cpp:386-393)
 cudaError_t triangle_areas(const float *pos, const uint32_t *idx, uint32_t first, uint32_t count, float *area,

@@ -11,7 +11,6 @@ namespace ilg {
 struct SceneView {
     const Node8 *nodes;
     const Tri *tris;
-    const uint32_t *prim_of;
     uint32_t n_nodes, n_tris;
 };
 
@@ -34,7 +33,7 @@ cudaError_t launch_closest_wt(const SceneView &s, const float4 *raw, const float
                               cudaStream_t st);
 cudaError_t launch_any_wt(const SceneView &s, const float4 *raw, const float4 *ro, const float4 *rd, uint32_t n,
                           uint8_t *occ, uint32_t *next, uint32_t *err, cudaStream_t st);
-cudaError_t build_raw_tris(const uint32_t *prim_of, const uint32_t *idx, const float *pos, uint32_t n, float4 *raw,
+cudaError_t build_raw_tris(const Tri *tris, const uint32_t *idx, const float *pos, uint32_t n, float4 *raw,
                            cudaStream_t st);
 
 // Loads the code of the closest-hit persistent kernel on the current device
