@@ -8,9 +8,9 @@
 //   3. radix sort     (code, triangle) pairs (CUB)
 //   4. k_karras       binary radix tree over the sorted codes (Karras 2012),
 //                     duplicate codes split by index
-//   5. k_refit        bottom-up AABBs, one atomic arrival counter per node
-//   5b. k_treelet     bottom-up treelet restructuring for least SAH cost
-//                     (Karras & Aila 2013); subtree triangle counts
+//   5. k_treelet      bottom-up AABBs and subtree triangle counts, one atomic
+//                     arrival counter per node, and treelet restructuring for
+//                     least SAH cost (Karras & Aila 2013)
 //   5c. k_collapse_cost  bottom-up SAH costs of the binary subtrees as 1..8
 //                     roots of an 8-wide node (Ylitie et al. 2017)
 //   6. k_collapse     level by level: each work item turns one binary node
@@ -21,10 +21,13 @@
 //                     triangle records of its leaf children.
 #include "bvh8.cuh"
 #include "build.cuh"
+#include "devinfo.cuh"
 
 #include <cub/device/device_radix_sort.cuh>
 
+#include <algorithm>
 #include <cfloat>
+#include <climits>
 #include <cmath>
 #include <utility>
 
@@ -65,7 +68,7 @@ __device__ __forceinline__ float area(const float3 &lo, const float3 &hi)
 // ---------------------------------------------------------------- step 1 ----
 __global__ void k_tri_bounds(const float *__restrict__ pos, uint32_t n_verts, const uint32_t *__restrict__ idx,
                              uint32_t n, float4 *__restrict__ tlo, float4 *__restrict__ thi,
-                             uint32_t *__restrict__ cbounds /* 6 flipped floats: min xyz, max xyz */,
+                             uint32_t *__restrict__ cbounds /* ordered maxima of -min xyz, max xyz; zeroed */,
                              uint32_t *__restrict__ err)
 {
     uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -88,23 +91,21 @@ __global__ void k_tri_bounds(const float *__restrict__ pos, uint32_t n_verts, co
         clo = make_float3(0.5f * (lo.x + hi.x), 0.5f * (lo.y + hi.y), 0.5f * (lo.z + hi.z));
         chi = clo;
     }
-    // warp reduce, then one atomic per warp
-    for (int o = 16; o > 0; o >>= 1) {
-        clo.x = fminf(clo.x, __shfl_xor_sync(0xffffffffu, clo.x, o));
-        clo.y = fminf(clo.y, __shfl_xor_sync(0xffffffffu, clo.y, o));
-        clo.z = fminf(clo.z, __shfl_xor_sync(0xffffffffu, clo.z, o));
-        chi.x = fmaxf(chi.x, __shfl_xor_sync(0xffffffffu, chi.x, o));
-        chi.y = fmaxf(chi.y, __shfl_xor_sync(0xffffffffu, chi.y, o));
-        chi.z = fmaxf(chi.z, __shfl_xor_sync(0xffffffffu, chi.z, o));
+    // block reduce over ordered integers, then one atomic per block and bound
+    // (one per warp kept 8 K warps waiting on six addresses: 34 us for 262 K
+    // triangles, 9 us so)
+    __shared__ uint32_t s_bound[6];
+    if (threadIdx.x < 6) s_bound[threadIdx.x] = 0u;
+    __syncthreads();
+    const uint32_t key[6] = {~float_flip(clo.x), ~float_flip(clo.y), ~float_flip(clo.z),
+                             float_flip(chi.x),  float_flip(chi.y),  float_flip(chi.z)};
+#pragma unroll
+    for (int k = 0; k < 6; k++) {
+        const uint32_t m = __reduce_max_sync(0xffffffffu, key[k]);
+        if ((threadIdx.x & 31) == 0) atomicMax(&s_bound[k], m);
     }
-    if ((threadIdx.x & 31) == 0) {
-        atomicMin(&cbounds[0], float_flip(clo.x));
-        atomicMin(&cbounds[1], float_flip(clo.y));
-        atomicMin(&cbounds[2], float_flip(clo.z));
-        atomicMax(&cbounds[3], float_flip(chi.x));
-        atomicMax(&cbounds[4], float_flip(chi.y));
-        atomicMax(&cbounds[5], float_flip(chi.z));
-    }
+    __syncthreads();
+    if (threadIdx.x < 6) atomicMax(&cbounds[threadIdx.x], s_bound[threadIdx.x]);
 }
 
 // ---------------------------------------------------------------- step 2 ----
@@ -114,7 +115,7 @@ __global__ void k_morton(const float4 *__restrict__ tlo, const float4 *__restric
 {
     uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
-    float3 lo = make_float3(float_unflip(cbounds[0]), float_unflip(cbounds[1]), float_unflip(cbounds[2]));
+    float3 lo = make_float3(float_unflip(~cbounds[0]), float_unflip(~cbounds[1]), float_unflip(~cbounds[2]));
     float3 hi = make_float3(float_unflip(cbounds[3]), float_unflip(cbounds[4]), float_unflip(cbounds[5]));
     float4 a = tlo[i], b = thi[i];
     float cx = 0.5f * (a.x + b.x), cy = 0.5f * (a.y + b.y), cz = 0.5f * (a.z + b.z);
@@ -140,7 +141,7 @@ __device__ __forceinline__ int delta(const uint32_t *keys, int n, int i, int j)
 }
 
 __global__ void k_karras(const uint32_t *__restrict__ keys, int n, int2 *__restrict__ child,
-                         int *__restrict__ parent_int, int *__restrict__ parent_leaf, int2 *__restrict__ range)
+                         int *__restrict__ parent_int, int *__restrict__ parent_leaf)
 {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n - 1) return;
@@ -163,52 +164,25 @@ __global__ void k_karras(const uint32_t *__restrict__ keys, int n, int2 *__restr
         t = (t + 1) >> 1;
     }
     int gamma = i + s * d + min(d, 0);
-    int first = min(i, j), last = max(i, j);
+    const int first = min(i, j), last = max(i, j);
     int left = (first == gamma) ? ~gamma : gamma;
     int right = (last == gamma + 1) ? ~(gamma + 1) : gamma + 1;
     child[i] = make_int2(left, right);
-    range[i] = make_int2(first, last);
     if (i == 0) parent_int[0] = -1;  // the root ends every bottom-up walk
     if (left >= 0) parent_int[left] = i; else parent_leaf[~left] = i;
     if (right >= 0) parent_int[right] = i; else parent_leaf[~right] = i;
 }
 
 // ---------------------------------------------------------------- step 5 ----
-__global__ void k_refit(int n, const uint32_t *__restrict__ sorted_tri, const float4 *__restrict__ tlo,
-                        const float4 *__restrict__ thi, const int2 *__restrict__ child,
-                        const int *__restrict__ parent_int, const int *__restrict__ parent_leaf,
-                        uint32_t *__restrict__ arrivals, float4 *__restrict__ nlo, float4 *__restrict__ nhi)
-{
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    int p = parent_leaf[i];
-    // bounded by the tree height (< n); each node's second arrival proceeds
-    for (int guard = 0; p >= 0 && p < n - 1 && guard < n; guard++) {
-        __threadfence();
-        if (atomicAdd(&arrivals[p], 1u) == 0) return;
-        __threadfence();
-        int2 c = child[p];
-        float4 alo, ahi, blo, bhi;
-        if (c.x >= 0) { alo = __ldcg(&nlo[c.x]); ahi = __ldcg(&nhi[c.x]); }
-        else { uint32_t t = sorted_tri[~c.x]; alo = tlo[t]; ahi = thi[t]; }
-        if (c.y >= 0) { blo = __ldcg(&nlo[c.y]); bhi = __ldcg(&nhi[c.y]); }
-        else { uint32_t t = sorted_tri[~c.y]; blo = tlo[t]; bhi = thi[t]; }
-        __stcg(&nlo[p], make_float4(fminf(alo.x, blo.x), fminf(alo.y, blo.y), fminf(alo.z, blo.z), 0.f));
-        __stcg(&nhi[p], make_float4(fmaxf(ahi.x, bhi.x), fmaxf(ahi.y, bhi.y), fmaxf(ahi.z, bhi.z), 0.f));
-        p = parent_int[p];
-    }
-}
-
-// ------------------------------------------------------------- step 5b ----
-// Treelet restructuring (Karras & Aila 2013, "Fast parallel construction of
-// high-quality bounding volume hierarchies"): a second bottom-up pass over
-// the binary tree. At each internal node p, once both of its subtrees are
-// final, the treelet of p (p and the internal nodes below it found by
+// Boxes and counts, and treelet restructuring (Karras & Aila 2013, "Fast
+// parallel construction of high-quality bounding volume hierarchies"), in
+// bottom-up passes over the binary tree. At each internal node p, once both of
+// its subtrees are final, the treelet of p (p and the internal nodes below it found by
 // repeatedly opening the treelet leaf of largest surface area, until
 // kTreeletLeaves leaves) is rebuilt with the topology of least SAH cost over
 // those leaves, found by dynamic programming over the leaves' subsets. The
 // treelet keeps its node indices and its root's box; only the topology
-// below the root changes. The pass also leaves every internal node's
+// below the root changes. The passes also leave every internal node's
 // triangle count in cnt (the collapse reads it).
 // SAH cost model: internal node kSahCi x its area, triangle kSahCt x its area.
 constexpr int kTreeletLeaves = 7;
@@ -217,6 +191,17 @@ constexpr int kTreeletLeaves = 7;
 // 2 passes 6928 / 2319, 3 passes 6988 / 2331
 constexpr int kTreeletPasses = 2;
 constexpr float kSahCi = 1.2f, kSahCt = 1.0f;
+
+// Arrives at a binary node; true for the second of its two arrivals, which
+// sees everything written before the first. The counter wraps back to 0 for
+// the next pass. (One acquire-release atomic: with a full fence on either
+// side the walk up the tree spent most of its time in fences.)
+__device__ __forceinline__ bool second_arrival(uint32_t *count)
+{
+    uint32_t old;
+    asm volatile("atom.inc.acq_rel.gpu.global.u32 %0, [%1], 1;" : "=r"(old) : "l"(count) : "memory");
+    return old != 0u;
+}
 
 __device__ __forceinline__ void handle_box(int c, const uint32_t *sorted_tri, const float4 *tlo, const float4 *thi,
                                            const float4 *nlo, const float4 *nhi, float3 &lo, float3 &hi)
@@ -234,198 +219,292 @@ struct SubsetTable {
     uint8_t s[127];
     uint8_t start[8];
 };
-__constant__ SubsetTable c_subsets;
-
-SubsetTable make_subset_table()
+constexpr SubsetTable make_subset_table()
 {
     SubsetTable t{};
     int k = 0;
     for (int size = 1; size <= kTreeletLeaves; size++) {
         t.start[size - 1] = (uint8_t)k;
         for (int S = 1; S < (1 << kTreeletLeaves); S++)
-            if (__builtin_popcount(S) == size) t.s[k++] = (uint8_t)S;
+        {
+            int bits = 0;
+            for (int b = 0; b < kTreeletLeaves; b++) bits += (S >> b) & 1;
+            if (bits == size) t.s[k++] = (uint8_t)S;
+        }
     }
     t.start[kTreeletLeaves] = (uint8_t)k;
     return t;
 }
+__constant__ SubsetTable c_subsets = make_subset_table();
 
 constexpr int kTreeletThreads = 128;
 constexpr int kTreeletWarps = kTreeletThreads / 32;
 
-// One warp rebuilds the treelet of root p: every lane forms the same treelet
-// (the reads are the same), the lanes fill the subsets of one size per round
-// (each its own subsets' splits, against the smaller subsets of the rounds
-// before), then lane 0 writes the new topology below p if it is cheaper.
-// p's count and cost are final. All 32 lanes call this together.
-__device__ void treelet_warp(int p, float costp, const uint32_t *sorted_tri, const float4 *tlo, const float4 *thi,
-                             int2 *child, int *parent_int, int *parent_leaf, float4 *nlo, float4 *nhi, int *cnt,
-                             float *cost, float *s_copt, uint8_t *s_split, float *s_box)
+struct TreeletShared {
+    float copt[1 << kTreeletLeaves];     // least cost of each subset of the leaves
+    float area[1 << kTreeletLeaves];     // the area of its box
+    uint8_t split[1 << kTreeletLeaves];  // the part with the lowest leaf of its best split
+    float box[kTreeletLeaves][6];
+    int leaf[kTreeletLeaves], count[kTreeletLeaves];
+    int inner[kTreeletLeaves - 1];       // the treelet's internal nodes, its root first
+    int subset[kTreeletLeaves - 1];      // the new topology: internal node i's leaves
+    int2 kids[kTreeletLeaves - 1];
+};
+
+// Bit patterns of non-negative floats order like the floats. The least cost
+// over the lanes of `group` and, among equal ones, the largest Q: the split
+// that a loop over Q downwards finds first.
+__device__ __forceinline__ void best_split(uint32_t group, float &cost, int &Q)
 {
+    const uint32_t bits = __float_as_uint(cost);
+    const uint32_t least = __reduce_min_sync(group, bits);
+    Q = (int)__reduce_max_sync(group, bits == least ? (uint32_t)Q : 0u);
+    cost = __uint_as_float(least);
+}
+
+// Inserts a zero bit at position b of x.
+__device__ __forceinline__ int open_bit(int x, int b) { return ((x >> b) << (b + 1)) | (x & ((1 << b) - 1)); }
+
+// Bound by the dependent loads and the shared-memory search of each warp's
+// chain of treelets, not by memory traffic. Measured on a B200, the two passes
+// over 262 K triangles (with the boxes' pass before the first): 2.28 ms with
+// one lane walking the treelet and solving sizes 6 and 7, 0.94 ms so; the
+// whole build, with the scratch kept and the eight-lane collapse (0.45 ->
+// 0.12 ms), 12.0 -> 1.24 ms, and 18.0 -> 2.6 ms for 1 M triangles.
+//
+// One warp rebuilds the treelet of root p (box area areap). Lane k < 7 holds
+// leaf k: its handle, box, cost and count, loaded together when the leaf
+// enters the treelet, so opening a node costs two dependent loads. The
+// subsets' box areas are found four a lane; then the subsets of one size are
+// solved per round: one lane a subset up to size 5, four lanes a subset at
+// size 6 (31 splits each) and the whole warp at size 7 (63 splits). The new
+// topology, if cheaper, is laid out by lane 0 and written by six lanes.
+// Every cost is the same sum of the same floats whichever lane finds it.
+// p's count and cost are final. All 32 lanes call this together.
+__device__ void treelet_warp(int p, float areap, const uint32_t *sorted_tri, const float4 *tlo, const float4 *thi,
+                             int2 *child, int *parent_int, int *parent_leaf, float4 *nlo, float4 *nhi, int *cnt,
+                             float *cost, TreeletShared &s)
+{
+    constexpr uint32_t kFull = 0xffffffffu;
+    constexpr int kAll = (1 << kTreeletLeaves) - 1;
     const int lane = threadIdx.x & 31;
-    __syncwarp();
-    __threadfence();  // the subtree below p is final: written before its nodes' arrivals
-    auto sub_cost = [&](int h) {
-        if (h >= 0) return __ldcg(&cost[h]);
-        float3 lo, hi;
+    __syncwarp();  // behind the leader's arrival, which saw the subtree below p final
+    int h = 0, count = 1;
+    float3 lo = make_float3(0.f, 0.f, 0.f), hi = lo;
+    float a = -1.f, c = 0.f;
+    auto take = [&](int handle) {  // this lane's leaf
+        h = handle;
         handle_box(h, sorted_tri, tlo, thi, nlo, nhi, lo, hi);
-        return kSahCt * area(lo, hi);
+        a = area(lo, hi);
+        count = h >= 0 ? __ldcg(&cnt[h]) : 1;
+        c = h >= 0 ? __ldcg(&cost[h]) : kSahCt * a;
     };
-    int tl[kTreeletLeaves], tin[kTreeletLeaves - 1];
-    const int2 c = __ldcg(&child[p]);
-    float3 plo, phi;
-    handle_box(p, sorted_tri, tlo, thi, nlo, nhi, plo, phi);
-    int n_l = 2, n_in = 1;
-    tl[0] = c.x;
-    tl[1] = c.y;
-    tin[0] = p;
-    float cur = kSahCi * area(plo, phi);
-    while (n_l < kTreeletLeaves) {
-        int best = -1;
-        float best_a = -1.f;
-        for (int k = 0; k < n_l; k++) {
-            if (tl[k] < 0) continue;
-            float3 lo, hi;
-            handle_box(tl[k], sorted_tri, tlo, thi, nlo, nhi, lo, hi);
-            const float a = area(lo, hi);
-            if (a > best_a) { best_a = a; best = k; }
-        }
-        if (best < 0) break;
-        const int2 cc = __ldcg(&child[tl[best]]);
-        tin[n_in++] = tl[best];
-        cur += kSahCi * best_a;
-        tl[best] = cc.x;
-        tl[n_l++] = cc.y;
+    int2 kids = __ldcg(&child[p]);
+    if (lane < 2) take(lane ? kids.y : kids.x);
+    float cur = kSahCi * areap;
+    int inner = p;  // lane i: internal node i of the treelet
+    for (int n_l = 2; n_l < kTreeletLeaves; n_l++) {
+        // the leaf of largest area that is a node, the first of equal ones
+        const uint32_t key = lane < n_l && h >= 0 && a >= 0.f ? __float_as_uint(a) + 1u : 0u;
+        const uint32_t best = __reduce_max_sync(kFull, key);
+        if (best == 0u) return;  // (not reached: p has >= 7 triangles)
+        const int w = __ffs(__ballot_sync(kFull, key == best)) - 1;
+        const int open = __shfl_sync(kFull, h, w);
+        if (lane == n_l - 1) inner = open;
+        cur += kSahCi * __uint_as_float(best - 1u);
+        kids = __ldcg(&child[open]);
+        if (lane == w || lane == n_l) take(lane == w ? kids.x : kids.y);
     }
-    if (n_l < kTreeletLeaves) return;  // (not reached: p has >= 7 triangles)
-    // leaf boxes and costs, one lane each
     if (lane < kTreeletLeaves) {
-        float3 lo, hi;
-        handle_box(tl[lane], sorted_tri, tlo, thi, nlo, nhi, lo, hi);
-        float *bx = s_box + 6 * lane;
-        bx[0] = lo.x; bx[1] = lo.y; bx[2] = lo.z; bx[3] = hi.x; bx[4] = hi.y; bx[5] = hi.z;
-        s_copt[1 << lane] = sub_cost(tl[lane]);
+        float *b = s.box[lane];
+        b[0] = lo.x; b[1] = lo.y; b[2] = lo.z; b[3] = hi.x; b[4] = hi.y; b[5] = hi.z;
+        s.copt[1 << lane] = c;
+        s.leaf[lane] = h;
+        s.count[lane] = count;
+        if (lane < kTreeletLeaves - 1) s.inner[lane] = inner;
     }
     __syncwarp();
-    for (int k = 0; k < kTreeletLeaves; k++) cur += s_copt[1 << k];
-    for (int size = 2; size <= kTreeletLeaves; size++) {
+#pragma unroll
+    for (int k = 0; k < kTreeletLeaves; k++) cur += s.copt[1 << k];
+    auto join = [&](float3 &l, float3 &u, int k) {
+        const float *b = s.box[k];
+        l = make_float3(fminf(l.x, b[0]), fminf(l.y, b[1]), fminf(l.z, b[2]));
+        u = make_float3(fmaxf(u.x, b[3]), fmaxf(u.y, b[4]), fmaxf(u.z, b[5]));
+    };
+    {
+        float3 l = make_float3(FLT_MAX, FLT_MAX, FLT_MAX), u = make_float3(-FLT_MAX, -FLT_MAX, -FLT_MAX);
+#pragma unroll
+        for (int k = 0; k < 5; k++)
+            if (lane >> k & 1) join(l, u, k);
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+            float3 l2 = l, u2 = u;
+            if (j & 1) join(l2, u2, 5);
+            if (j & 2) join(l2, u2, 6);
+            s.area[lane + 32 * j] = area(l2, u2);
+        }
+    }
+    __syncwarp();
+    // splits low | Q against S ^ low ^ Q, for Q downwards over the proper
+    // subsets of S without its lowest leaf
+    for (int size = 2; size <= 5; size++) {
         for (int j = c_subsets.start[size - 1] + lane; j < c_subsets.start[size]; j += 32) {
-            const int S = c_subsets.s[j];
-            float3 lo = make_float3(FLT_MAX, FLT_MAX, FLT_MAX), hi = make_float3(-FLT_MAX, -FLT_MAX, -FLT_MAX);
-            for (int k = 0; k < kTreeletLeaves; k++) {
-                if (!(S & (1 << k))) continue;
-                const float *bx = s_box + 6 * k;
-                lo = make_float3(fminf(lo.x, bx[0]), fminf(lo.y, bx[1]), fminf(lo.z, bx[2]));
-                hi = make_float3(fmaxf(hi.x, bx[3]), fmaxf(hi.y, bx[4]), fmaxf(hi.z, bx[5]));
-            }
-            // splits P | S ^ P with P holding S's lowest leaf (each split once)
-            const int low = S & -S;
+            const int S = c_subsets.s[j], low = S & -S, R = S ^ low;
             float best = FLT_MAX;
-            int bp = low;
-            for (int P = (S - 1) & S; P > 0; P = (P - 1) & S) {
-                if (!(P & low)) continue;
-                const float cc = s_copt[P] + s_copt[S ^ P];
-                if (cc < best) { best = cc; bp = P; }
+            int bq = 0;
+            for (int Q = (R - 1) & R;; Q = (Q - 1) & R) {
+                const float cc = s.copt[low | Q] + s.copt[R ^ Q];
+                if (cc < best) { best = cc; bq = Q; }
+                if (Q == 0) break;
             }
-            s_copt[S] = kSahCi * area(lo, hi) + best;
-            s_split[S] = (uint8_t)bp;
+            s.copt[S] = kSahCi * s.area[S] + best;
+            s.split[S] = (uint8_t)(low | bq);
         }
         __syncwarp();
     }
-    constexpr int kAll = (1 << kTreeletLeaves) - 1;
-    if (lane == 0 && s_copt[kAll] < cur * 0.9999f) {
-        // rebuild below p with the treelet's own internal nodes
-        int st_s[kTreeletLeaves], st_node[kTreeletLeaves];
-        int sp = 0, pool = 1;
-        st_s[sp] = kAll;
-        st_node[sp++] = p;
-        for (int it = 0; it < kTreeletLeaves && sp > 0; it++) {
-            const int S = st_s[--sp], node = st_node[sp];
-            const int parts[2] = {s_split[S], S ^ s_split[S]};
-            int h[2];
-            for (int q = 0; q < 2; q++) {
-                const int P = parts[q];
-                if ((P & (P - 1)) == 0) {
-                    h[q] = tl[__ffs(P) - 1];
-                } else {
-                    h[q] = tin[pool++];
-                    st_s[sp] = P;
-                    st_node[sp++] = h[q];
-                }
-                if (h[q] >= 0) __stcg(&parent_int[h[q]], node);
-                else __stcg(&parent_leaf[~h[q]], node);
-            }
-            __stcg(&child[node], make_int2(h[0], h[1]));
-            if (node != p) {
-                float3 lo = make_float3(FLT_MAX, FLT_MAX, FLT_MAX), hi = make_float3(-FLT_MAX, -FLT_MAX, -FLT_MAX);
-                int cn = 0;
-                for (int k = 0; k < kTreeletLeaves; k++) {
-                    if (!(S & (1 << k))) continue;
-                    const float *bx = s_box + 6 * k;
-                    lo = make_float3(fminf(lo.x, bx[0]), fminf(lo.y, bx[1]), fminf(lo.z, bx[2]));
-                    hi = make_float3(fmaxf(hi.x, bx[3]), fmaxf(hi.y, bx[4]), fmaxf(hi.z, bx[5]));
-                    cn += tl[k] >= 0 ? __ldcg(&cnt[tl[k]]) : 1;
-                }
-                __stcg(&nlo[node], make_float4(lo.x, lo.y, lo.z, 0.f));
-                __stcg(&nhi[node], make_float4(hi.x, hi.y, hi.z, 0.f));
-                __stcg(&cnt[node], cn);
-            }
-            __stcg(&cost[node], s_copt[S]);
+    if (lane < 28) {  // size 6: all leaves but e
+        const uint32_t group = 15u << (lane & 28);
+        const int e = lane >> 2, S = kAll ^ (1 << e), low = S & -S, R = S ^ low;
+        float best = FLT_MAX;
+        int bq = 0;
+        for (int i = 30 - (lane & 3); i >= 0; i -= 4) {
+            // bits of i to the places of R: 0..6 without 0 and e (e == 0: without 0 and 1)
+            const int Q = e == 0 ? i << 2 : open_bit(i << 1, e);
+            const float cc = s.copt[low | Q] + s.copt[R ^ Q];
+            if (cc < best) { best = cc; bq = Q; }
+        }
+        best_split(group, best, bq);
+        if ((lane & 3) == 0) {
+            s.copt[S] = kSahCi * s.area[S] + best;
+            s.split[S] = (uint8_t)(low | bq);
         }
     }
-    (void)costp;
     __syncwarp();
+    float all;
+    {
+        const int R = kAll ^ 1;
+        float best = FLT_MAX;
+        int bq = 0;
+#pragma unroll
+        for (int j = 1; j >= 0; j--) {
+            const int Q = 2 * (lane + 32 * j);
+            if (Q == R) continue;
+            const float cc = s.copt[1 | Q] + s.copt[R ^ Q];
+            if (cc < best) { best = cc; bq = Q; }
+        }
+        best_split(kFull, best, bq);
+        all = kSahCi * s.area[kAll] + best;
+        if (lane == 0) {
+            s.copt[kAll] = all;
+            s.split[kAll] = (uint8_t)(1 | bq);
+        }
+    }
+    if (!(all < cur * 0.9999f)) {
+        __syncwarp();
+        return;
+    }
+    if (lane == 0) {
+        int used = 1;
+        s.subset[0] = kAll;
+        for (int i = 0; i < kTreeletLeaves - 1; i++) {
+            const int S = s.subset[i];
+            int hs[2];
+#pragma unroll
+            for (int q = 0; q < 2; q++) {
+                const int P = q ? S ^ s.split[S] : s.split[S];
+                if ((P & (P - 1)) == 0) {
+                    hs[q] = s.leaf[__ffs(P) - 1];
+                } else {
+                    s.subset[used] = P;
+                    hs[q] = s.inner[used++];
+                }
+            }
+            s.kids[i] = make_int2(hs[0], hs[1]);
+        }
+    }
+    __syncwarp();
+    if (lane < kTreeletLeaves - 1) {
+        const int node = s.inner[lane], S = s.subset[lane];
+        const int2 k2 = s.kids[lane];
+        if (k2.x >= 0) __stcg(&parent_int[k2.x], node);
+        else __stcg(&parent_leaf[~k2.x], node);
+        if (k2.y >= 0) __stcg(&parent_int[k2.y], node);
+        else __stcg(&parent_leaf[~k2.y], node);
+        __stcg(&child[node], k2);
+        __stcg(&cost[node], s.copt[S]);
+        if (lane) {
+            float3 l = make_float3(FLT_MAX, FLT_MAX, FLT_MAX), u = make_float3(-FLT_MAX, -FLT_MAX, -FLT_MAX);
+            int cn = 0;
+#pragma unroll
+            for (int k = 0; k < kTreeletLeaves; k++) {
+                if (!(S >> k & 1)) continue;
+                join(l, u, k);
+                cn += s.count[k];
+            }
+            __stcg(&nlo[node], make_float4(l.x, l.y, l.z, 0.f));
+            __stcg(&nhi[node], make_float4(u.x, u.y, u.z, 0.f));
+            __stcg(&cnt[node], cn);
+        }
+    }
+    __syncwarp();  // before the leader's arrival at p's parent, which releases these writes
 }
 
-// The bottom-up pass: every lane walks up from its leaf; a lane whose node
-// has both subtrees final (second arrival) sets the node's count and cost,
-// and the warp then rebuilds, one after another, the treelets of the nodes
-// its lanes hold that have >= kTreeletLeaves triangles. Lanes stay in the
-// loop until the whole warp is done (the treelet work uses all 32).
+// The bottom-up pass: every lane with a leaf walks up from it; a lane whose
+// node has both subtrees final (second arrival) sets the node's box
+// (kBoxes: the first pass), count and cost, and the warp then rebuilds, one
+// after another, the treelets of the nodes its lanes hold that have >=
+// kTreeletLeaves triangles. Lanes stay in the loop until the whole warp is
+// done (the treelet work uses all 32). The arrival counters wrap back to 0.
+template <bool kBoxes>
 __global__ void __launch_bounds__(kTreeletThreads) k_treelet(int n, const uint32_t *__restrict__ sorted_tri,
                                                              const float4 *__restrict__ tlo,
                                                              const float4 *__restrict__ thi, int2 *child,
                                                              int *parent_int, int *parent_leaf,
                                                              uint32_t *__restrict__ arrivals, float4 *nlo,
-                                                             float4 *nhi, int *cnt, float *cost, int restructure)
+                                                             float4 *nhi, int *cnt, float *cost, int restructure,
+                                                             int leaves)
 {
-    __shared__ float s_copt[kTreeletWarps][1 << kTreeletLeaves];
-    __shared__ uint8_t s_split[kTreeletWarps][1 << kTreeletLeaves];
-    __shared__ float s_box[kTreeletWarps][6 * kTreeletLeaves];
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    __shared__ TreeletShared shared[kTreeletWarps];
     const int w = threadIdx.x >> 5;
-    int p = i < n ? parent_leaf[i] : -1;
-    bool alive = i < n;
+    const int lane = threadIdx.x & 31, i = (blockIdx.x * kTreeletWarps + w) * leaves + lane;
+    bool alive = lane < leaves && i < n;
+    int p = alive ? parent_leaf[i] : -1;
     for (int guard = 0; guard <= n; guard++) {
         bool ready = false;
-        float costp = 0.f;
+        float ap = 0.f;
         if (alive && (p < 0 || p >= n - 1)) alive = false;
         if (alive) {
-            __threadfence();
-            if (atomicAdd(&arrivals[p], 1u) == 0) {
+            if (!second_arrival(&arrivals[p])) {
                 alive = false;
             } else {
-                __threadfence();
-                ready = true;
                 const int2 c = __ldcg(&child[p]);
-                float3 plo, phi;
-                handle_box(p, sorted_tri, tlo, thi, nlo, nhi, plo, phi);
                 int cp = 0;
-                float cc = kSahCi * area(plo, phi);
+                float part[2];
+                float3 plo = make_float3(FLT_MAX, FLT_MAX, FLT_MAX), phi = make_float3(-FLT_MAX, -FLT_MAX, -FLT_MAX);
+#pragma unroll
                 for (int q = 0; q < 2; q++) {
                     const int h = q ? c.y : c.x;
-                    if (h >= 0) {
-                        cp += __ldcg(&cnt[h]);
-                        cc += __ldcg(&cost[h]);
-                    } else {
+                    if (kBoxes || h < 0) {
                         float3 lo, hi;
                         handle_box(h, sorted_tri, tlo, thi, nlo, nhi, lo, hi);
-                        cp += 1;
-                        cc += kSahCt * area(lo, hi);
+                        if (kBoxes) {
+                            plo = make_float3(fminf(plo.x, lo.x), fminf(plo.y, lo.y), fminf(plo.z, lo.z));
+                            phi = make_float3(fmaxf(phi.x, hi.x), fmaxf(phi.y, hi.y), fmaxf(phi.z, hi.z));
+                        }
+                        part[q] = kSahCt * area(lo, hi);
                     }
+                    if (h >= 0) part[q] = __ldcg(&cost[h]);
+                    cp += h >= 0 ? __ldcg(&cnt[h]) : 1;
                 }
+                if (kBoxes) {
+                    __stcg(&nlo[p], make_float4(plo.x, plo.y, plo.z, 0.f));
+                    __stcg(&nhi[p], make_float4(phi.x, phi.y, phi.z, 0.f));
+                } else {
+                    handle_box(p, sorted_tri, tlo, thi, nlo, nhi, plo, phi);
+                }
+                ap = area(plo, phi);
                 __stcg(&cnt[p], cp);
-                __stcg(&cost[p], cc);
-                costp = cc;
+                __stcg(&cost[p], kSahCi * ap + part[0] + part[1]);
                 ready = restructure && cp >= kTreeletLeaves;
             }
         }
@@ -434,9 +513,8 @@ __global__ void __launch_bounds__(kTreeletThreads) k_treelet(int n, const uint32
             const int leader = __ffs(todo) - 1;
             todo &= todo - 1;
             const int q = __shfl_sync(0xffffffffu, p, leader);
-            const float qc = __shfl_sync(0xffffffffu, costp, leader);
-            treelet_warp(q, qc, sorted_tri, tlo, thi, child, parent_int, parent_leaf, nlo, nhi, cnt, cost, s_copt[w],
-                         s_split[w], s_box[w]);
+            const float qa = __shfl_sync(0xffffffffu, ap, leader);
+            treelet_warp(q, qa, sorted_tri, tlo, thi, child, parent_int, parent_leaf, nlo, nhi, cnt, cost, shared[w]);
         }
         if (alive) p = __ldcg(&parent_int[p]);
         if (!__any_sync(0xffffffffu, alive)) break;
@@ -486,9 +564,7 @@ __global__ void __launch_bounds__(128) k_collapse_cost(int n, const uint32_t *__
     if (i >= n) return;
     int p = parent_leaf[i];
     for (int guard = 0; p >= 0 && p < n - 1 && guard < n; guard++) {
-        __threadfence();
-        if (atomicAdd(&arrivals[p], 1u) == 0) return;
-        __threadfence();
+        if (!second_arrival(&arrivals[p])) return;
         const int2 c = child[p];
         float ca[8], cb[8];
         root_costs(c.x, sorted_tri, tlo, thi, dpc, ca);
@@ -578,6 +654,25 @@ __device__ __forceinline__ int leaf_tris(int c, const int2 *child, int (&out)[kL
     return m;
 }
 
+// The record of input triangle t.
+__device__ __forceinline__ void write_tri(Tri *dst, uint32_t t, const float *__restrict__ pos,
+                                          const uint32_t *__restrict__ idx)
+{
+    const uint32_t a = idx[3 * t], b = idx[3 * t + 1], c = idx[3 * t + 2];
+    const float v0x = pos[3 * a], v0y = pos[3 * a + 1], v0z = pos[3 * a + 2];
+    const float e1x = __fsub_rn(pos[3 * b], v0x), e1y = __fsub_rn(pos[3 * b + 1], v0y),
+                e1z = __fsub_rn(pos[3 * b + 2], v0z);
+    const float e2x = __fsub_rn(pos[3 * c], v0x), e2y = __fsub_rn(pos[3 * c + 1], v0y),
+                e2z = __fsub_rn(pos[3 * c + 2], v0z);
+    const float nx = __fsub_rn(__fmul_rn(e1y, e2z), __fmul_rn(e1z, e2y));
+    const float ny = __fsub_rn(__fmul_rn(e1z, e2x), __fmul_rn(e1x, e2z));
+    const float nz = __fsub_rn(__fmul_rn(e1x, e2y), __fmul_rn(e1y, e2x));
+    dst->a = make_float4(v0x, v0y, v0z, nx);
+    dst->b = make_float4(e1x, e1y, e1z, ny);
+    dst->c = make_float4(e2x, e2y, e2z, nz);
+    dst->id = make_uint4(t, 0u, 0u, 0u);
+}
+
 // Quantisation step for one axis: the smallest power of two 2^e with
 // extent / 2^e <= 255 - 2 (one step of slack each side), and never below
 // `min_step` so that a step stays many float ulps wide.
@@ -593,186 +688,234 @@ __device__ __forceinline__ int quant_exp(float extent, float min_step)
 
 __device__ __forceinline__ float exp2i(int e) { return ldexpf(1.0f, e); }
 
-__global__ void k_collapse(const Work *__restrict__ in, const uint32_t *__restrict__ in_count, Work *__restrict__ out,
-                           uint32_t *__restrict__ out_count, uint32_t out_cap, const int2 *__restrict__ child,
-                           const int *__restrict__ cnt, const uint8_t *__restrict__ dpd, const float4 *__restrict__ nlo,
-                           const float4 *__restrict__ nhi, const uint32_t *__restrict__ sorted_tri,
-                           const float4 *__restrict__ tlo, const float4 *__restrict__ thi,
-                           const float *__restrict__ pos, const uint32_t *__restrict__ idx, Node8 *__restrict__ nodes,
-                           uint32_t *__restrict__ node_count, uint32_t node_cap, Tri *__restrict__ tris,
-                           uint32_t *__restrict__ tri_count, uint32_t tri_cap,
-                           float min_step, uint32_t *__restrict__ err)
+// One 8-wide node per group of eight lanes. The levels are short chains of
+// dependent loads, not much work: with one thread a node (which kept the
+// children, their scores and the slots in local memory) a level took 40 to
+// 50 us whatever its size.
+constexpr int kCollapseThreads = 128;
+
+__global__ void __launch_bounds__(kCollapseThreads)
+    k_collapse(const Work *__restrict__ in, const uint32_t *__restrict__ in_count, Work *__restrict__ out,
+               uint32_t *__restrict__ out_count, uint32_t out_cap, const int2 *__restrict__ child,
+               const int *__restrict__ cnt, const uint8_t *__restrict__ dpd, const float4 *__restrict__ nlo,
+               const float4 *__restrict__ nhi, const uint32_t *__restrict__ sorted_tri, const float4 *__restrict__ tlo,
+               const float4 *__restrict__ thi, const float *__restrict__ pos, const uint32_t *__restrict__ idx,
+               Node8 *__restrict__ nodes, uint32_t *__restrict__ node_count, uint32_t node_cap, Tri *__restrict__ tris,
+               uint32_t *__restrict__ tri_count, uint32_t tri_cap, float min_step, uint32_t *__restrict__ levels,
+               uint32_t *__restrict__ err)
 {
-    uint32_t w = blockIdx.x * blockDim.x + threadIdx.x;
-    if (w >= *in_count) return;
-    const Work job = in[w];
+    constexpr uint32_t kFull = 0xffffffffu;
+    constexpr int kNone = INT_MIN;
+    __shared__ uint32_t s_planes[kCollapseThreads / 8][12];  // per group: the node's plane bytes
+    __shared__ uint8_t s_at[kCollapseThreads];               // per group: the child in each slot
+    const int lane = threadIdx.x & 31, l = lane & 7, shift = lane & 24, group = threadIdx.x >> 3;
+    uint8_t *planes = reinterpret_cast<uint8_t *>(s_planes[group]);
+    // The host does not know how many items a level has: the grid strides
+    // over them. A level without items ends the build.
+    const uint32_t items = min(*in_count, out_cap);
+    if (blockIdx.x == 0 && threadIdx.x == 0 && items) *levels += 1u;
+    const uint32_t per_block = kCollapseThreads / 8, stride = gridDim.x * per_block;
+    for (uint32_t w0 = blockIdx.x * per_block; w0 < items; w0 += stride) {
+        const uint32_t w = w0 + group;
+        const bool live = w < items;
+        const Work job = live ? in[w] : Work{~0, 0u};
+        auto sum8 = [&](uint32_t v) {
+            for (int o = 1; o < 8; o <<= 1) v += __shfl_xor_sync(kFull, v, o);
+            return v;
+        };
+        auto min8 = [&](float v) {
+            for (int o = 1; o < 8; o <<= 1) v = fminf(v, __shfl_xor_sync(kFull, v, o));
+            return v;
+        };
+        auto ballot8 = [&](bool v) { return __ballot_sync(kFull, v) >> shift & 0xffu; };
 
-    int ch[8];
-    int m = 0;
-    if (job.bin >= 0) {
-        // the roots the collapse costs chose for this node's subtree below
-        // it: its children's split of 8 roots, each side followed down to the
-        // handles that stand as one root
-        const int2 c = child[job.bin];
-        const int k8 = dpd[16 * (size_t)job.bin + 7];
-        int st_h[16], st_i[16], sp = 0;
-        st_h[sp] = c.y;
-        st_i[sp++] = 8 - k8;
-        st_h[sp] = c.x;
-        st_i[sp++] = k8;
-        for (int it = 0; it < 32 && sp > 0 && m < 8; it++) {
-            const int h = st_h[--sp], r = st_i[sp];
-            const int j = h >= 0 ? dpd[16 * (size_t)h + 8 + r - 1] : 1;
-            if (j <= 1 || sp + 2 > 16) {
-                ch[m++] = h;
-                continue;
+        // The roots the collapse costs chose for the subtree below this
+        // node, left to right: a handle h that may spread over r roots starts
+        // at a lane and owns it and the r - 1 behind; a split into k and
+        // j - k roots leaves the left part there and puts the right part k
+        // lanes on.
+        int h = kNone, roots = 0;
+        if (live && job.bin < 0 && l == 0) h = job.bin;  // single-triangle scene
+        if (live && job.bin >= 0) {
+            const int2 c = child[job.bin];
+            const int k8 = dpd[16 * (size_t)job.bin + 7];
+            if (l == 0) { h = c.x; roots = k8; }
+            if (l == k8) { h = c.y; roots = 8 - k8; }
+        }
+        for (int round = 0; round < 8; round++) {
+            int j = 1, k = 0;
+            int2 c = make_int2(0, 0);
+            if (h >= 0) {
+                const uint4 d = *reinterpret_cast<const uint4 *>(dpd + 16 * (size_t)h);
+                c = child[h];
+                auto byte = [&](int b) {
+                    const uint32_t word = b < 8 ? (b < 4 ? d.x : d.y) : (b < 12 ? d.z : d.w);
+                    return (int)(word >> (8 * (b & 3)) & 0xffu);
+                };
+                j = byte(8 + roots - 1);
+                if (j > 1) k = byte(j - 1);
             }
-            const int k = dpd[16 * (size_t)h + j - 1];
-            const int2 cc = child[h];
-            st_h[sp] = cc.y;
-            st_i[sp++] = j - k;
-            st_h[sp] = cc.x;
-            st_i[sp++] = k;
+            const bool split = j > 1;
+            if (!__any_sync(kFull, split)) break;
+            const uint32_t owners = ballot8(h != kNone);
+            // the lane that owns this one, and whether its right part starts here
+            const int owner = 31 - __clz((owners & ((2u << l) - 1u)) | 1u);
+            const int ok = __shfl_sync(kFull, split ? k : 0, shift + owner);
+            const int oj = __shfl_sync(kFull, j, shift + owner), oy = __shfl_sync(kFull, c.y, shift + owner);
+            if (split) {
+                h = c.x;
+                roots = k;
+            } else if (h == kNone && ok > 0 && owner + ok == l) {
+                h = oy;
+                roots = oj - ok;
+            }
         }
-        if (sp > 0) { atomicOr(err, 16u); return; }
-    } else {
-        ch[m++] = job.bin;  // single-triangle scene
-    }
-
-    // child boxes, centroids, classification
-    float3 clo[8], chi[8];
-    float3 plo = make_float3(FLT_MAX, FLT_MAX, FLT_MAX), phi = make_float3(-FLT_MAX, -FLT_MAX, -FLT_MAX);
-    int n_int = 0, n_leaf_tris = 0;
-    for (int k = 0; k < m; k++) {
-        child_box(ch[k], sorted_tri, tlo, thi, nlo, nhi, clo[k], chi[k]);
-        plo = make_float3(fminf(plo.x, clo[k].x), fminf(plo.y, clo[k].y), fminf(plo.z, clo[k].z));
-        phi = make_float3(fmaxf(phi.x, chi[k].x), fmaxf(phi.y, chi[k].y), fmaxf(phi.z, chi[k].z));
-        if (is_node_root(ch[k], dpd)) n_int++;
-        else n_leaf_tris += child_count(ch[k], cnt);
-    }
-
-    // slot assignment: slot s is the corner with bit k set = positive along axis k
-    int slot_of[8];
-    {
-        float3 pc = make_float3(0.5f * (plo.x + phi.x), 0.5f * (plo.y + phi.y), 0.5f * (plo.z + phi.z));
-        float score[8][8];
-        for (int k = 0; k < m; k++) {
-            float3 c = make_float3(0.5f * (clo[k].x + chi[k].x) - pc.x, 0.5f * (clo[k].y + chi[k].y) - pc.y,
-                                   0.5f * (clo[k].z + chi[k].z) - pc.z);
-            for (int s = 0; s < 8; s++)
-                score[k][s] = ((s & 1) ? c.x : -c.x) + ((s & 2) ? c.y : -c.y) + ((s & 4) ? c.z : -c.z);
+        // child k = the k-th owner: its box, kind and triangles
+        const uint32_t owners = ballot8(h != kNone);
+        const int m = __popc(owners);
+        const bool has = l < m;
+        if (h != kNone) s_at[threadIdx.x - l + __popc(owners & ((1u << l) - 1u))] = (uint8_t)l;
+        __syncwarp();
+        h = __shfl_sync(kFull, h, shift + (has ? s_at[threadIdx.x] : 0));
+        float3 clo = make_float3(FLT_MAX, FLT_MAX, FLT_MAX), chi = make_float3(-FLT_MAX, -FLT_MAX, -FLT_MAX);
+        bool node = false;
+        int n_tris = 0;
+        if (has) {
+            child_box(h, sorted_tri, tlo, thi, nlo, nhi, clo, chi);
+            node = is_node_root(h, dpd);
+            n_tris = node ? 0 : child_count(h, cnt);
         }
-        uint32_t used_slots = 0, used_kids = 0;
-        for (int it = 0; it < m; it++) {
-            float best = -FLT_MAX;
-            int bk = -1, bs = -1;
-            for (int k = 0; k < m; k++) {
-                if (used_kids & (1u << k)) continue;
-                for (int s = 0; s < 8; s++) {
-                    if (used_slots & (1u << s)) continue;
-                    if (score[k][s] > best || bk < 0) { best = score[k][s]; bk = k; bs = s; }
+        const float3 plo = make_float3(min8(clo.x), min8(clo.y), min8(clo.z));
+        const float3 phi = make_float3(-min8(-chi.x), -min8(-chi.y), -min8(-chi.z));
+
+        // Slots: slot s is the corner with bit k set = positive along axis k.
+        // The best remaining (child, slot) pair takes its slot, the first in
+        // (child, slot) order of equal ones.
+        int slot = -1;
+        {
+            const float3 pc = make_float3(0.5f * (plo.x + phi.x), 0.5f * (plo.y + phi.y), 0.5f * (plo.z + phi.z));
+            const float3 c = make_float3(0.5f * (clo.x + chi.x) - pc.x, 0.5f * (clo.y + chi.y) - pc.y,
+                                         0.5f * (clo.z + chi.z) - pc.z);
+            uint32_t used = 0;
+            for (int it = 0; it < 8; it++) {
+                // 0 = no candidate; a NaN score ranks below every other
+                uint32_t best = 0;
+                int bs = 0;
+                if (has && slot < 0) {
+#pragma unroll
+                    for (int s = 0; s < 8; s++) {
+                        if (used >> s & 1u) continue;
+                        // (+ 0 turns -0 into +0, which compare equal)
+                        const float score = ((s & 1) ? c.x : -c.x) + ((s & 2) ? c.y : -c.y) + ((s & 4) ? c.z : -c.z) + 0.f;
+                        const uint32_t key = score == score ? max(float_flip(score), 2u) : 1u;
+                        if (key > best) { best = key; bs = s; }
+                    }
                 }
+                uint32_t top = best;
+                for (int o = 1; o < 8; o <<= 1) top = max(top, __shfl_xor_sync(kFull, top, o));
+                const uint32_t winners = ballot8(best == top && top != 0u);
+                const int who = winners ? __ffs(winners) - 1 : 0;
+                const int ws = __shfl_sync(kFull, bs, shift + who);
+                if (winners) used |= 1u << ws;
+                if (winners && l == who) slot = ws;
+                if (!__any_sync(kFull, winners != 0u)) break;
             }
-            used_kids |= 1u << bk;
-            used_slots |= 1u << bs;
-            slot_of[bk] = bs;
         }
-    }
 
-    // allocate children and triangle records
-    uint32_t child_base = 0, tri_base = 0;
-    if (n_int) {
-        child_base = atomicAdd(node_count, (uint32_t)n_int);
-        if (child_base + n_int > node_cap) { atomicOr(err, 2u); return; }
-    }
-    if (n_leaf_tris) {
-        tri_base = atomicAdd(tri_count, (uint32_t)n_leaf_tris);
-        if (tri_base + n_leaf_tris > tri_cap) { atomicOr(err, 4u); return; }
-    }
+        // node and triangle records: one allocation a group
+        const uint32_t n_int = __popc(ballot8(node)), n_leaf = sum8((uint32_t)n_tris);
+        uint32_t child_base = 0, tri_base = 0, queue = 0;
+        if (live && l == 0 && n_int) child_base = atomicAdd(node_count, n_int);
+        if (live && l == 1 && n_leaf) tri_base = atomicAdd(tri_count, n_leaf);
+        if (live && l == 2 && n_int) queue = atomicAdd(out_count, n_int);
+        child_base = __shfl_sync(kFull, child_base, shift);
+        tri_base = __shfl_sync(kFull, tri_base, shift + 1);
+        queue = __shfl_sync(kFull, queue, shift + 2);
+        const uint32_t full = (child_base + n_int > node_cap ? 2u : 0u) | (tri_base + n_leaf > tri_cap ? 4u : 0u) |
+                              (queue + n_int > out_cap ? 8u : 0u);
+        if (full && live && l == 0) atomicOr(err, full);
+        const bool write = live && !full;
 
-    // quantisation frame
-    int ex = quant_exp(phi.x - plo.x, min_step), ey = quant_exp(phi.y - plo.y, min_step),
-        ez = quant_exp(phi.z - plo.z, min_step);
-    float sx = exp2i(ex), sy = exp2i(ey), sz = exp2i(ez);
-    // origin one step below the union so that floor() never goes negative
-    float3 org = make_float3(plo.x - sx, plo.y - sy, plo.z - sz);
+        // quantisation frame: origin one step below the union so that
+        // floor() never goes negative
+        const int ex = quant_exp(phi.x - plo.x, min_step), ey = quant_exp(phi.y - plo.y, min_step),
+                  ez = quant_exp(phi.z - plo.z, min_step);
+        const float sx = exp2i(ex), sy = exp2i(ey), sz = exp2i(ez);
+        const float3 org = make_float3(plo.x - sx, plo.y - sy, plo.z - sz);
 
-    uint8_t qlx[8], qly[8], qlz[8], qhx[8], qhy[8], qhz[8];
-    for (int s = 0; s < 8; s++) qlx[s] = qly[s] = qlz[s] = qhx[s] = qhy[s] = qhz[s] = 0;
-    uint32_t slots = 0;
-
-    // internal children in slot order -> contiguous child nodes
-    uint32_t imask = 0;
-    for (int k = 0; k < m; k++)
-        if (is_node_root(ch[k], dpd)) imask |= 1u << slot_of[k];
-    int tri_off = 0;
-    for (int s = 0; s < 8; s++) {
-        int k = -1;
-        for (int q = 0; q < m; q++)
-            if (slot_of[q] == s) k = q;
-        if (k < 0) continue;
-        // conservative 8-bit box: floor/ceil in double (exact for float inputs),
-        // one extra step of slack each side
-        double lx = floor(((double)clo[k].x - org.x) / sx) - 1, ly = floor(((double)clo[k].y - org.y) / sy) - 1,
-               lz = floor(((double)clo[k].z - org.z) / sz) - 1;
-        double hx = ceil(((double)chi[k].x - org.x) / sx) + 1, hy = ceil(((double)chi[k].y - org.y) / sy) + 1,
-               hz = ceil(((double)chi[k].z - org.z) / sz) + 1;
-        qlx[s] = (uint8_t)fmin(fmax(lx, 0.0), 255.0);
-        qly[s] = (uint8_t)fmin(fmax(ly, 0.0), 255.0);
-        qlz[s] = (uint8_t)fmin(fmax(lz, 0.0), 255.0);
-        qhx[s] = (uint8_t)fmin(fmax(hx, 0.0), 255.0);
-        qhy[s] = (uint8_t)fmin(fmax(hy, 0.0), 255.0);
-        qhz[s] = (uint8_t)fmin(fmax(hz, 0.0), 255.0);
-        if (imask & (1u << s)) {
-            slots |= 8u << (4 * s);
-            uint32_t ci = child_base + __popc(imask & ((1u << s) - 1u));
-            uint32_t slot = atomicAdd(out_count, 1u);
-            if (slot >= out_cap) { atomicOr(err, 8u); continue; }
-            out[slot] = Work{ch[k], ci};
-        } else {
-            int pos_of[kLeafMax];
-            const int nt = leaf_tris(ch[k], child, pos_of);
-            slots |= ((1u << nt) - 1u) << (4 * s);
-            for (int q = 0; q < nt; q++) {
-                uint32_t t = sorted_tri[pos_of[q]];
-                uint32_t a = idx[3 * t], b = idx[3 * t + 1], c = idx[3 * t + 2];
-                float v0x = pos[3 * a], v0y = pos[3 * a + 1], v0z = pos[3 * a + 2];
-                float e1x = __fsub_rn(pos[3 * b], v0x), e1y = __fsub_rn(pos[3 * b + 1], v0y),
-                      e1z = __fsub_rn(pos[3 * b + 2], v0z);
-                float e2x = __fsub_rn(pos[3 * c], v0x), e2y = __fsub_rn(pos[3 * c + 1], v0y),
-                      e2z = __fsub_rn(pos[3 * c + 2], v0z);
-                float nx = __fsub_rn(__fmul_rn(e1y, e2z), __fmul_rn(e1z, e2y));
-                float ny = __fsub_rn(__fmul_rn(e1z, e2x), __fmul_rn(e1x, e2z));
-                float nz = __fsub_rn(__fmul_rn(e1x, e2y), __fmul_rn(e1y, e2x));
-                Tri tr;
-                tr.a = make_float4(v0x, v0y, v0z, nx);
-                tr.b = make_float4(e1x, e1y, e1z, ny);
-                tr.c = make_float4(e2x, e2y, e2z, nz);
-                tr.id = make_uint4(t, 0u, 0u, 0u);
-                tris[tri_base + tri_off + q] = tr;
+        // lane s: the child in slot s
+        __syncwarp();
+        s_at[threadIdx.x] = 0xff;
+        __syncwarp();
+        if (slot >= 0) s_at[threadIdx.x - l + slot] = (uint8_t)l;
+        __syncwarp();
+        const uint32_t k = s_at[threadIdx.x];
+        const bool filled = k != 0xffu;
+        const int from = shift + (filled ? (int)k : l);
+        h = __shfl_sync(kFull, h, from);
+        node = __shfl_sync(kFull, (int)node, from) && filled;
+        n_tris = __shfl_sync(kFull, n_tris, from);
+        if (!filled) n_tris = 0;
+        clo = make_float3(__shfl_sync(kFull, clo.x, from), __shfl_sync(kFull, clo.y, from), __shfl_sync(kFull, clo.z, from));
+        chi = make_float3(__shfl_sync(kFull, chi.x, from), __shfl_sync(kFull, chi.y, from), __shfl_sync(kFull, chi.z, from));
+        const uint32_t inner = ballot8(node);
+        uint32_t tri_off = (uint32_t)n_tris;  // inclusive prefix sum over the slots
+        for (int o = 1; o < 8; o <<= 1) {
+            const uint32_t up = __shfl_up_sync(kFull, tri_off, o, 8);
+            if (l >= o) tri_off += up;
+        }
+        tri_off -= (uint32_t)n_tris;
+        // conservative 8-bit box: floor/ceil in double (exact for float
+        // inputs), one extra step of slack each side
+        auto low = [&](float v, float o, float s) {
+            return filled ? (uint8_t)fmin(fmax(floor(((double)v - o) / s) - 1, 0.0), 255.0) : (uint8_t)0;
+        };
+        auto high = [&](float v, float o, float s) {
+            return filled ? (uint8_t)fmin(fmax(ceil(((double)v - o) / s) + 1, 0.0), 255.0) : (uint8_t)0;
+        };
+        planes[l] = low(clo.x, org.x, sx);
+        planes[8 + l] = high(chi.x, org.x, sx);
+        planes[16 + l] = low(clo.y, org.y, sy);
+        planes[24 + l] = high(chi.y, org.y, sy);
+        planes[32 + l] = low(clo.z, org.z, sz);
+        planes[40 + l] = high(chi.z, org.z, sz);
+        const uint32_t slots = sum8((node ? 8u : (1u << n_tris) - 1u) << (4 * l));
+        __syncwarp();
+        if (write && l < 6) {
+            uint4 q;
+            if (l == 0) {
+                q = make_uint4(__float_as_uint(org.x), __float_as_uint(org.y), __float_as_uint(org.z), child_base);
+            } else if (l == 1) {
+                q = make_uint4((uint32_t)(ex + 127) << 23, (uint32_t)(ey + 127) << 23, (uint32_t)(ez + 127) << 23,
+                               tri_base);
+            } else if (l == 5) {
+                q = make_uint4(slots, 0u, 0u, 0u);
+            } else {
+                const uint32_t *b = s_planes[group] + 4 * (l - 2);
+                q = make_uint4(b[0], b[1], b[2], b[3]);
             }
-            tri_off += nt;
+            nodes[job.node].q[l] = q;
         }
+        if (write && node) {
+            const uint32_t nth = __popc(inner & ((1u << l) - 1u));
+            out[queue + nth] = Work{h, child_base + nth};
+        }
+        if (write && n_tris) {
+            int at[kLeafMax];
+            leaf_tris(h, child, at);
+#pragma unroll
+            for (int q = 0; q < kLeafMax; q++)
+                if (q < n_tris) write_tri(tris + tri_base + tri_off + q, sorted_tri[at[q]], pos, idx);
+        }
+        __syncwarp();  // the planes are read before the next item's are written
     }
-
-    auto pack4 = [](const uint8_t *b) {
-        return (uint32_t)b[0] | ((uint32_t)b[1] << 8) | ((uint32_t)b[2] << 16) | ((uint32_t)b[3] << 24);
-    };
-    Node8 nd;
-    nd.q[0] = make_uint4(__float_as_uint(org.x), __float_as_uint(org.y), __float_as_uint(org.z), child_base);
-    nd.q[1] = make_uint4((uint32_t)(ex + 127) << 23, (uint32_t)(ey + 127) << 23, (uint32_t)(ez + 127) << 23, tri_base);
-    nd.q[2] = make_uint4(pack4(qlx), pack4(qlx + 4), pack4(qhx), pack4(qhx + 4));
-    nd.q[3] = make_uint4(pack4(qly), pack4(qly + 4), pack4(qhy), pack4(qhy + 4));
-    nd.q[4] = make_uint4(pack4(qlz), pack4(qlz + 4), pack4(qhz), pack4(qhz + 4));
-    nd.q[5] = make_uint4(slots, 0u, 0u, 0u);
-    nodes[job.node] = nd;
 }
 
-__global__ void k_root(Work *q, uint32_t *count, int n, uint32_t *node_count)
+__global__ void k_root(Work *q, int n, uint32_t *counters)
 {
     q[0] = Work{n > 1 ? 0 : ~0, 0u};
-    *count = 1;
-    *node_count = 1;
+    counters[0] = 1;  // the root node
+    counters[4] = 1;  // level 0's work item
 }
 
 inline uint32_t div_up(uint64_t a, uint32_t b) { return (uint32_t)((a + b - 1) / b); }
@@ -803,11 +946,9 @@ int bvh_build(BuildBuffers &B, const float *d_pos, uint32_t n_verts, const uint3
     const uint32_t node_cap = n;           // 8-wide nodes never exceed the triangle count
     const uint32_t tri_cap = n;
     const uint32_t queue_cap = n + 1;
-    ILG_CK(B.reserve(n, sort_tmp, node_cap, queue_cap, st));
+    ILG_CK(B.reserve(n, sort_tmp, node_cap, queue_cap));
 
-    ILG_CK(cudaMemsetAsync(B.err, 0, sizeof(uint32_t), st));
-    uint32_t init[6] = {0xffffffffu, 0xffffffffu, 0xffffffffu, 0u, 0u, 0u};
-    ILG_CK(cudaMemcpyAsync(B.cbounds, init, sizeof(init), cudaMemcpyHostToDevice, st));
+    ILG_CK(cudaMemsetAsync(B.counters, 0, BuildBuffers::kCounters * sizeof(uint32_t), st));
     const uint32_t T = 256;
     k_tri_bounds<<<div_up(n, T), T, 0, st>>>(d_pos, n_verts, d_idx, n, B.tlo, B.thi, B.cbounds, B.err);
     k_morton<<<div_up(n, T), T, 0, st>>>(B.tlo, B.thi, n, B.cbounds, B.keys, B.vals);
@@ -815,58 +956,54 @@ int bvh_build(BuildBuffers &B, const float *d_pos, uint32_t n_verts, const uint3
     ILG_CK(cub::DeviceRadixSort::SortPairs(B.sort_tmp, sort_tmp, B.keys, B.keys_alt, B.vals, B.vals_alt, (int)n, 0,
                                            30, st));
     if (n > 1) {
-        k_karras<<<div_up(n - 1, T), T, 0, st>>>(B.keys_alt, (int)n, B.child, B.parent_int, B.parent_leaf, B.range);
+        k_karras<<<div_up(n - 1, T), T, 0, st>>>(B.keys_alt, (int)n, B.child, B.parent_int, B.parent_leaf);
         ILG_CK(cudaMemsetAsync(B.arrivals, 0, sizeof(uint32_t) * (n - 1), st));
-        k_refit<<<div_up(n, T), T, 0, st>>>((int)n, B.vals_alt, B.tlo, B.thi, B.child, B.parent_int, B.parent_leaf,
-                                             B.arrivals, B.nlo, B.nhi);
-        ILG_CK(cudaGetLastError());
-        if (res.treelets) {
-            static const SubsetTable table = make_subset_table();
-            ILG_CK(cudaMemcpyToSymbolAsync(c_subsets, &table, sizeof(table), 0, cudaMemcpyHostToDevice, st));
-        }
+        // Leaves a warp starts from: it rebuilds the treelets of its lanes
+        // one after another, so small meshes take fewer, for shorter chains
+        // on more SMs; enough warps to fill the GPU anyway take all 32 (1 M
+        // triangles: 4 leaves 4.4 ms, 8 3.8, 16 3.4, 32 3.2 for the build).
+        int leaves = 32;
+        while (leaves > 4 && n / (uint32_t)leaves < (uint32_t)current_sm_count() * 24u) leaves /= 2;
+        const uint32_t tblocks = div_up(n, kTreeletWarps * (uint32_t)leaves);
         for (int pass = 0; pass < (res.treelets ? kTreeletPasses : 1); pass++) {
-            ILG_CK(cudaMemsetAsync(B.arrivals, 0, sizeof(uint32_t) * (n - 1), st));
-            k_treelet<<<div_up(n, kTreeletThreads), kTreeletThreads, 0, st>>>((int)n, B.vals_alt, B.tlo, B.thi, B.child, B.parent_int,
-                                                      B.parent_leaf, B.arrivals, B.nlo, B.nhi, B.cnt, B.cost,
-                                                      res.treelets ? 1 : 0);
+            (pass == 0 ? k_treelet<true> : k_treelet<false>)<<<tblocks, kTreeletThreads, 0, st>>>(
+                (int)n, B.vals_alt, B.tlo, B.thi, B.child, B.parent_int, B.parent_leaf, B.arrivals, B.nlo, B.nhi,
+                B.cnt, B.cost, res.treelets ? 1 : 0, leaves);
             ILG_CK(cudaGetLastError());
         }
-        ILG_CK(cudaMemsetAsync(B.arrivals, 0, sizeof(uint32_t) * (n - 1), st));
         k_collapse_cost<<<div_up(n, 128), 128, 0, st>>>((int)n, B.vals_alt, B.tlo, B.thi, B.child, B.parent_int,
                                                         B.parent_leaf, B.arrivals, B.nlo, B.nhi, B.cnt, B.dpc, B.dpd);
         ILG_CK(cudaGetLastError());
     }
-    ILG_CK(cudaMemsetAsync(B.counters, 0, 4 * sizeof(uint32_t), st));
-    // counters: [0] node_count, [1] tri_count, [2] queue A count, [3] queue B count
-    k_root<<<1, 1, 0, st>>>((Work *)B.qa_raw, B.counters + 2, (int)n, B.counters + 0);
+    k_root<<<1, 1, 0, st>>>((Work *)B.qa_raw, (int)n, B.counters);
     ILG_CK(cudaGetLastError());
 
+    // Levels go to the stream kLevelBatch at a time (a tree of a few million
+    // triangles has 7 to 10), each over as many items as the previous one
+    // made; the host looks at the counters once a batch.
+    constexpr int kLevelBatch = 12;
     const float min_step = res.min_step;
     Work *qin = (Work *)B.qa_raw, *qout = (Work *)B.qb_raw;
-    uint32_t *cin = B.counters + 2, *cout = B.counters + 3;
-    uint32_t host_in = 1;
-    uint32_t depth = 0;
-    while (host_in > 0) {
-        ILG_CK(cudaMemsetAsync(cout, 0, sizeof(uint32_t), st));
-        k_collapse<<<div_up(host_in, 64), 64, 0, st>>>(qin, cin, qout, cout, queue_cap, B.child, B.cnt, B.dpd, B.nlo,
-                                                        B.nhi, B.vals_alt, B.tlo, B.thi, d_pos, d_idx, B.nodes,
-                                                        B.counters + 0, node_cap, B.tris, B.counters + 1,
-                                                        tri_cap, min_step, B.err);
+    const uint32_t blocks = std::min<uint32_t>(div_up(n, kCollapseThreads / 8), (uint32_t)current_sm_count() * 16u);
+    uint32_t h[BuildBuffers::kCounters];
+    for (int level = 0;;) {
+        for (int k = 0; k < kLevelBatch && level < kMaxLevels; k++, level++) {
+            k_collapse<<<blocks, kCollapseThreads, 0, st>>>(qin, B.counters + 4 + level, qout, B.counters + 5 + level, queue_cap,
+                                              B.child, B.cnt, B.dpd, B.nlo, B.nhi, B.vals_alt, B.tlo, B.thi, d_pos,
+                                              d_idx, B.nodes, B.counters + 0, node_cap, B.tris, B.counters + 1,
+                                              tri_cap, min_step, B.counters + 2, B.err);
+            std::swap(qin, qout);
+        }
         ILG_CK(cudaGetLastError());
-        ILG_CK(cudaMemcpyAsync(&host_in, cout, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
+        ILG_CK(cudaMemcpyAsync(h, B.counters, sizeof(h), cudaMemcpyDeviceToHost, st));
         ILG_CK(cudaStreamSynchronize(st));
-        depth++;
-        if (depth > 200) {
+        if (h[4 + level] == 0) break;
+        if (level >= kMaxLevels) {
             snprintf(err, err_len, "ilg_build: collapse did not converge");
             return 5;
         }
-        std::swap(qin, qout);
-        std::swap(cin, cout);
     }
-    uint32_t h[4], herr = 0;
-    ILG_CK(cudaMemcpyAsync(h, B.counters, sizeof(h), cudaMemcpyDeviceToHost, st));
-    ILG_CK(cudaMemcpyAsync(&herr, B.err, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
-    ILG_CK(cudaStreamSynchronize(st));
+    const uint32_t herr = h[3], depth = h[2];
     if (herr & 1u) {
         snprintf(err, err_len, "ilg_build: triangle index out of range of the vertex array");
         return 1;

@@ -68,9 +68,9 @@ typedef struct ilg_opts {
 } ilg_opts;
 
 /* ilg_opts.build_flags. By default ilg_build restructures the Morton tree by
- * treelets for least SAH cost (two passes; about 12 ms at 1 M triangles and
- * 0.1-0.4 s at 21 M on a B200, for 15-25 % faster traversal); ILG_BUILD_FAST
- * skips that step (about 9 / 19 ms), for scenes rebuilt often. Both trees
+ * treelets for least SAH cost (two passes; 2.6 ms at 1 M triangles and 44 ms
+ * at 21 M on a B200, for 15-25 % faster traversal); ILG_BUILD_FAST skips that
+ * step (0.8 / 18 ms), for scenes rebuilt often. Both trees
  * give the same hits, up to which of two hits less than 1e-5 apart wins. */
 #define ILG_BUILD_FAST 0x1u
 
