@@ -192,6 +192,21 @@ constexpr int kTreeletLeaves = 7;
 constexpr int kTreeletPasses = 2;
 constexpr float kSahCi = 1.2f, kSahCt = 1.0f;
 
+// Half the surface area of a box, and of a subset of a treelet's leaves. Which
+// of two topologies of almost equal cost wins depends on the last bit, so
+// every rounding of the costs is spelled out here: the tree of a mesh does
+// not change with how the compiler contracts the sums around it.
+__device__ __forceinline__ float box_area(const float3 &lo, const float3 &hi)
+{
+    const float dx = fmaxf(hi.x - lo.x, 0.f), dy = fmaxf(hi.y - lo.y, 0.f), dz = fmaxf(hi.z - lo.z, 0.f);
+    return fmaf(dz, dx, fmaf(dx, dy, __fmul_rn(dy, dz)));
+}
+__device__ __forceinline__ float subset_area(const float3 &lo, const float3 &hi)
+{
+    const float dx = fmaxf(hi.x - lo.x, 0.f), dy = fmaxf(hi.y - lo.y, 0.f), dz = fmaxf(hi.z - lo.z, 0.f);
+    return fmaf(dz, dx, fmaf(dy, dz, __fmul_rn(dx, dy)));
+}
+
 // Arrives at a binary node; true for the second of its two arrivals, which
 // sees everything written before the first. The counter wraps back to 0 for
 // the next pass. (One acquire-release atomic: with a full fence on either
@@ -295,7 +310,7 @@ __device__ void treelet_warp(int p, float areap, const uint32_t *sorted_tri, con
     auto take = [&](int handle) {  // this lane's leaf
         h = handle;
         handle_box(h, sorted_tri, tlo, thi, nlo, nhi, lo, hi);
-        a = area(lo, hi);
+        a = box_area(lo, hi);
         count = h >= 0 ? __ldcg(&cnt[h]) : 1;
         c = h >= 0 ? __ldcg(&cost[h]) : kSahCt * a;
     };
@@ -311,7 +326,7 @@ __device__ void treelet_warp(int p, float areap, const uint32_t *sorted_tri, con
         const int w = __ffs(__ballot_sync(kFull, key == best)) - 1;
         const int open = __shfl_sync(kFull, h, w);
         if (lane == n_l - 1) inner = open;
-        cur += kSahCi * __uint_as_float(best - 1u);
+        cur = fmaf(kSahCi, __uint_as_float(best - 1u), cur);
         kids = __ldcg(&child[open]);
         if (lane == w || lane == n_l) take(lane == w ? kids.x : kids.y);
     }
@@ -341,7 +356,7 @@ __device__ void treelet_warp(int p, float areap, const uint32_t *sorted_tri, con
             float3 l2 = l, u2 = u;
             if (j & 1) join(l2, u2, 5);
             if (j & 2) join(l2, u2, 6);
-            s.area[lane + 32 * j] = area(l2, u2);
+            s.area[lane + 32 * j] = subset_area(l2, u2);
         }
     }
     __syncwarp();
@@ -357,7 +372,7 @@ __device__ void treelet_warp(int p, float areap, const uint32_t *sorted_tri, con
                 if (cc < best) { best = cc; bq = Q; }
                 if (Q == 0) break;
             }
-            s.copt[S] = kSahCi * s.area[S] + best;
+            s.copt[S] = fmaf(kSahCi, s.area[S], best);
             s.split[S] = (uint8_t)(low | bq);
         }
         __syncwarp();
@@ -375,7 +390,7 @@ __device__ void treelet_warp(int p, float areap, const uint32_t *sorted_tri, con
         }
         best_split(group, best, bq);
         if ((lane & 3) == 0) {
-            s.copt[S] = kSahCi * s.area[S] + best;
+            s.copt[S] = fmaf(kSahCi, s.area[S], best);
             s.split[S] = (uint8_t)(low | bq);
         }
     }
@@ -393,7 +408,7 @@ __device__ void treelet_warp(int p, float areap, const uint32_t *sorted_tri, con
             if (cc < best) { best = cc; bq = Q; }
         }
         best_split(kFull, best, bq);
-        all = kSahCi * s.area[kAll] + best;
+        all = fmaf(kSahCi, s.area[kAll], best);
         if (lane == 0) {
             s.copt[kAll] = all;
             s.split[kAll] = (uint8_t)(1 | bq);
@@ -491,7 +506,7 @@ __global__ void __launch_bounds__(kTreeletThreads) k_treelet(int n, const uint32
                             plo = make_float3(fminf(plo.x, lo.x), fminf(plo.y, lo.y), fminf(plo.z, lo.z));
                             phi = make_float3(fmaxf(phi.x, hi.x), fmaxf(phi.y, hi.y), fmaxf(phi.z, hi.z));
                         }
-                        part[q] = kSahCt * area(lo, hi);
+                        part[q] = kSahCt * box_area(lo, hi);
                     }
                     if (h >= 0) part[q] = __ldcg(&cost[h]);
                     cp += h >= 0 ? __ldcg(&cnt[h]) : 1;
@@ -502,9 +517,9 @@ __global__ void __launch_bounds__(kTreeletThreads) k_treelet(int n, const uint32
                 } else {
                     handle_box(p, sorted_tri, tlo, thi, nlo, nhi, plo, phi);
                 }
-                ap = area(plo, phi);
+                ap = box_area(plo, phi);
                 __stcg(&cnt[p], cp);
-                __stcg(&cost[p], kSahCi * ap + part[0] + part[1]);
+                __stcg(&cost[p], __fadd_rn(fmaf(kSahCi, ap, part[0]), part[1]));
                 ready = restructure && cp >= kTreeletLeaves;
             }
         }
