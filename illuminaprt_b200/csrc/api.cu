@@ -1020,8 +1020,10 @@ static int prepare_scene(ilg_ctx *runner, ilg_ctx *ctx, const ilg_camera_frame &
     return ILG_OK;
 }
 
-// Renders the scenes of `recs` (path ranges and pixel bases filled here) in
-// waves of at most `cap_req` paths on the runner's buffers and stream.
+// Renders the scenes of `recs` (path ranges and pixel bases filled here) on
+// the runner's buffers and stream: as one persistent launch (one_launch), or
+// in waves of at most `cap_req` paths (0 = automatic) with `block` threads a
+// block (0 = 128).
 static int run_render(ilg_ctx *ctx, std::vector<SceneRec> &recs, uint32_t cap_req, uint32_t block,
                       uint32_t cache_depth, uint32_t train_every, uint32_t train_steps, uint32_t train_batch,
                       uint64_t *total_paths_out, bool aux = false, bool count = false, uint32_t train_tail = 0,
@@ -1030,6 +1032,7 @@ static int run_render(ilg_ctx *ctx, std::vector<SceneRec> &recs, uint32_t cap_re
     if (one_launch && (cache_depth || aux || count))
         return fail(ctx, ILG_EINVAL,
                     "render: ILG_RENDER_PERSISTENT renders plain images only (no cache, Direct / Albedo or counts)");
+    if (block == 0) block = 128;
     cudaStream_t st = ctx->stream;
     uint64_t total = 0, pixels64 = 0;
     uint32_t pixels = 0, depth_max = 0, nl = 1;
@@ -1055,11 +1058,13 @@ static int run_render(ilg_ctx *ctx, std::vector<SceneRec> &recs, uint32_t cap_re
     } else {
         cap = (uint32_t)std::min<uint64_t>(cap, total);
     }
-    CK(ctx->q_o0.reserve(cap)); CK(ctx->q_d0.reserve(cap)); CK(ctx->q_o1.reserve(cap)); CK(ctx->q_d1.reserve(cap));
-    CK(ctx->q_p0.reserve(cap)); CK(ctx->q_p1.reserve(cap)); CK(ctx->beta.reserve(cap));
-    CK(ctx->hit_tri.reserve(cap)); CK(ctx->hit_t.reserve(cap)); CK(ctx->path_scene.reserve(cap));
-    CK(ctx->s_o.reserve((size_t)cap * nl)); CK(ctx->s_d.reserve((size_t)cap * nl)); CK(ctx->s_c.reserve((size_t)cap * nl));
-    CK(ctx->s_sid.reserve((size_t)cap * nl));
+    if (!one_launch) {
+        CK(ctx->q_o0.reserve(cap)); CK(ctx->q_d0.reserve(cap)); CK(ctx->q_o1.reserve(cap)); CK(ctx->q_d1.reserve(cap));
+        CK(ctx->q_p0.reserve(cap)); CK(ctx->q_p1.reserve(cap)); CK(ctx->beta.reserve(cap));
+        CK(ctx->hit_tri.reserve(cap)); CK(ctx->hit_t.reserve(cap)); CK(ctx->path_scene.reserve(cap));
+        CK(ctx->s_o.reserve((size_t)cap * nl)); CK(ctx->s_d.reserve((size_t)cap * nl)); CK(ctx->s_c.reserve((size_t)cap * nl));
+        CK(ctx->s_sid.reserve((size_t)cap * nl));
+    }
     CK(ctx->counts.reserve(9)); CK(ctx->accum.reserve((size_t)pixels + 1));
     CK(ctx->scene_table.reserve(recs.size()));
     CK(cudaMemcpyAsync(ctx->scene_table.ptr, recs.data(), recs.size() * sizeof(SceneRec), cudaMemcpyHostToDevice, st));
@@ -1144,6 +1149,14 @@ static int run_render(ilg_ctx *ctx, std::vector<SceneRec> &recs, uint32_t cap_re
         mlp = ctx->mlp_view();
     }
 
+    if (one_launch) {
+        size_t bytes = 0;
+        CK(render_persistent_bytes(R, total, nl, bytes));
+        const size_t had = ctx->persist_pool.cap;
+        CK(ctx->persist_next.reserve(1));
+        CK(ctx->persist_pool.reserve(bytes));
+        if (ctx->persist_pool.cap != had) ctx->drop_graph();  // the graph holds the pool's address
+    }
 
     // The frame (every wave, every bounce) is one CUDA graph. Nothing in it
     // depends on the host between launches (queue counts stay on the device),
@@ -1159,11 +1172,10 @@ static int run_render(ilg_ctx *ctx, std::vector<SceneRec> &recs, uint32_t cap_re
     }
     if (!ctx->graph_exec || ctx->graph_key.size() != sizeof(key) || memcmp(ctx->graph_key.data(), key, sizeof(key))) {
         ctx->drop_graph();
-        if (one_launch) CK(ctx->persist_next.reserve(1));
         CK(cudaStreamBeginCapture(st, cudaStreamCaptureModeRelaxed));
         cudaError_t ce = cudaSuccess;
         if (one_launch) {
-            ce = render_persistent(R, total, ctx->persist_next.ptr, &launches, st);
+            ce = render_persistent(R, total, nl, ctx->persist_next.ptr, ctx->persist_pool.ptr, &launches, st);
         } else {
             for (uint64_t g0 = 0; g0 < total && ce == cudaSuccess; g0 += cap) {
                 const uint32_t k = (uint32_t)std::min<uint64_t>(cap, total - g0);
@@ -1247,7 +1259,7 @@ int render_one(ilg_ctx *ctx, const ilg_camera_frame &frame, const ilg_render_opt
     recs[0].ray_d = ray_d;
     const uint32_t wh = recs[0].wh;
     const bool aux = direct_rgb || albedo_rgb;
-    rc = run_render(ctx, recs, opts->paths_per_wave, 128, cache_depth, opts->train_every ? opts->train_every : 16u,
+    rc = run_render(ctx, recs, opts->paths_per_wave, 0, cache_depth, opts->train_every ? opts->train_every : 16u,
                     opts->train_steps, opts->train_batch ? opts->train_batch : 16384u, nullptr, aux,
                     ctx->counted, opts->train_tail, opts->train_epochs ? opts->train_epochs : 1u, hash_cache,
                     (flags & ILG_RENDER_PERSISTENT) != 0);
@@ -1392,7 +1404,7 @@ int ilg_render_batch(ilg_ctx *runner, const ilg_batch_item *items, uint32_t n, u
         if (rc) return rc;
     }
     runner->counted = (flags & ILG_RENDER_COUNT) != 0;
-    int rc = run_render(runner, recs, paths_per_wave, block ? block : 128, 0, 16, 0, 16384, nullptr, false,
+    int rc = run_render(runner, recs, paths_per_wave, block, 0, 16, 0, 16384, nullptr, false,
                         runner->counted, 0, 1, false, (flags & ILG_RENDER_PERSISTENT) != 0);
     if (rc) return rc;
     uint32_t max_wh = 0;

@@ -106,6 +106,7 @@ struct ilg_ctx {
     ilg::DevBuf<unsigned long long> render_stats;
     // path counter of the one-launch renderer (ILG_RENDER_PERSISTENT)
     ilg::DevBuf<unsigned long long> persist_next;
+    ilg::DevBuf<unsigned char> persist_pool;  // its warps' paths and rays
     bool counted = false;
     // the last frame's instantiated CUDA graph and the launch configuration it was captured for
     cudaGraphExec_t graph_exec = nullptr;
@@ -170,7 +171,7 @@ struct ilg_ctx {
         drop_graph();
         pos.release(); idx.release(); mat.release();
         bb.release_all();
-        raw_tris.release(); raw_ready = false; render_stats.release(); persist_next.release();
+        raw_tris.release(); raw_ready = false; render_stats.release(); persist_next.release(); persist_pool.release();
         post_acc.release(); post_in.release(); post_out.release(); post_scratch.release();
         post_pixels = post_frames = 0;
         ro.release(); rd.release(); hprim.release(); ht.release(); hu.release(); hv.release(); hocc.release();

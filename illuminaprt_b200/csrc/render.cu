@@ -99,10 +99,7 @@ __device__ __forceinline__ uint32_t push_slot(bool want, uint32_t *count)
 
 __device__ __forceinline__ void add_pixel(float4 *accum, uint32_t pixel, float3 c)
 {
-    float *a = reinterpret_cast<float *>(accum + pixel);
-    atomicAdd(a, c.x);
-    atomicAdd(a + 1, c.y);
-    atomicAdd(a + 2, c.z);
+    atomicAdd(accum + pixel, make_float4(c.x, c.y, c.z, 0.f));  // one vector reduction
 }
 
 // scene of a global path index (the scenes' path ranges are consecutive)
@@ -125,11 +122,40 @@ __device__ __forceinline__ void path_ident(const SceneRec &S, uint64_t g, uint32
                                            uint32_t &x, uint32_t &y)
 {
     const uint64_t local = g - S.path_begin;
-    const uint64_t sample = local / S.wh;
-    pixel = (uint32_t)(local - sample * S.wh);
+    uint64_t sample;
+    if (local >> 32) {
+        sample = local / S.wh;
+        pixel = (uint32_t)(local - sample * S.wh);
+    } else {  // (a 64-bit division is some 100 instructions)
+        const uint32_t s = (uint32_t)local / S.wh;
+        sample = s;
+        pixel = (uint32_t)local - s * S.wh;
+    }
     x = S.region_x + pixel % S.region_w;
     y = S.region_y + pixel / S.region_w;
     key = path_key(S.seed, sample * S.full_wh + (uint64_t)y * S.width + x);
+}
+
+// The first ray of global path g of scene S: the caller's ray
+// (IIntegrator::Radiance(..., ray, ...), whose first intersection uses the
+// ray's own [Min, Max]) or a camera ray.
+__device__ __forceinline__ void first_ray(const SceneRec &S, uint64_t g, uint32_t &pixel, uint64_t &key, float4 &o,
+                                          float4 &d)
+{
+    uint32_t x, y;
+    path_ident(S, g, pixel, key, x, y);
+    if (S.ray_o) {
+        o = S.ray_o[pixel];
+        d = S.ray_d[pixel];
+        return;
+    }
+    // BoxFilter shifts the [0,1) sample by -0.5 (Core/Filter/BoxFilter.cpp:20-28)
+    const float xi1 = rnd(key, kDimCam) - 0.5f, xi2 = rnd(key, kDimCam + 1) - 0.5f;
+    const float fx = x * S.rcp_w + xi1 * S.rcp_w, fy = y * S.rcp_h + xi2 * S.rcp_h;
+    const float3 target = S.corner + S.across * fx + S.up * fy;
+    const float3 dd = normalize3(target - S.centre);
+    o = make_float4(S.centre.x, S.centre.y, S.centre.z, 0.f);
+    d = make_float4(dd.x, dd.y, dd.z, FLT_MAX);
 }
 
 __global__ void k_camera(RenderDev R, uint32_t n_paths, uint64_t wave_begin)
@@ -140,25 +166,11 @@ __global__ void k_camera(RenderDev R, uint32_t n_paths, uint64_t wave_begin)
     const uint64_t g = wave_begin + p;
     const uint32_t sid = scene_of(R, g);
     const SceneRec &S = R.scenes[sid];
-    uint32_t pixel, x, y;
+    uint32_t pixel;
     uint64_t key;
-    path_ident(S, g, pixel, key, x, y);
-    if (S.ray_o) {
-        // a path from the caller's ray (IIntegrator::Radiance(..., ray, ...),
-        // whose first intersection uses the ray's own [Min, Max])
-        R.q_o[0][p] = S.ray_o[pixel];
-        R.q_d[0][p] = S.ray_d[pixel];
-    } else {
-        // BoxFilter shifts the [0,1) sample by -0.5 (Core/Filter/BoxFilter.cpp:20-28)
-        const float xi1 = rnd(key, kDimCam) - 0.5f, xi2 = rnd(key, kDimCam + 1) - 0.5f;
-        const float fx = x * S.rcp_w + xi1 * S.rcp_w, fy = y * S.rcp_h + xi2 * S.rcp_h;
-        const float3 target = S.corner + S.across * fx + S.up * fy;
-        const float3 d = normalize3(target - S.centre);
-        R.q_o[0][p] = make_float4(S.centre.x, S.centre.y, S.centre.z, 0.f);
-        R.q_d[0][p] = make_float4(d.x, d.y, d.z, FLT_MAX);
-    }
+    first_ray(S, g, pixel, key, R.q_o[0][p], R.q_d[0][p]);
     R.q_path[0][p] = p;
-    R.path_scene[p] = sid;
+    if (R.n_scenes > 1u) R.path_scene[p] = sid;
     R.beta[p] = make_float4(1.f, 1.f, 1.f, 0.f);
     if (R.cache_depth) {
         uint32_t slot = 0xffffffffu;
@@ -243,7 +255,7 @@ __global__ void __launch_bounds__(256) k_extend(RenderDev R, int cur)
     unsigned long long nn = 0, nt = 0;
     if (live) {
         const float4 o = R.q_o[cur][i], d = R.q_d[cur][i];
-        const SceneRec &S = R.scenes[R.path_scene[R.q_path[cur][i]]];
+        const SceneRec &S = R.scenes[R.n_scenes > 1u ? R.path_scene[R.q_path[cur][i]] : 0u];
         int best;
         float bt, bu, bv;
         trace_one<false, kStats>(S.nodes, S.tris, S.n_nodes, S.n_tris, o, d, best, bt, bu, bv, R.err, nn, nt);
@@ -476,6 +488,12 @@ __device__ __forceinline__ bool continue_path(const SceneRec &S, uint64_t key, u
     return true;
 }
 
+// kCache: a render with the radiance cache. kOne: a render of one scene (no
+// scene index to load before everything else). The kernel waits on chains of
+// dependent loads (ray -> path -> scene -> hit triangle -> material), so what
+// it needs is warps in flight: the plain one-scene form takes a third fewer
+// registers and two loads less in the chain than the general one.
+template <bool kCache, bool kOne>
 __global__ void __launch_bounds__(256) k_shade(RenderDev R, int cur, uint32_t depth, uint64_t wave_begin)
 {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -493,8 +511,8 @@ __global__ void __launch_bounds__(256) k_shade(RenderDev R, int cur, uint32_t de
 
     if (i < R.count[cur]) {
         path = R.q_path[cur][i];
-        if (R.cache_depth) tslot = R.train_slot[path];
-        sid = R.path_scene[path];
+        if (kCache) tslot = R.train_slot[path];
+        if (!kOne) sid = R.path_scene[path];
         const SceneRec &S = R.scenes[sid];
         const float4 o = R.q_o[cur][i], d = R.q_d[cur][i];
         const int ti = R.hit_tri[i];
@@ -507,7 +525,7 @@ __global__ void __launch_bounds__(256) k_shade(RenderDev R, int cur, uint32_t de
         // samples at that vertex and beyond, escapes after it) only trains the
         // cache and goes to the discard slot past the last pixel.
         const uint32_t image_pixel = pixel;
-        if (R.cache_depth && tslot != 0xffffffffu &&
+        if (kCache && tslot != 0xffffffffu &&
             (ti >= 0 ? depth >= R.cache_depth : depth > R.cache_depth))
             pixel = R.discard_pixel;
         const float4 beta4 = R.beta[path];
@@ -521,7 +539,7 @@ __global__ void __launch_bounds__(256) k_shade(RenderDev R, int cur, uint32_t de
             // the reference's infinite lights, seen by a camera ray or after a
             // specular bounce (PathIntegrator.cpp:84-92 and :194-198)
             if ((depth == 0 || after_specular) && S.inf_escape > 0.f) add = add + beta * S.inf_escape;
-            if (tslot != 0xffffffffu && depth >= 2 && !is_black(add)) credit(R, tslot, depth - 1, add);
+            if (kCache && tslot != 0xffffffffu && depth >= 2 && !is_black(add)) credit(R, tslot, depth - 1, add);
         } else if (depth <= S.max_depth) {
             const Tri tr = S.tris[ti];
             const uint32_t attr = tr.id.y;
@@ -545,7 +563,7 @@ __global__ void __launch_bounds__(256) k_shade(RenderDev R, int cur, uint32_t de
                 dot3(W, wo) > 0.f) {
                 const float3 e = beta * S.lights[light_id].emit;
                 add = add + e;
-                if (tslot != 0xffffffffu && depth >= 2) credit(R, tslot, depth - 1, e);
+                if (kCache && tslot != 0xffffffffu && depth >= 2) credit(R, tslot, depth - 1, e);
             }
             // RadianceContext::Albedo = the first hit's Material::Rho
             // (PathIntegrator.cpp:121): the reflectance; for the GGX conductor
@@ -556,11 +574,11 @@ __global__ void __launch_bounds__(256) k_shade(RenderDev R, int cur, uint32_t de
                           m.kind == 1u ? m.f0 : (m.kind == 3u ? m.albedo + m.f0 : m.albedo));
             const bool specular = m.kind >= 2u;
 
-            const bool at_cache = depth < S.max_depth && R.cache_depth && depth == R.cache_depth;
+            const bool at_cache = kCache && depth < S.max_depth && depth == R.cache_depth;
             // a training path with a short tail stops into the cache too; the
             // cache's answer there completes the targets of its records
             // (self-training), not its pixel
-            const bool at_tail = depth < S.max_depth && R.train_tail && tslot != 0xffffffffu &&
+            const bool at_tail = kCache && depth < S.max_depth && R.train_tail && tslot != 0xffffffffu &&
                                  depth == R.cache_depth + R.train_tail;
             if (at_cache) {
                 // the cache supplies the radiance leaving this vertex to the pixel
@@ -577,7 +595,7 @@ __global__ void __launch_bounds__(256) k_shade(RenderDev R, int cur, uint32_t de
             if ((at_cache && tslot == 0xffffffffu) || at_tail) {
                 // the path stops here
             } else if (depth < S.max_depth) {
-                if (tslot != 0xffffffffu && depth >= 1) {
+                if (kCache && tslot != 0xffffffffu && depth >= 1) {
                     // training record of this vertex; its target fills in as the tail is traced
                     const uint32_t ri = atomicAdd(R.rec_count, 1u);
                     uint32_t stored = 0xffffffffu;
@@ -608,8 +626,8 @@ __global__ void __launch_bounds__(256) k_shade(RenderDev R, int cur, uint32_t de
                             // bit 31 marks a light sample of the first vertex (Direct)
                             const uint32_t tag = (depth == 0 && R.accum_direct) ? 0x80000000u : 0u;
                             R.s_c[s] = make_float4(sc.x, sc.y, sc.z, __uint_as_float(pixel | tag));
-                            R.s_sid[s] = sid;
-                            if (R.cache_depth)
+                            if (!kOne) R.s_sid[s] = sid;
+                            if (kCache)
                                 R.s_meta[s] = tslot == 0xffffffffu ? 0xffffffffu : ((tslot << 8) | depth);
                         } else {
                             atomicOr(R.err, 16u);
@@ -640,7 +658,7 @@ __global__ void __launch_bounds__(256) k_shade(RenderDev R, int cur, uint32_t de
             atomicOr(R.err, 8u);
         }
     }
-    if (R.cache_depth) {
+    if (kCache) {
         const uint32_t q = push_slot(query, R.qry_count);
         if (query) {
             if (q < R.capacity) {
@@ -683,7 +701,7 @@ __global__ void __launch_bounds__(256) k_shadow(RenderDev R)
     int best = -2;
     if (live) {
         const float4 o = R.s_o[i], d = R.s_d[i];
-        const SceneRec &S = R.scenes[R.s_sid[i]];
+        const SceneRec &S = R.scenes[R.n_scenes > 1u ? R.s_sid[i] : 0u];
         float bt, bu, bv;
         trace_one<true, kStats>(S.nodes, S.tris, S.n_nodes, S.n_tris, o, d, best, bt, bu, bv, R.err, nn, nt);
     }
@@ -787,223 +805,286 @@ __global__ void __launch_bounds__(kStackColumns, 7) k_shadow_dyn(RenderDev R, ui
 }
 
 // ---------------------------------------------------------------------------
-// The whole render as one persistent launch: each lane carries one path from
-// its camera ray through every bounce (closest hit, shading, one shadow ray
-// per light, the next ray) and takes a new path from a device counter when
-// its path ends; a warp refills once kRefillLanesPersistent of its lanes are
-// idle. The paths of every scene of a batch, of any length, flow through the
-// same kernel with no host round trip and no queue in memory. Closest-hit
-// and shadow rays share one traversal loop (ray_tri<kMixed>), so lanes
-// tracing either kind stay on the same code; lanes whose ray finished wait
-// and shade together. The sample sequence, the shading code (light_sample,
-// continue_path) and the traversal are the wavefront's, so every path is the
-// wavefront path of the same index and the images agree up to the order of
-// the float additions into each pixel. Plain renders only: no radiance
-// cache, no Direct / Albedo outputs, no work counters.
+// The whole render as one persistent launch. Each warp owns kPathSlots paths,
+// twice its lanes, and three lists of its own: rays to trace (closest-hit and
+// shadow rays), paths whose ray has hit and that wait to be shaded, and the
+// lanes' rays in flight. Idle lanes take rays from the first list; when it
+// runs short, 32 waiting paths are shaded together: each adds what its vertex
+// emits, appends a shadow ray per light sample and its next ray, and a path
+// that ended is replaced by a new one, of any scene of the batch, from a
+// device counter. With two paths a lane there are always 32 to shade or a ray
+// for every lane, so both the traversal loop and the shading code run with
+// full warps, and no warp waits for another.
+//
+// A ray in flight is parked in shared memory while its warp shades, so the
+// kernel fits 80 to 96 registers. Measured on a B200, 12 scenes of up to 128 K
+// triangles / the 5.2 M-triangle field at 1920x1080x4: one path a lane, shading
+// once three quarters of the warp had stopped tracing, 19.4 / 29.6 ms; with
+// the pool 11.9 / 19.8 (spilling at 96 registers), 9.2 / 17.1 parked, 9.4 /
+// 15.9 at 80 registers; 128 paths a warp gain nothing. The wavefront takes
+// 10.2 / 17.6.
+//
+// The sample sequence, the shading code (light_sample, continue_path) and the
+// traversal are the wavefront's, so every path is the wavefront path of the
+// same index and the images agree up to the order of the float additions into
+// each pixel. Plain renders only: no radiance cache, no Direct / Albedo
+// outputs, no work counters.
 // ---------------------------------------------------------------------------
-struct PathLane {
-    uint32_t sid, pixel, depth;
-    uint64_t key;
-    float3 beta;           // throughput at the current vertex
-    bool after_specular;   // the previous bounce was specular
-    // the vertex being lit: light samples still to trace, then the next ray
-    float3 p, W, wo_l, nee_beta, next_beta;
-    uint32_t mat_id, light_id, next_light;
-    bool specular, cont;
-    float4 no, nd;         // the next ray (when cont)
-    float3 c;              // contribution of the shadow ray in flight
-};
-
-__device__ __forceinline__ void start_path(const RenderDev &R, uint64_t g, PathLane &P, RayState &r)
-{
-    const uint32_t sid = scene_of(R, g);
-    const SceneRec &S = R.scenes[sid];
-    uint32_t pixel, x, y;
-    uint64_t key;
-    path_ident(S, g, pixel, key, x, y);
-    float4 o, d;
-    if (S.ray_o) {
-        o = S.ray_o[pixel];
-        d = S.ray_d[pixel];
-    } else {
-        const float xi1 = rnd(key, kDimCam) - 0.5f, xi2 = rnd(key, kDimCam + 1) - 0.5f;
-        const float fx = x * S.rcp_w + xi1 * S.rcp_w, fy = y * S.rcp_h + xi2 * S.rcp_h;
-        const float3 target = S.corner + S.across * fx + S.up * fy;
-        const float3 dd = normalize3(target - S.centre);
-        o = make_float4(S.centre.x, S.centre.y, S.centre.z, 0.f);
-        d = make_float4(dd.x, dd.y, dd.z, FLT_MAX);
-    }
-    P.sid = sid;
-    P.pixel = pixel + S.pixel_base;
-    P.depth = 0;
-    P.key = key;
-    P.beta = make_float3(1.f, 1.f, 1.f);
-    P.after_specular = false;
-    ray_init(r, o, d, S.n_nodes);
-    r.any = false;
-}
-
-// The next light sample of the vertex with a contribution, as a shadow ray
-// in r; false when none is left.
-__device__ __forceinline__ bool next_light_sample(const RenderDev &R, PathLane &P, RayState &r)
-{
-    const SceneRec &S = R.scenes[P.sid];
-    if (P.specular) return false;
-    float3 U, V;
-    onb_from_w(P.W, U, V);
-    const Mat m = S.mats[P.mat_id < S.n_mats ? P.mat_id : 0];
-    for (uint32_t l = P.next_light; l < S.n_lights && l < kMaxLights; l++) {
-        if (l == P.light_id) continue;
-        float4 so, sd;
-        if (light_sample(S, l, P.key, P.depth, P.p, U, V, P.W, P.wo_l, m, P.nee_beta, so, sd, P.c)) {
-            P.next_light = l + 1;
-            ray_init(r, so, sd, S.n_nodes);
-            r.any = true;
-            return true;
-        }
-    }
-    return false;
-}
-
-// After the vertex's light samples: the next ray, or the end of the path.
-__device__ __forceinline__ bool next_bounce(const RenderDev &R, PathLane &P, RayState &r)
-{
-    if (!P.cont) return false;
-    P.beta = P.next_beta;
-    P.after_specular = P.specular;
-    P.depth++;
-    ray_init(r, P.no, P.nd, R.scenes[P.sid].n_nodes);
-    r.any = false;
-    return true;
-}
-
-// The closest hit of the path's ray is in r: what the vertex adds, and the
-// vertex's state for its light samples and next ray (k_shade's rules).
-// Returns whether the path goes on from this vertex.
-__device__ __forceinline__ bool shade_vertex(const RenderDev &R, PathLane &P, const RayState &r, float4 o, float4 d)
-{
-    const SceneRec &S = R.scenes[P.sid];
-    const int ti = r.best;
-    const uint32_t depth = P.depth;
-    float3 add = make_float3(0.f, 0.f, 0.f);
-    if (ti < 0) {
-        if (ti == -1) {
-            add = P.beta * S.sky;
-            if ((depth == 0 || P.after_specular) && S.inf_escape > 0.f) add = add + P.beta * S.inf_escape;
-            if (!is_black(add)) add_pixel(R.accum, P.pixel, add);
-        }
-        return false;
-    }
-    if (depth > S.max_depth) return false;
-    const Tri tr = S.tris[ti];
-    const uint32_t attr = tr.id.y;
-    const uint32_t mat_id = attr & 0xffffu, light_id = attr >> 16;
-    const Mat m = S.mats[mat_id < S.n_mats ? mat_id : 0];
-    const float3 ng = normalize3(make_float3(tr.a.w, tr.b.w, tr.c.w));
-    const float t = r.tcur;
-    const float3 p = make_float3(o.x + t * d.x, o.y + t * d.y, o.z + t * d.z);
-    const float3 wo = normalize3(make_float3(d.x, d.y, d.z)) * -1.f;
-    const float3 W = ng;
-    float3 U, V;
-    onb_from_w(W, U, V);
-    const float3 wo_l = make_float3(dot3(U, wo), dot3(V, wo), dot3(W, wo));
-    if ((depth == 0 || P.after_specular) && light_id != 0xffffu && light_id < S.n_lights && dot3(W, wo) > 0.f)
-        add = add + P.beta * S.lights[light_id].emit;
-    if (!is_black(add)) add_pixel(R.accum, P.pixel, add);
-    if (depth >= S.max_depth) return false;
-    P.specular = m.kind >= 2u;
-    P.p = p;
-    P.W = W;
-    P.wo_l = wo_l;
-    P.mat_id = mat_id;
-    P.light_id = light_id;
-    P.next_light = 0;
-    P.nee_beta = P.beta;
-    P.next_beta = P.beta;
-    P.cont = continue_path(S, P.key, depth, m, P.specular, p, ng, U, V, W, wo_l, P.next_beta, P.no, P.nd);
-    return true;
-}
-
 constexpr int kPersistThreads = 128;
-// A warp of the one-launch renderer takes new paths once 16 of its lanes are
-// idle (a path start costs a camera ray and a scene lookup; 8 measured 2 %
-// slower on the 32-scene batch, 4 5 % slower).
-constexpr uint32_t kRefillLanesPersistent = 16;
+constexpr uint32_t kPathSlots = 64;
+constexpr int kNewPath = -3;  // hit of a slot that waits for a path
 
-__global__ void __launch_bounds__(kPersistThreads) k_render_persistent(RenderDev R, uint64_t total, unsigned long long *next)
+// One warp's part of the pool, in device memory: the paths, then a stack of
+// rays. A shading step runs when fewer than 32 rays are left and appends at
+// most 32 x (1 + lights).
+struct WarpPool {
+    float4 *beta;          // throughput, w = the previous bounce was specular
+    uint4 *id;             // sample key (x, y), pixel, scene | depth << 16
+    float4 *hit_o, *hit_d; // the finished ray: origin, t; direction, triangle
+    float4 *ray_o, *ray_d, *ray_c;  // ray; shadow rays: contribution, pixel
+    uint32_t *ray_m;       // scene | slot << 16; bit 31: a shadow ray
+};
+__host__ __device__ constexpr size_t pool_bytes(uint32_t lights)
 {
-    const uint32_t lane = threadIdx.x & 31u;
-    uint2 stack[kMaxStack];
-    RayState r;
-    // The path state lives in shared memory, one slot per thread (the kernel
-    // runs 128 threads a block): in registers it spilled the traversal's
-    // working set; in shared memory the kernel renders 1.17x faster.
-    __shared__ PathLane lanes[kPersistThreads];
-    __shared__ float4 ray_io[kPersistThreads][2];  // the closest-hit ray in flight (for shading)
-    PathLane &P = lanes[threadIdx.x];
-    float4 &ro = ray_io[threadIdx.x][0], &rd = ray_io[threadIdx.x][1];
-    ro = make_float4(0.f, 0.f, 0.f, 0.f);
-    rd = ro;
-    bool active = false, exhausted = false;  // exhausted is warp-uniform
-    // 0: tracing; 1: closest hit found, waiting to shade; 2: shadow ray done, waiting to be counted
-    uint32_t state = 0;
+    return kPathSlots * 64u + 32u * (2u + lights) * 52u;
+}
+__device__ __forceinline__ WarpPool warp_pool(unsigned char *base, uint32_t lights)
+{
+    const uint32_t rays = 32u * (2u + lights);
+    float4 *f = reinterpret_cast<float4 *>(base);
+    WarpPool P;
+    P.beta = f;
+    P.id = reinterpret_cast<uint4 *>(f + kPathSlots);
+    P.hit_o = f + 2 * kPathSlots;
+    P.hit_d = f + 3 * kPathSlots;
+    P.ray_o = f + 4 * kPathSlots;
+    P.ray_d = P.ray_o + rays;
+    P.ray_c = P.ray_d + rays;
+    P.ray_m = reinterpret_cast<uint32_t *>(P.ray_c + rays);
+    return P;
+}
+
+// A lane's ray in flight, kept in shared memory while its warp shades: the
+// shading code needs the registers.
+constexpr int kParkedWords = 20;
+struct Parked {
+    uint32_t w[kParkedWords][kPersistThreads];
+};
+__device__ __forceinline__ void park(Parked &s, const RayState &r)
+{
+    const uint32_t v[kParkedWords] = {
+        __float_as_uint(r.ox), __float_as_uint(r.oy), __float_as_uint(r.oz), __float_as_uint(r.dx), __float_as_uint(r.dy),
+        __float_as_uint(r.dz), __float_as_uint(r.tmin), __float_as_uint(r.tcur), r.ng_base, r.ng_hits, r.tg_base,
+        r.tg_slots, r.tg_hits, r.tq_base, r.tq_slots, r.tq_hits, r.budget, (uint32_t)r.sp, (uint32_t)r.best, r.any};
+#pragma unroll
+    for (int k = 0; k < kParkedWords; k++) s.w[k][threadIdx.x] = v[k];
+}
+__device__ __forceinline__ void unpark(const Parked &s, RayState &r)
+{
+    auto u = [&](int k) { return s.w[k][threadIdx.x]; };
+    auto f = [&](int k) { return __uint_as_float(s.w[k][threadIdx.x]); };
+    ray_init(r, make_float4(f(0), f(1), f(2), f(6)), make_float4(f(3), f(4), f(5), f(7)), 0u);
+    r.ng_base = u(8);
+    r.ng_hits = u(9);
+    r.tg_base = u(10);
+    r.tg_slots = u(11);
+    r.tg_hits = u(12);
+    r.tq_base = u(13);
+    r.tq_slots = u(14);
+    r.tq_hits = u(15);
+    r.budget = u(16);
+    r.sp = (int)u(17);
+    r.best = (int)u(18);
+    r.any = u(19) != 0u;
+}
+
+template <bool kOne>
+__global__ void __launch_bounds__(kPersistThreads, kOne ? 6 : 5)
+    k_render_persistent(RenderDev R, uint64_t total, unsigned long long *next, unsigned char *pool, uint32_t lights)
+{
+    constexpr uint32_t kFull = 0xffffffffu;
+    __shared__ uint2 sstack[kShortStack * kStackColumns];
+    __shared__ float4 s_shadow[kPersistThreads];               // the lane's shadow ray: contribution, pixel
+    __shared__ uint8_t s_wait[kPersistThreads / 32][kPathSlots];  // slots of the paths to shade
+    __shared__ Parked s_park;
+    uint2 lstack[kMaxStack - kShortStack];
+    const SplitStack stack{sstack + threadIdx.x, lstack};
+    const uint32_t lane = threadIdx.x & 31u, below = (1u << lane) - 1u, magic = plane_magic(R.n_scenes);
+    uint8_t *wait = s_wait[threadIdx.x >> 5];
+    const WarpPool P = warp_pool(
+        pool + (size_t)(blockIdx.x * (kPersistThreads / 32) + (threadIdx.x >> 5)) * pool_bytes(lights), lights);
+    for (uint32_t k = lane; k < kPathSlots; k += 32u) {
+        wait[k] = (uint8_t)k;
+        P.hit_d[k] = make_float4(0.f, 0.f, 0.f, __int_as_float(kNewPath));
+    }
+    __syncwarp();
+    uint32_t n_wait = kPathSlots, n_rays = 0;  // warp-uniform, as is exhausted
+    bool exhausted = false;
     TraceScene scene{nullptr, nullptr, 0u, 0u};
-    const uint32_t magic = plane_magic(R.n_scenes);
-    while (true) {
-        const uint32_t idle = __ballot_sync(0xffffffffu, !active);
-        if (!exhausted && (__popc(idle) >= kRefillLanesPersistent || idle == 0xffffffffu)) {
-            const uint32_t leader = __ffs(idle) - 1u;
+    if (kOne) bind_scene(scene, R.scenes[0]);
+    RayState r;
+    ray_init(r, make_float4(0.f, 0.f, 0.f, 0.f), make_float4(0.f, 0.f, 1.f, 0.f), 0u);
+    ray_stop(r);
+    r.any = false;
+    bool has = false;
+    uint32_t meta = 0;  // of the lane's ray
+
+    // Appends a ray for every lane of the warp that wants one.
+    auto push = [&](bool want, float4 o, float4 d, float4 c, uint32_t m) {
+        const uint32_t lanes = __ballot_sync(kFull, want);
+        if (want) {
+            const uint32_t at = n_rays + __popc(lanes & below);
+            P.ray_o[at] = o;
+            P.ray_d[at] = d;
+            if (m >> 31) P.ray_c[at] = c;
+            P.ray_m[at] = m;
+        }
+        n_rays += __popc(lanes);
+    };
+
+    // Shades the last min(32, n_wait) waiting paths.
+    auto shade = [&]() {
+        const uint32_t m = min(32u, n_wait);
+        n_wait -= m;
+        bool live = lane < m, cont = false, lit = false;
+        const uint32_t slot = live ? wait[n_wait + lane] : 0u;
+        float4 no = make_float4(0.f, 0.f, 0.f, 0.f), nd = no;
+        float3 beta = make_float3(1.f, 1.f, 1.f);
+        uint64_t key = 0;
+        uint32_t pixel = 0, sid = 0, depth = 0, light_id = 0xffffu, n_lights = 0;
+        Mat mat;
+        float3 p, W = make_float3(0.f, 0.f, 1.f), U = W, V = W, wo_l = W;
+        bool specular = false;
+        int ti = kNewPath;
+        if (live) {
+            const float4 hd = P.hit_d[slot];
+            ti = __float_as_int(hd.w);
+            if (ti != kNewPath) {
+                const float4 ho = P.hit_o[slot], b4 = P.beta[slot];
+                const uint4 id = P.id[slot];
+                key = (uint64_t)id.x | (uint64_t)id.y << 32;
+                pixel = id.z;
+                sid = kOne ? 0u : id.w & 0xffffu;
+                depth = id.w >> 16;
+                beta = make_float3(b4.x, b4.y, b4.z);
+                const bool after_specular = b4.w != 0.f;
+                const SceneRec &S = R.scenes[sid];
+                float3 add = make_float3(0.f, 0.f, 0.f);
+                if (ti == -1) {
+                    add = beta * S.sky;
+                    if ((depth == 0 || after_specular) && S.inf_escape > 0.f) add = add + beta * S.inf_escape;
+                } else if (ti >= 0 && depth <= S.max_depth) {
+                    const Tri tr = S.tris[ti];
+                    const uint32_t mat_id = tr.id.y & 0xffffu;
+                    light_id = tr.id.y >> 16;
+                    mat = S.mats[mat_id < S.n_mats ? mat_id : 0];
+                    W = normalize3(make_float3(tr.a.w, tr.b.w, tr.c.w));
+                    const float t = ho.w;
+                    p = make_float3(ho.x + t * hd.x, ho.y + t * hd.y, ho.z + t * hd.z);
+                    const float3 wo = normalize3(make_float3(hd.x, hd.y, hd.z)) * -1.f;
+                    onb_from_w(W, U, V);
+                    wo_l = make_float3(dot3(U, wo), dot3(V, wo), dot3(W, wo));
+                    if ((depth == 0 || after_specular) && light_id != 0xffffu && light_id < S.n_lights &&
+                        dot3(W, wo) > 0.f)
+                        add = add + beta * S.lights[light_id].emit;
+                    if (depth < S.max_depth) {
+                        specular = mat.kind >= 2u;
+                        lit = !specular;
+                        n_lights = min(S.n_lights, kMaxLights);
+                        cont = true;
+                    }
+                }
+                if (!is_black(add)) add_pixel(R.accum, pixel, add);
+            }
+        }
+        for (uint32_t l = 0; __any_sync(kFull, lit && l < n_lights); l++) {
+            float4 so = no, sd = no;
+            float3 c = make_float3(0.f, 0.f, 0.f);
+            const bool ok = lit && l < n_lights && l != light_id &&
+                            light_sample(R.scenes[sid], l, key, depth, p, U, V, W, wo_l, mat, beta, so, sd, c);
+            push(ok, so, sd, make_float4(c.x, c.y, c.z, __uint_as_float(pixel)), 0x80000000u | sid);
+        }
+        if (cont)
+            cont = continue_path(R.scenes[sid], key, depth, mat, specular, p, W, U, V, W, wo_l, beta, no, nd);
+        float flag = specular ? 1.f : 0.f;
+        depth++;
+        // ended paths (and slots that had none) take new ones
+        const uint32_t need = __ballot_sync(kFull, live && !cont);
+        if (need && !exhausted) {
             unsigned long long base = 0;
-            if (lane == leader) base = atomicAdd(next, (unsigned long long)__popc(idle));
-            base = __shfl_sync(0xffffffffu, base, leader);
-            if (base >= total) exhausted = true;
-            if (!active) {
-                const uint64_t k = base + __popc(idle & ((1u << lane) - 1u));
-                if (k < total) {
-                    start_path(R, k, P, r);
-                    bind_scene(scene, R.scenes[P.sid]);
-                    ro = make_float4(r.ox, r.oy, r.oz, r.tmin);
-                    rd = make_float4(r.dx, r.dy, r.dz, r.tcur);
-                    active = true;
-                    state = 0;
-                }
+            if (lane == 0u) base = atomicAdd(next, (unsigned long long)__popc(need));
+            base = __shfl_sync(kFull, base, 0);
+            exhausted = base + __popc(need) >= total;
+            const uint64_t g = base + __popc(need & below);
+            if (live && !cont && g < total) {
+                sid = kOne ? 0u : scene_of(R, g);
+                const SceneRec &S = R.scenes[sid];
+                first_ray(S, g, pixel, key, no, nd);
+                pixel += S.pixel_base;
+                beta = make_float3(1.f, 1.f, 1.f);
+                flag = 0.f;
+                depth = 0;
+                cont = true;
             }
         }
-        const uint32_t live = __ballot_sync(0xffffffffu, active);
-        if (live == 0u) break;
-        const bool trace = active && state == 0u;
+        if (cont) {
+            P.beta[slot] = make_float4(beta.x, beta.y, beta.z, flag);
+            P.id[slot] = make_uint4((uint32_t)key, (uint32_t)(key >> 32), pixel, sid | depth << 16);
+        }
+        push(cont, no, nd, no, sid | slot << 16);
         __syncwarp();
-        if (trace && r.tq_hits == 0u && ray_has_nodes(r)) ray_node(r, stack, scene.nodes, scene.n_nodes, magic, R.err);
-        while (true) {
-            const uint32_t tri = __ballot_sync(0xffffffffu, trace && r.tg_hits != 0u);
-            const uint32_t node = __ballot_sync(0xffffffffu, trace && r.tq_hits == 0u && ray_has_nodes(r));
-            if (tri == 0u || (__popc(tri) < kTriLanes && __popc(node) >= kNodeLanes)) break;
-            if (trace && r.tg_hits) ray_tri<false, false, false, false, true>(r, scene.tris, scene.n_tris, R.err);
-        }
-        if (trace && r.tg_hits == 0u && !ray_has_nodes(r)) state = r.any ? 2u : 1u;
-        // Shading and shadow results run for the waiting lanes together, once
-        // three quarters of the warp's paths wait or none is tracing, so that
-        // this code runs with most lanes converged instead of one lane at a
-        // time (measured on a B200: half the warp 215, three quarters 233,
-        // seven eighths 243, all 239 Msamples/s on the 32-scene batch; on the
-        // field 175 / 184 / 179 / 152).
-        const uint32_t waiting = __ballot_sync(0xffffffffu, active && state != 0u);
-        const uint32_t tracing = live & ~waiting;
-        if (waiting && (4u * __popc(waiting) >= 3u * __popc(live) || tracing == 0u)) {
-            // a shadow ray's light sample counts when nothing is in the way;
-            // a closest hit is shaded; then either lane takes the vertex's
-            // next light sample or its next ray (one copy of that code, so
-            // the kernel stays small enough for the instruction cache)
-            if (active && state == 2u && r.best == -1) add_pixel(R.accum, P.pixel, P.c);
-            if (active && state == 1u) active = shade_vertex(R, P, r, ro, rd);
-            if (active && state != 0u) {
-                active = next_light_sample(R, P, r) || next_bounce(R, P, r);
-                state = 0;
-                if (active && !r.any) {
-                    ro = make_float4(r.ox, r.oy, r.oz, r.tmin);
-                    rd = make_float4(r.dx, r.dy, r.dz, r.tcur);
-                }
+    };
+
+    while (true) {
+        const uint32_t idle = __ballot_sync(kFull, r.tg_hits == 0u && !ray_has_nodes(r));
+        if (__popc(idle) >= kRefillLanes || idle == kFull) {
+            // results of the finished rays
+            const bool mine = (idle >> lane) & 1u, done = mine && has, closest = done && !(meta >> 31);
+            const uint32_t hits = __ballot_sync(kFull, closest);
+            if (closest) {
+                const uint32_t slot = meta >> 16;
+                P.hit_o[slot] = make_float4(r.ox, r.oy, r.oz, r.tcur);
+                P.hit_d[slot] = make_float4(r.dx, r.dy, r.dz, __int_as_float(r.best));
+                wait[n_wait + __popc(hits & below)] = (uint8_t)slot;
+            } else if (done && r.best == -1) {
+                const float4 c = s_shadow[threadIdx.x];
+                add_pixel(R.accum, __float_as_uint(c.w), make_float3(c.x, c.y, c.z));
             }
+            if (mine) has = false;
+            n_wait += __popc(hits);
+            __syncwarp();
+            // rays for the idle lanes: shade while they run short, with full
+            // warps unless few rays are in flight
+            const uint32_t want = __popc(idle);
+            if (n_rays < want && n_wait > 0u && (n_wait >= 32u || want > 24u)) {
+                park(s_park, r);
+                __syncwarp();
+                do shade();
+                while (n_rays < want && n_wait > 0u && (n_wait >= 32u || want > 24u));
+                unpark(s_park, r);
+                if (!kOne) bind_scene(scene, R.scenes[meta & 0xffffu]);
+            }
+            const uint32_t rank = __popc(idle & below), take = min(want, n_rays);
+            if (mine && rank < take) {
+                const uint32_t at = n_rays - 1u - rank;
+                const float4 o = P.ray_o[at], d = P.ray_d[at];
+                meta = P.ray_m[at];
+                if (!kOne) bind_scene(scene, R.scenes[meta & 0xffffu]);
+                ray_init(r, o, d, scene.n_nodes);
+                r.any = (meta >> 31) != 0u;
+                if (r.any) s_shadow[threadIdx.x] = P.ray_c[at];
+                has = true;
+            }
+            n_rays -= take;
+            if (take == 0u && idle == kFull) break;  // no ray, and so no path left to shade
+        }
+        __syncwarp();
+        if (r.tq_hits == 0u && ray_has_nodes(r)) ray_node(r, stack, scene.nodes, scene.n_nodes, magic, R.err);
+        while (true) {
+            const uint32_t tri = __ballot_sync(kFull, r.tg_hits != 0u);
+            const uint32_t node = __ballot_sync(kFull, r.tq_hits == 0u && ray_has_nodes(r));
+            if (tri == 0u || (__popc(tri) < kTriLanes && __popc(node) >= kNodeLanes)) break;
+            if (r.tg_hits) ray_tri<false, false, false, false, true>(r, scene.tris, scene.n_tris, R.err);
         }
     }
 }
@@ -1201,7 +1282,9 @@ cudaError_t render_wave(const RenderDev &R, uint32_t n_paths, uint64_t wave_begi
             n_launch++;
         }
         traced = false;
-        k_shade<<<blocks_for(n_paths, T), T, 0, st>>>(R, cur, depth, wave_begin);
+        (R.cache_depth ? (one ? k_shade<true, true> : k_shade<true, false>)
+                       : (one ? k_shade<false, true> : k_shade<false, false>))<<<blocks_for(n_paths, T), T, 0, st>>>(
+            R, cur, depth, wave_begin);
         n_launch++;
         if (R.cache_depth && cache && (depth == R.cache_depth || (R.train_tail && depth == tail))) {
             if (R.hc_keys)
@@ -1240,18 +1323,38 @@ cudaError_t render_wave(const RenderDev &R, uint32_t n_paths, uint64_t wave_begi
     return cudaSuccess;
 }
 
-cudaError_t render_persistent(const RenderDev &R, uint64_t total, unsigned long long *next, uint32_t *launches,
-                              cudaStream_t st)
+// Warps of the one-launch renderer on the current device, at most.
+static cudaError_t persistent_grid(uint64_t total, bool one, uint32_t &blocks)
+{
+    int per_sm = 0;
+    cudaError_t e = one ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_render_persistent<true>, kPersistThreads, 0)
+                        : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_render_persistent<false>, kPersistThreads, 0);
+    if (e != cudaSuccess) return e;
+    // small renders: a path a lane rather than two, on more SMs
+    const uint64_t want = (total + kPersistThreads - 1) / kPersistThreads;
+    const uint64_t cap = (uint64_t)current_sm_count() * (uint64_t)(per_sm > 0 ? per_sm : 1);
+    blocks = (uint32_t)(want < cap ? (want > 0 ? want : 1) : cap);
+    return cudaSuccess;
+}
+
+cudaError_t render_persistent_bytes(const RenderDev &R, uint64_t total, uint32_t lights, size_t &bytes)
+{
+    uint32_t blocks = 0;
+    const cudaError_t e = persistent_grid(total, R.n_scenes == 1u, blocks);
+    bytes = (size_t)blocks * (kPersistThreads / 32) * pool_bytes(lights);
+    return e;
+}
+
+cudaError_t render_persistent(const RenderDev &R, uint64_t total, uint32_t lights, unsigned long long *next,
+                              unsigned char *pool, uint32_t *launches, cudaStream_t st)
 {
     cudaError_t e = cudaMemsetAsync(next, 0, sizeof(unsigned long long), st);
     if (e != cudaSuccess) return e;
-    int per_sm = 0;
-    if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_render_persistent, kPersistThreads, 0)) != cudaSuccess)
-        return e;
-    const uint64_t want = (total + 127) / 128;
-    const uint64_t cap = (uint64_t)current_sm_count() * (uint64_t)(per_sm > 0 ? per_sm : 1);
-    const uint32_t blocks = (uint32_t)(want < cap ? (want > 0 ? want : 1) : cap);
-    k_render_persistent<<<blocks, kPersistThreads, 0, st>>>(R, total, next);
+    const bool one = R.n_scenes == 1u;
+    uint32_t blocks = 0;
+    if ((e = persistent_grid(total, one, blocks)) != cudaSuccess) return e;
+    (one ? k_render_persistent<true> : k_render_persistent<false>)<<<blocks, kPersistThreads, 0, st>>>(R, total, next,
+                                                                                                   pool, lights);
     if (launches) *launches += 1;
     return cudaGetLastError();
 }

@@ -272,11 +272,11 @@ ILG_API int ilg_render(ilg_ctx *ctx, const ilg_camera *cam, const ilg_render_opt
  * These are the per-sample bytes of the path tracer's memory roofline. */
 #define ILG_RENDER_COUNT 0x4u
 /* ilg_render / ilg_render_batch flag: the whole render as one persistent
- * kernel launch instead of the wavefront's launches per bounce. Each GPU
- * thread carries one path through all its bounces (closest hit, shading, a
+ * kernel launch instead of the wavefront's launches per bounce. Each warp
+ * carries a pool of paths through all their bounces (closest hit, shading, a
  * shadow ray per light, the next ray) and takes a new path, of any scene of
- * a batch, when its path ends. Same paths as the wavefront (same sample
- * sequence and arithmetic): the images agree up to float summation order.
+ * a batch, when one ends. Same paths as the wavefront (same sample sequence
+ * and arithmetic): the images agree up to float summation order.
  * Plain renders only (no cache options, ILG_RENDER_COUNT, or Direct /
  * Albedo outputs). */
 #define ILG_RENDER_PERSISTENT 0x20u
