@@ -98,7 +98,7 @@ struct ilg_ctx {
     ilg::DevBuf<float4> hc_vals;
     ilg::DevBuf<float> rec_feat, rec_tgt, qry_feat, qry_out;
     ilg::DevBuf<float4> rec_beta, qry_beta;
-    uint32_t last_train_records = 0;
+    uint32_t last_rec_cap = 0;      // the last cached render stored at most this many training records
     bool last_hash_update = false;  // the last cached render updated the hash-grid cache
     float last_train_loss = 0.f;
     uint32_t last_render_launches = 0;
@@ -126,7 +126,9 @@ struct ilg_ctx {
     ilg::DevBuf<__nv_bfloat16> mlp_wf, mlp_wb, mlp_wu, mlp_wv, mlp_xcm, mlp_hcm, mlp_dzcm;
     bool mlp_ready = false;
     uint32_t mlp_encoding = 0;  // ILG_MLP_ENC_*
-    uint32_t mlp_step = 0;
+    ilg::DevBuf<uint32_t> mlp_step;   // Adam steps so far
+    ilg::DevBuf<float2> mlp_bias;     // their bias corrections
+    bool mlp_grads_clear = false;     // both gradient buffers are zero
     float mlp_lr = 1e-2f;
 
     ilg::MlpDev mlp_view() const
@@ -134,7 +136,7 @@ struct ilg_ctx {
         ilg::MlpDev M;
         memset(&M, 0, sizeof(M));  // zero padding: the struct's bytes key the cached render graph
         M.w = mlp_w.ptr; M.m = mlp_m.ptr; M.v = mlp_v.ptr; M.grad = mlp_grad.ptr; M.loss = mlp_loss.ptr;
-        M.wf = mlp_wf.ptr; M.wb = mlp_wb.ptr; M.wu = mlp_wu.ptr; M.wv = mlp_wv.ptr; M.err = derr.ptr; M.xcm = mlp_xcm.ptr; M.hcm = mlp_hcm.ptr; M.dzcm = mlp_dzcm.ptr;
+        M.wf = mlp_wf.ptr; M.wb = mlp_wb.ptr; M.wu = mlp_wu.ptr; M.wv = mlp_wv.ptr; M.err = derr.ptr; M.step = mlp_step.ptr; M.bias = mlp_bias.ptr; M.xcm = mlp_xcm.ptr; M.hcm = mlp_hcm.ptr; M.dzcm = mlp_dzcm.ptr;
         M.cap = (uint32_t)(mlp_xcm.cap / ilg::kMlpIn);
         M.grid = mlp_grid.ptr; M.grid_grad = mlp_grid_grad.ptr; M.grid_m = mlp_grid_m.ptr; M.grid_v = mlp_grid_v.ptr;
         ilg::grid_resolution(M.grid_res);
@@ -188,6 +190,6 @@ struct ilg_ctx {
         mlp_w.release(); mlp_m.release(); mlp_v.release(); mlp_grad.release(); mlp_loss.release();
         mlp_grid.release(); mlp_grid_grad.release(); mlp_grid_m.release(); mlp_grid_v.release(); mlp_enc.release();
         mlp_raw.release(); mlp_tgt.release(); mlp_out.release(); mlp_wf.release(); mlp_wb.release(); mlp_wu.release(); mlp_wv.release();
-        mlp_xcm.release(); mlp_hcm.release(); mlp_dzcm.release();
+        mlp_xcm.release(); mlp_step.release(); mlp_bias.release(); mlp_hcm.release(); mlp_dzcm.release();
     }
 };

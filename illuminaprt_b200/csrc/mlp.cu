@@ -15,8 +15,8 @@
 //                    the batch, FP32 partial sums added atomically
 //   k_grid_bwd       dX of the grid columns = dZ0 W0^T, scattered to the
 //                    hash-grid corners of every level (FP32 atomics)
-// followed by k_mlp_adam (FP32 master weights, refreshes the BF16 copies)
-// and k_grid_adam (the grid features).
+// followed by k_adam (FP32 master weights, refreshing the BF16 copies, and the
+// grid features).
 #include "devinfo.cuh"
 #include "mlp.cuh"
 
@@ -393,22 +393,59 @@ __global__ void k_mlp_copies(MlpDev M)
     write_copies(M, i, M.w[i]);
 }
 
-__global__ void k_mlp_adam(MlpDev M, float lr, float bc1, float bc2)
+__device__ __forceinline__ float adam_update(float w, float g, float &m, float &v, float lr, float2 bc)
 {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= kMlpParams) return;
-    const int l = layer_of(i);
-    if (l == kMlpLayers - 1 && ((i - mlp_off(l)) % mlp_out(l)) >= 3) return;
     const float b1 = 0.9f, b2 = 0.99f, eps = 1e-15f;
-    const float gr = M.grad[i];
-    const float m = b1 * M.m[i] + (1.f - b1) * gr;
-    const float v = b2 * M.v[i] + (1.f - b2) * gr * gr;
-    M.m[i] = m;
-    M.v[i] = v;
-    const float w = M.w[i] - lr * (m / bc1) / (sqrtf(v / bc2) + eps);
-    M.w[i] = w;
-    write_copies(M, i, w);
+    m = b1 * m + (1.f - b1) * g;
+    v = b2 * v + (1.f - b2) * g * g;
+    return w - lr * (m / bc.x) / (sqrtf(v / bc.y) + eps);
 }
+
+// One Adam step of the weights and, after them, the grid features (kGrid4
+// groups of four). // kClear: the gradients are left zero for the next step. Bound by the grid's
+// four arrays of 4 MB.
+constexpr int kAdamThreads = 256;
+constexpr int kWeightBlocks = (kMlpParams + kAdamThreads - 1) / kAdamThreads;
+constexpr int kGridBlocks = (int)(kGridParams / 4 + kAdamThreads - 1) / kAdamThreads;
+
+template <bool kClear>
+__global__ void __launch_bounds__(kAdamThreads) k_adam(MlpDev M, float lr, uint32_t n, const TrainRows rows)
+{
+    if (rows_of(n, rows) == 0u) return;
+    const float2 bc = M.bias[min(*M.step, (uint32_t)kAdamSteps - 1u)];
+    if (blockIdx.x < kWeightBlocks) {
+        const int i = blockIdx.x * kAdamThreads + threadIdx.x;
+        if (i >= kMlpParams) return;
+        const int l = layer_of(i);
+        if (l == kMlpLayers - 1 && ((i - mlp_off(l)) % mlp_out(l)) >= 3) return;
+        float m = M.m[i], v = M.v[i];
+        const float w = adam_update(M.w[i], M.grad[i], m, v, lr, bc);
+        M.m[i] = m;
+        M.v[i] = v;
+        M.w[i] = w;
+        if (kClear) M.grad[i] = 0.f;
+        write_copies(M, i, w);
+        return;
+    }
+    const uint32_t i = (blockIdx.x - kWeightBlocks) * kAdamThreads + threadIdx.x;
+    if (i >= kGridParams / 4) return;
+    float4 *gm = reinterpret_cast<float4 *>(M.grid_m) + i, *gv = reinterpret_cast<float4 *>(M.grid_v) + i,
+           *gw = reinterpret_cast<float4 *>(M.grid) + i, *gg = reinterpret_cast<float4 *>(M.grid_grad) + i;
+    float4 m = *gm, v = *gv, w = *gw;
+    const float4 g = *gg;
+    w.x = adam_update(w.x, g.x, m.x, v.x, lr, bc);
+    w.y = adam_update(w.y, g.y, m.y, v.y, lr, bc);
+    w.z = adam_update(w.z, g.z, m.z, v.z, lr, bc);
+    w.w = adam_update(w.w, g.w, m.w, v.w, lr, bc);
+    *gm = m;
+    *gv = v;
+    *gw = w;
+    if (kClear) *gg = make_float4(0.f, 0.f, 0.f, 0.f);
+}
+
+// Counts an Adam step before k_adam reads the count (k_mlp_dw_tc does it for
+// the batches whose size the device knows).
+__global__ void k_adam_step(MlpDev M) { *M.step += 1u; }
 
 __global__ void k_grid_init(MlpDev M, uint32_t seed)
 {
@@ -429,8 +466,11 @@ constexpr int kGridBwdThreads = 256;
 // thread per row left the SMs a few warps each). The row's dZ0 loads are
 // shared by the 16 lanes of a half-warp (one address per load); W0's rows are
 // padded to 65 floats so that the 16 levels of a half-warp read 16 banks.
-__global__ void __launch_bounds__(kGridBwdThreads) k_grid_bwd(MlpDev M, const float *__restrict__ raw, uint32_t n)
+__global__ void __launch_bounds__(kGridBwdThreads) k_grid_bwd(MlpDev M, const float *__restrict__ raw, uint32_t n,
+                                                              const TrainRows rows)
 {
+    n = rows_of(n, rows);
+    if ((uint64_t)blockIdx.x * blockDim.x >= (uint64_t)n * kGridLevels) return;
     __shared__ float w0[2 * kGridLevels][kMlpHid + 1];
     for (int i = threadIdx.x; i < 2 * kGridLevels * kMlpHid; i += blockDim.x)
         w0[i / kMlpHid][i % kMlpHid] = __bfloat162float(__float2bfloat16_rn(M.w[mlp_off(0) + i]));
@@ -468,19 +508,6 @@ __global__ void __launch_bounds__(kGridBwdThreads) k_grid_bwd(MlpDev M, const fl
 inline unsigned grid_bwd_blocks(uint32_t n)
 {
     return (unsigned)(((uint64_t)n * kGridLevels + kGridBwdThreads - 1) / kGridBwdThreads);
-}
-
-__global__ void k_grid_adam(MlpDev M, float lr, float bc1, float bc2)
-{
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= kGridParams) return;
-    const float b1 = 0.9f, b2 = 0.99f, eps = 1e-15f;
-    const float gr = M.grid_grad[i];
-    const float m = b1 * M.grid_m[i] + (1.f - b1) * gr;
-    const float v = b2 * M.grid_v[i] + (1.f - b2) * gr * gr;
-    M.grid_m[i] = m;
-    M.grid_v[i] = v;
-    M.grid[i] -= lr * (m / bc1) / (sqrtf(v / bc2) + eps);
 }
 
 inline uint32_t grid_for(uint32_t n_rows, int sms)
@@ -549,7 +576,7 @@ cudaError_t mlp_grads(const MlpDev &M, const float *raw, const float *target, ui
             return e;
         if ((e = mlp_train_tc(M, raw, target, n, st)) != cudaSuccess) return e;
         if (has_grid)
-            k_grid_bwd<<<grid_bwd_blocks(n), kGridBwdThreads, 0, st>>>(M, raw, n);
+            k_grid_bwd<<<grid_bwd_blocks(n), kGridBwdThreads, 0, st>>>(M, raw, n, TrainRows{nullptr, 0u, 0u});
         if ((e = mlp_dw_tc(M, n_pad, st)) != cudaSuccess) return e;
         return cudaGetLastError();
     }
@@ -566,7 +593,7 @@ cudaError_t mlp_grads(const MlpDev &M, const float *raw, const float *target, ui
     const uint32_t grid = grid_for(n, num_sms());
     k_mlp_fwd<true><<<grid, 128, smem_f, st>>>(M, raw, n, nullptr, nullptr);
     k_mlp_bwd<<<grid, 128, smem_b, st>>>(M, raw, target, n);
-    if (has_grid) k_grid_bwd<<<grid_bwd_blocks(n), kGridBwdThreads, 0, st>>>(M, raw, n);
+    if (has_grid) k_grid_bwd<<<grid_bwd_blocks(n), kGridBwdThreads, 0, st>>>(M, raw, n, TrainRows{nullptr, 0u, 0u});
     const uint32_t chunks = (n_pad + kDwChunk - 1) / kDwChunk;
     for (int l = 0; l < kMlpLayers; l++) {
         const __nv_bfloat16 *A = l == 0 ? M.xcm : M.hcm + (size_t)(l - 1) * kMlpHid * M.cap;
@@ -581,11 +608,33 @@ cudaError_t mlp_grads(const MlpDev &M, const float *raw, const float *target, ui
     return cudaGetLastError();
 }
 
-cudaError_t mlp_adam(const MlpDev &M, uint32_t step, float lr, cudaStream_t st)
+cudaError_t mlp_adam(const MlpDev &M, float lr, cudaStream_t st)
 {
-    const float bc1 = 1.f - powf(0.9f, (float)step), bc2 = 1.f - powf(0.99f, (float)step);
-    k_mlp_adam<<<(kMlpParams + 255) / 256, 256, 0, st>>>(M, lr, bc1, bc2);
-    if (M.encoding == kEncHashGrid) k_grid_adam<<<(kGridParams + 255) / 256, 256, 0, st>>>(M, lr, bc1, bc2);
+    const TrainRows all{nullptr, 0u, 0u};
+    const int blocks = kWeightBlocks + (M.encoding == kEncHashGrid ? kGridBlocks : 0);
+    k_adam_step<<<1, 1, 0, st>>>(M);
+    k_adam<false><<<blocks, kAdamThreads, 0, st>>>(M, lr, 1u, all);
+    return cudaGetLastError();
+}
+
+cudaError_t mlp_clear_grads(const MlpDev &M, cudaStream_t st)
+{
+    cudaError_t e = cudaMemsetAsync(M.grad, 0, kMlpParams * sizeof(float), st);
+    if (e == cudaSuccess && M.encoding == kEncHashGrid)
+        e = cudaMemsetAsync(M.grid_grad, 0, kGridParams * sizeof(float), st);
+    return e;
+}
+
+cudaError_t mlp_train_rows(const MlpDev &M, const float *raw, const float *target, uint32_t n, const TrainRows &rows,
+                           float lr, cudaStream_t st)
+{
+    if (n == 0 || n > M.cap) return cudaErrorInvalidValue;
+    cudaError_t e = mlp_train_tc(M, raw, target, n, st, rows);
+    if (e != cudaSuccess) return e;
+    const bool has_grid = M.encoding == kEncHashGrid;
+    if (has_grid) k_grid_bwd<<<grid_bwd_blocks(n), kGridBwdThreads, 0, st>>>(M, raw, n, rows);
+    if ((e = mlp_dw_tc(M, (n + 15) / 16 * 16, st, rows)) != cudaSuccess) return e;
+    k_adam<true><<<kWeightBlocks + (has_grid ? kGridBlocks : 0), kAdamThreads, 0, st>>>(M, lr, n, rows);
     return cudaGetLastError();
 }
 

@@ -101,7 +101,23 @@ struct MlpDev {
     uint32_t *enc;
     uint32_t enc_cap;
     uint32_t encoding;        // kEncHashGrid or kEncFreq12 (no grid: enc null, grid untouched)
+    uint32_t *step;           // Adam steps so far
+    const float2 *bias;       // per step (the last entry for all later ones): 1 - 0.9^step, 1 - 0.99^step
 };
+constexpr int kAdamSteps = 2560;  // entries of bias: 1 - 0.99^2560 rounds to 1
+
+// A training batch whose size the device knows: rows `first` onwards of the
+// min(*count, cap) records there are (null count: the size the host gave).
+struct TrainRows {
+    const uint32_t *count;
+    uint32_t cap, first;
+};
+__device__ __forceinline__ uint32_t rows_of(uint32_t n, const TrainRows &t)
+{
+    if (!t.count) return n;
+    const uint32_t have = min(*t.count, t.cap);
+    return have > t.first ? min(n, have - t.first) : 0u;
+}
 
 // N_l of every level (host).
 void grid_resolution(uint32_t (&res)[kGridLevels]);
@@ -254,11 +270,19 @@ cudaError_t mlp_infer_tc(const MlpDev &M, const float *raw, uint32_t n, float *o
 // (mlp_train_tc.cu).
 cudaError_t mlp_grads(const MlpDev &M, const float *raw, const float *target, uint32_t n, cudaStream_t st,
                       bool warp_mma = false);
+// One Adam step on the rows that `rows` says (at most n), with the gradients
+// cleared before (mlp_clear_grads) and left cleared; nothing when there are
+// none. raw, target: the rows from rows.first on. Never waits for the host.
+cudaError_t mlp_train_rows(const MlpDev &M, const float *raw, const float *target, uint32_t n, const TrainRows &rows,
+                           float lr, cudaStream_t st);
+cudaError_t mlp_clear_grads(const MlpDev &M, cudaStream_t st);
 // Forward with activations kept, loss and backward (tcgen05): X, H_0..H_4 and
 // dZ_0..dZ_5 into M.xcm / hcm / dzcm, the loss into M.loss.
-cudaError_t mlp_train_tc(const MlpDev &M, const float *raw, const float *target, uint32_t n, cudaStream_t st);
+cudaError_t mlp_train_tc(const MlpDev &M, const float *raw, const float *target, uint32_t n, cudaStream_t st,
+                         const TrainRows &rows = TrainRows{nullptr, 0u, 0u});
 // dW_l += H_{l-1}^T dZ_l for every layer from the column-major activations (tcgen05).
-cudaError_t mlp_dw_tc(const MlpDev &M, uint32_t n_pad, cudaStream_t st);
-cudaError_t mlp_adam(const MlpDev &M, uint32_t step, float lr, cudaStream_t st);
+cudaError_t mlp_dw_tc(const MlpDev &M, uint32_t n_pad, cudaStream_t st,
+                      const TrainRows &rows = TrainRows{nullptr, 0u, 0u});
+cudaError_t mlp_adam(const MlpDev &M, float lr, cudaStream_t st);
 
 }  // namespace ilg

@@ -71,8 +71,11 @@ __device__ __forceinline__ void cta_sync_for_mma()
 
 __global__ void __launch_bounds__(kTrRows, 1) k_mlp_train_tc(const MlpDev M, const float *__restrict__ raw,
                                                              const float *__restrict__ target, uint32_t n,
-                                                             uint32_t n_pad)
+                                                             const TrainRows rows)
 {
+    n = rows_of(n, rows);
+    if (n == 0u) return;
+    const uint32_t n_pad = (n + 15u) / 16u * 16u;
     extern __shared__ __align__(1024) unsigned char smem[];
     unsigned char *wf_s = smem, *wb_s = smem + kTrWf, *xz_s = wb_s + kTrWb, *h_s = xz_s + kTrX;
     __shared__ __align__(8) uint64_t bar;
@@ -254,8 +257,12 @@ __global__ void __launch_bounds__(kTrRows, 1) k_mlp_train_tc(const MlpDev M, con
 constexpr uint32_t kDwTcRowsPerCta = 512;
 constexpr int kDwTcK = 64;                  // rows per MMA group
 
-__global__ void __launch_bounds__(128) k_mlp_dw_tc(const MlpDev M, uint32_t n_pad)
+__global__ void __launch_bounds__(128) k_mlp_dw_tc(const MlpDev M, uint32_t n_pad, const TrainRows rows)
 {
+    n_pad = (rows_of(n_pad, rows) + 15u) / 16u * 16u;
+    if (blockIdx.x * kDwTcRowsPerCta >= n_pad) return;
+    // counts the Adam step whose kernel comes next
+    if (rows.count && blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) *M.step += 1u;
     __shared__ __align__(1024) unsigned char a_s[128 * kDwTcK * 2];  // M = 128 features x K = 64 rows
     __shared__ __align__(1024) unsigned char b_s[64 * kDwTcK * 2];   // N (<= 64) features x K = 64 rows
     __shared__ __align__(8) uint64_t bar;
@@ -345,7 +352,8 @@ __global__ void __launch_bounds__(128) k_mlp_dw_tc(const MlpDev M, uint32_t n_pa
 
 }  // namespace
 
-cudaError_t mlp_train_tc(const MlpDev &M, const float *raw, const float *target, uint32_t n, cudaStream_t st)
+cudaError_t mlp_train_tc(const MlpDev &M, const float *raw, const float *target, uint32_t n, cudaStream_t st,
+                         const TrainRows &rows)
 {
     if (n == 0) return cudaSuccess;
     if ((uintptr_t)raw & 15u) return cudaErrorMisalignedAddress;  // rows are read as 16-byte vectors
@@ -355,18 +363,18 @@ cudaError_t mlp_train_tc(const MlpDev &M, const float *raw, const float *target,
     if (e != cudaSuccess) return e;
     const uint32_t tiles = (n + kTrRows - 1) / kTrRows;
     const uint32_t sms = (uint32_t)current_sm_count();
-    k_mlp_train_tc<<<tiles < sms ? tiles : sms, kTrRows, kTrSmem, st>>>(M, raw, target, n, n_pad);
+    k_mlp_train_tc<<<tiles < sms ? tiles : sms, kTrRows, kTrSmem, st>>>(M, raw, target, n, rows);
     return cudaGetLastError();
 }
 
-cudaError_t mlp_dw_tc(const MlpDev &M, uint32_t n_pad, cudaStream_t st)
+cudaError_t mlp_dw_tc(const MlpDev &M, uint32_t n_pad, cudaStream_t st, const TrainRows &rows)
 {
     if (n_pad == 0) return cudaSuccess;
     if (n_pad > M.cap || (n_pad & 15u) || (M.cap & 15u)) return cudaErrorInvalidValue;
     const dim3 grid((n_pad + kDwTcRowsPerCta - 1) / kDwTcRowsPerCta, kMlpLayers);
     // 6 KB of unused dynamic shared memory keep at most 7 CTAs on an SM, so
     // their 64-column TMEM allocations always fit the SM's 512 columns
-    k_mlp_dw_tc<<<grid, 128, 6 * 1024, st>>>(M, n_pad);
+    k_mlp_dw_tc<<<grid, 128, 6 * 1024, st>>>(M, n_pad, rows);
     return cudaGetLastError();
 }
 

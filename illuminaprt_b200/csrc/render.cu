@@ -1190,10 +1190,10 @@ __device__ __forceinline__ uint32_t hc_slot(unsigned long long key, uint32_t mas
     return (uint32_t)h & mask;
 }
 
-__global__ void k_hc_update(RenderDev R, uint32_t n)
+__global__ void k_hc_update(RenderDev R)
 {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
+    if (i >= min(*R.rec_count, R.rec_cap)) return;
     const float *f = R.rec_feat + (size_t)i * kMlpRaw;
     const unsigned long long key = hc_key(f) + 1ull;
     const uint32_t mask = kHashCacheCells - 1u;
@@ -1236,10 +1236,9 @@ __global__ void k_hc_query(RenderDev R, uint32_t cap)
     R.qry_out[3 * i + 2] = y.z;
 }
 
-cudaError_t hash_cache_update(const RenderDev &R, uint32_t n_rec, cudaStream_t st)
+cudaError_t hash_cache_update(const RenderDev &R, cudaStream_t st)
 {
-    if (n_rec == 0) return cudaSuccess;
-    k_hc_update<<<blocks_for(n_rec, 256), 256, 0, st>>>(R, n_rec);
+    k_hc_update<<<blocks_for(R.rec_cap, 256), 256, 0, st>>>(R);
     return cudaGetLastError();
 }
 

@@ -143,9 +143,9 @@ cudaError_t render_persistent_bytes(const RenderDev &R, uint64_t total, uint32_t
 cudaError_t render_persistent(const RenderDev &R, uint64_t total, uint32_t lights, unsigned long long *next,
                               unsigned char *pool, uint32_t *launches, cudaStream_t st);
 
-// Hash-grid radiance cache: the n_rec training records of a call (raw
-// features + targets) are added to their cells.
+// Hash-grid radiance cache: the training records of a call (raw features +
+// targets) are added to their cells.
 constexpr uint32_t kHashCacheCells = 1u << 22;
-cudaError_t hash_cache_update(const RenderDev &R, uint32_t n_rec, cudaStream_t st);
+cudaError_t hash_cache_update(const RenderDev &R, cudaStream_t st);
 
 }  // namespace ilg

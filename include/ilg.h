@@ -231,7 +231,7 @@ typedef struct ilg_render_opts {
     uint32_t max_depth;      /* RayDepth (factory default 6) */
     float epsilon;           /* reflect epsilon (factory default 1e-4) */
     uint32_t seed;           /* sample-sequence seed */
-    uint32_t paths_per_wave; /* wavefront size; 0 = automatic */
+    uint32_t paths_per_wave; /* wavefront size; 0 = automatic (small plain renders: one persistent launch) */
     float sky[3];            /* constant environment radiance; 0 = none */
     /* radiance cache (needs ilg_mlp_init): 0 = plain path tracing; k >= 1 =
      * rendering paths stop into the cache at their k-th bounce vertex, one
@@ -276,7 +276,9 @@ ILG_API int ilg_render(ilg_ctx *ctx, const ilg_camera *cam, const ilg_render_opt
  * carries a pool of paths through all their bounces (closest hit, shading, a
  * shadow ray per light, the next ray) and takes a new path, of any scene of
  * a batch, when one ends. Same paths as the wavefront (same sample sequence
- * and arithmetic): the images agree up to float summation order.
+ * and arithmetic): the images agree up to float summation order. Plain
+ * renders of at most 2^21 paths take it without the flag when no wave or
+ * block size is given.
  * Plain renders only (no cache options, ILG_RENDER_COUNT, or Direct /
  * Albedo outputs). */
 #define ILG_RENDER_PERSISTENT 0x20u
@@ -408,7 +410,8 @@ ILG_API int ilg_mlp_train_step(ilg_ctx *ctx, const float *raw, const float *targ
  * path lengths share the queues. The runner context supplies the wavefront
  * buffers and the stream; all contexts must be on its device.
  * paths_per_wave: 0 = automatic; block: threads per block of the extend,
- * shade and shadow kernels (64, 128 or 256; 0 = 128). flags: ILG_DEVICE_PTRS,
+ * shade and shadow kernels (64, 128 or 256; 0 = 128). Either one given: the
+ * wavefront, however small the batch. flags: ILG_DEVICE_PTRS,
  * ILG_RENDER_COUNT (the batch's traversal work for ilg_render_counts on the
  * runner). */
 typedef struct ilg_batch_item {
