@@ -201,9 +201,11 @@ __device__ __forceinline__ void freq_double(float &s, float &c)
     c = __fmul_rn(__fsub_rn(c, s), __fadd_rn(c, s));
     s = s2;
 }
+// x * 2^b, exactly what ldexpf gives, for small b >= 0
+__device__ __forceinline__ float times_pow2(float x, int b) { return __fmul_rn(x, (float)(1 << b)); }
 __device__ __forceinline__ void freq_band(float x, int b, float &s, float &c)
 {
-    sincospif(ldexpf(x, b & ~3), &s, &c);
+    sincospif(times_pow2(x, b & ~3), &s, &c);
     for (int k = 0; k < (b & 3); k++) freq_double(s, c);
 }
 
@@ -238,7 +240,7 @@ __device__ __forceinline__ float2 encode_pair(const float *f, int c, const MlpDe
         const int k = c - 32, axis = k >> 3, band = (k & 7) >> 1;
         const float x = axis == 0 ? f[0] : (axis == 1 ? f[1] : f[2]);
         float s, co;
-        sincospif(ldexpf(x, band), &s, &co);
+        sincospif(times_pow2(x, band), &s, &co);
         return make_float2(s, co);
     }
     if (c < 72) return sh_pair(f[3], f[4], f[5], (c - 56) >> 1);
