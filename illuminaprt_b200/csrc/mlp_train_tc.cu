@@ -1,7 +1,7 @@
 // Radiance-cache training on the 5th-generation tensor cores.
 //
-// k_mlp_train_tc: one CTA of 128 threads per SM takes 128-row tiles of the
-// batch (one row per thread, the TMEM lane of the row's accumulator) through
+// k_mlp_train_tc: one CTA of 512 threads per SM takes 128-row tiles of the
+// batch through
 //   * the forward pass: the encoded input X and the hidden activations
 //     H_0..H_4 (ReLU, rounded to BF16) stay in shared memory as K-major
 //     A tiles, every layer one tcgen05.mma group (M = 128, K = 96 or 64,
@@ -10,17 +10,25 @@
 //     in the denominator) and dL/dy, rounded to BF16 as dZ_5;
 //   * the backward pass: dH_{l-1} = dZ_l W_l^T as one MMA group per layer
 //     against the backward weight copy (W_l as N = in x K = out), masked by
-//     H_{l-1} > 0 and rounded to BF16 as dZ_{l-1}, written over the A tile
-//     it came from;
-// storing X, H_l and dZ_l column-major (rows contiguous per feature) for the
-// weight gradients.
+//     H_{l-1} > 0 and rounded to BF16 as dZ_{l-1};
+//   * the weight gradients: dW_l = H_{l-1}^T dZ_l as MMAs over the tile's
+//     128 rows with both operands read MN-major from the very tiles above (an
+//     8 x 8 core matrix with the features contiguous is K-major for the
+//     layers and MN-major for their transposes). Each layer's sum has its own
+//     TMEM columns, grows over the CTA's tiles and is added to the FP32
+//     gradient once, at the end, in 16-byte vector atomics. These MMAs go out
+//     behind the layer's own and run under its epilogue; dZ alternates between
+//     two tiles for that.
+// Only dZ_0 leaves the CTA (column-major, for the grid's gradient).
 //
-// k_mlp_dw_tc: dW_l = H_{l-1}^T dZ_l for every layer l, split over the
-// batch: a CTA owns 512 rows of one layer and accumulates, 64 rows at a
-// time, M = 128 features (the layer's 96 or 64, the rest zero) x N = 64 (16
-// for the output layer) in TMEM, both operands loaded from the column-major
-// activations, which are K-major for this product; the partial sums are
-// added atomically to the FP32 gradient.
+// Bound by a tile's serial chain: encode, eleven layers of barrier, issue,
+// MMA, wait, load, convert and store. Four threads share a row (its TMEM lane
+// can be read by the four warps of one lane quarter) to shorten every link.
+// Measured on a B200, gradients of 16,384 rows with the hash grid: 67.8 us with
+// a thread a row, weights copied through registers and the activations written
+// out for a second kernel that summed the weight gradients a K step at a time
+// (53.8 with both of those kernels pipelined but apart); 43.3 us so, of which the
+// encoding is about a third and the gradient's atomics 4.
 //
 // The arithmetic is the warp-level kernels' (mlp.cu): BF16 operands at the
 // same points, FP32 accumulation. Every mbarrier wait is bounded and raises
@@ -37,95 +45,139 @@ namespace {
 using namespace umma;
 
 constexpr int kTrRows = 128;
-constexpr uint32_t kTrTmemCols = 64;
+constexpr int kTrSplit = 4;                      // threads a row: 16 of a layer's 64 columns each
+constexpr int kTrThreads = kTrRows * kTrSplit;
+static_assert(kMlpHid == 16 * kTrSplit && kMlpIn / 8 == 3 * kTrSplit, "columns of a row's threads");
+// TMEM columns: the layers' accumulator, then dW_0..dW_4, then dW_5
+constexpr uint32_t kTrTmemCols = 512;
+__host__ __device__ constexpr uint32_t dw_col(int l) { return 64u + 64u * (uint32_t)l; }
+static_assert(dw_col(kMlpLayers - 1) + 16 <= kTrTmemCols, "TMEM columns");
 constexpr size_t kTrWf = ((kUmmaElems * 2 + 1023) / 1024) * 1024;     // forward weights
 constexpr size_t kTrWb = ((kUmmaBwdElems * 2 + 1023) / 1024) * 1024;  // backward weights
-constexpr size_t kTrX = (size_t)kTrRows * kMlpIn * 2;                 // X tile, then the dZ tiles
-constexpr size_t kTrH = (size_t)kTrRows * kMlpHid * 2;                // one hidden tile
-constexpr size_t kTrSmem = kTrWf + kTrWb + kTrX + 5 * kTrH;
+constexpr size_t kTrX = (size_t)kTrRows * kMlpIn * 2;                 // X tile
+constexpr size_t kTrH = (size_t)kTrRows * kMlpHid * 2;                // one hidden tile, one dZ tile
+constexpr size_t kTrSmem = kTrWf + kTrWb + kTrX + 7 * kTrH;
 static_assert(kTrSmem <= 227 * 1024, "shared memory of the training kernel");
 static_assert(kTrX % 1024 == 0 && kTrH % 1024 == 0, "tile alignment");
 
 // One layer's MMAs, D (TMEM, 128 x N) = A (128 x K) B^T (B: N x K), both
 // K-major tiles of 8-row x 16-byte core matrices; issued by one thread and
 // committed to `bar`.
-__device__ __forceinline__ void issue_layer(uint32_t tmem, uint32_t a_addr, uint32_t b_addr, int K, int N, uint32_t bar)
+template <int K, int N>
+__device__ __forceinline__ void issue_layer(uint32_t tmem, uint32_t a_addr, uint32_t b_addr, uint32_t bar)
 {
-    const uint32_t idesc = umma_idesc(kTrRows, N);
-    for (int s = 0; s < K / 16; s++) {
-        const uint64_t da = umma_desc(a_addr + s * 256, 128, (K / 8) * 128);
-        const uint64_t db = umma_desc(b_addr + s * 256, 128, (K / 8) * 128);
-        mma_bf16(tmem, da, db, idesc, s > 0 ? 1u : 0u);
-    }
+    const uint64_t da = umma_desc(a_addr, 128, (K / 8) * 128), db = umma_desc(b_addr, 128, (K / 8) * 128);
+#pragma unroll
+    for (int s = 0; s < K / 16; s++)  // 256 bytes on, in units of 16
+        mma_bf16(tmem, da + 16u * s, db + 16u * s, umma_idesc(kTrRows, N), s > 0 ? 1u : 0u);
     mma_commit(bar);
 }
 
-// Every thread's smem writes visible to the tensor core, then the issue.
-__device__ __forceinline__ void cta_sync_for_mma()
+// dW (TMEM, in x N) += A^T B over the tile's 128 rows: A the K-major tile of
+// a layer's input (kIn features), B the one of its dZ (kOut columns), both
+// read MN-major: 128 bytes to the next 8 features, a row of core matrices to
+// the next 8 rows. M is 128 whatever kIn: the features past it are what lies
+// behind (shared memory of this CTA) and fill lanes that nothing reads.
+template <int kIn, int kOut>
+__device__ __forceinline__ void issue_dw(uint32_t tmem, uint32_t a_addr, uint32_t b_addr, bool add)
 {
-    fence_async_smem();
-    fence_before_sync();
-    __syncthreads();
-    fence_after_sync();
+    constexpr uint32_t a_rows = (kIn / 8) * 128, b_rows = (kOut / 8) * 128;
+    constexpr uint32_t idesc = umma_idesc(128, kOut) | 1u << 15 | 1u << 16;  // A and B MN-major
+    const uint64_t da = umma_desc(a_addr, a_rows, 128), db = umma_desc(b_addr, b_rows, 128);
+#pragma unroll
+    for (int s = 0; s < kTrRows / 16; s++)
+        mma_bf16(tmem, da + s * (2 * a_rows / 16), db + s * (2 * b_rows / 16), idesc, (s > 0 || add) ? 1u : 0u);
 }
 
-__global__ void __launch_bounds__(kTrRows, 1) k_mlp_train_tc(const MlpDev M, const float *__restrict__ raw,
-                                                             const float *__restrict__ target, uint32_t n,
-                                                             const TrainRows rows)
+// `bytes` (a multiple of 16, both addresses aligned to it) from global to
+// shared memory by the copy engine, counted on `bar`.
+__device__ __forceinline__ void bulk_load(uint32_t dst, const void *src, uint32_t bytes, uint32_t bar)
+{
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst),
+                 "l"(src), "r"(bytes), "r"(bar)
+                 : "memory");
+}
+
+__global__ void __launch_bounds__(kTrThreads, 1) k_mlp_train_tc(const MlpDev M, const float *__restrict__ raw,
+                                                                const float *__restrict__ target, uint32_t n,
+                                                                const TrainRows rows)
 {
     n = rows_of(n, rows);
-    if (n == 0u) return;
-    const uint32_t n_pad = (n + 15u) / 16u * 16u;
+    if (blockIdx.x * kTrRows >= n) return;
+    // counts the Adam step whose kernel comes next
+    if (rows.count && blockIdx.x == 0 && threadIdx.x == 0) *M.step += 1u;
     extern __shared__ __align__(1024) unsigned char smem[];
-    unsigned char *wf_s = smem, *wb_s = smem + kTrWf, *xz_s = wb_s + kTrWb, *h_s = xz_s + kTrX;
-    __shared__ __align__(8) uint64_t bar;
+    unsigned char *wf_s = smem, *wb_s = smem + kTrWf, *x_s = wb_s + kTrWb, *h_s = x_s + kTrX, *dz_s = h_s + 5 * kTrH;
+    __shared__ __align__(8) uint64_t bar, wbar;
     __shared__ uint32_t tmem_base_s;
 
-    const int tid = threadIdx.x, warp = tid >> 5;
-    {
-        const uint4 *src = reinterpret_cast<const uint4 *>(M.wu);
-        uint4 *dst = reinterpret_cast<uint4 *>(wf_s);
-        for (int i = tid; i < kUmmaElems / 8; i += kTrRows) dst[i] = src[i];
-        src = reinterpret_cast<const uint4 *>(M.wv);
-        dst = reinterpret_cast<uint4 *>(wb_s);
-        for (int i = tid; i < kUmmaBwdElems / 8; i += kTrRows) dst[i] = src[i];
+    const int warp = threadIdx.x >> 5, part = threadIdx.x / kTrRows, tid = threadIdx.x % kTrRows;
+    const uint32_t bar_a = smem_u32(&bar), wbar_a = smem_u32(&wbar);
+    const uint32_t wf_a = smem_u32(wf_s), wb_a = smem_u32(wb_s), x_a = smem_u32(x_s), h_a = smem_u32(h_s);
+    const uint32_t dz_a = smem_u32(dz_s);
+    if (threadIdx.x == 0) {
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar_a) : "memory");
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(wbar_a) : "memory");
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        // the weights arrive while the first tile is encoded
+        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(wbar_a),
+                     "r"((uint32_t)(kUmmaElems + kUmmaBwdElems) * 2u)
+                     : "memory");
+        bulk_load(wf_a, M.wu, kUmmaElems * 2, wbar_a);
+        bulk_load(wb_a, M.wv, kUmmaBwdElems * 2, wbar_a);
     }
     if (warp == 0) {
+        __syncwarp();
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_base_s)),
                      "r"(kTrTmemCols)
                      : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
-    if (tid == 0) {
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&bar)) : "memory");
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    }
-    cta_sync_for_mma();
+    fence_before_sync();
+    __syncthreads();
+    fence_after_sync();
     const uint32_t tmem = tmem_base_s;
-    const uint32_t taddr = tmem + ((uint32_t)(warp * 32) << 16);
-    const uint32_t bar_a = smem_u32(&bar);
-    const uint32_t wf_a = smem_u32(wf_s), wb_a = smem_u32(wb_s), xz_a = smem_u32(xz_s), h_a = smem_u32(h_s);
+    const uint32_t taddr = tmem + ((uint32_t)((warp & 3) * 32) << 16) + 16u * part;  // this thread's 16 columns
     const size_t cap = M.cap;
     const float inv_count = 1.f / (3.f * (float)n);
     uint32_t phase = 0;
     bool ok = true;
     float loss = 0.f;
 
-    // waits for the layer's MMAs; false (and the error bit) if the wait ran out
-    auto wait_layer = [&]() {
-        const bool waited = mbar_wait(bar_a, phase);
-        if (!waited) atomicOr(M.err, kErrWait);
-        ok = __syncthreads_and(waited) != 0;
-        phase ^= 1u;
+    // Every thread's part of the A tile in place; false when a wait of any
+    // thread ran out before.
+    auto ready = [&]() {
+        fence_async_smem();
+        fence_before_sync();
+        ok = __syncthreads_and(ok) != 0;
         fence_after_sync();
         return ok;
     };
+    // waits for the layer's MMAs (a wait that runs out sets the error bit)
+    auto wait_layer = [&]() {
+        if (!mbar_wait(bar_a, phase)) {
+            atomicOr(M.err, kErrWait);
+            ok = false;
+        }
+        phase ^= 1u;
+        fence_after_sync();
+    };
+    // this thread's 16 accumulator values
+    auto load_acc = [&](float (&v)[16]) {
+        tmem_ld16(taddr, v);
+        tmem_wait_ld();
+    };
+    auto put16 = [&](unsigned char *tile, const float (&v)[16]) {
+        put_chunk(tile, tid, 2 * part, kMlpHid, v);
+        put_chunk(tile, tid, 2 * part + 1, kMlpHid, v + 8);
+    };
 
     const uint32_t n_tiles = (n + kTrRows - 1) / kTrRows;
-    for (uint32_t tile = blockIdx.x; tile < n_tiles && ok; tile += gridDim.x) {
+    for (uint32_t tile = blockIdx.x; tile < n_tiles; tile += gridDim.x) {
         const uint32_t row = tile * kTrRows + tid;
-        const bool live = row < n, keep = row < n_pad;
-        // the encoded input: A tile of layer 0, and X column-major for dW_0
+        const bool live = row < n, add = tile != blockIdx.x;
+        // the encoded input: the A tile of layer 0. Each of the row's threads takes every fourth 8-column chunk (with
+        // the hash grid: four levels and two chunks of the rest).
         {
             float f[kMlpRaw];
             const float4 *src = reinterpret_cast<const float4 *>(raw + (size_t)row * kMlpRaw);
@@ -137,8 +189,20 @@ __global__ void __launch_bounds__(kTrRows, 1) k_mlp_train_tc(const MlpDev M, con
                 f[4 * k + 2] = q.z;
                 f[4 * k + 3] = q.w;
             }
+            int c = part;
+            if (M.encoding == kEncHashGrid) {
+                float v[8];
+#pragma unroll
+                for (int e = 0; e < 8; e += 2) {  // the loads of the four levels go out together
+                    const float2 p = grid_features(M, 4 * part + e / 2, f[0], f[1], f[2]);
+                    v[e] = live ? p.x : 0.f;
+                    v[e + 1] = live ? p.y : 0.f;
+                }
+                put_chunk(x_s, tid, c, kMlpIn, v);
+                c += kTrSplit;
+            }
 #pragma unroll 1
-            for (int c = 0; c < kMlpIn / 8; c++) {
+            for (; c < kMlpIn / 8; c += kTrSplit) {
                 float v[8];
 #pragma unroll
                 for (int e = 0; e < 8; e += 2) {
@@ -146,203 +210,122 @@ __global__ void __launch_bounds__(kTrRows, 1) k_mlp_train_tc(const MlpDev M, con
                     v[e] = live ? p.x : 0.f;
                     v[e + 1] = live ? p.y : 0.f;
                 }
-                put_chunk(xz_s, tid, c, kMlpIn, v);
-                if (keep) {
-#pragma unroll
-                    for (int e = 0; e < 8; e++) M.xcm[(size_t)(8 * c + e) * cap + row] = __float2bfloat16_rn(v[e]);
-                }
+                put_chunk(x_s, tid, c, kMlpIn, v);
             }
+        }
+        if (!mbar_wait(wbar_a, 0u)) {  // the weights (a tile after the first finds them there)
+            atomicOr(M.err, kErrWait);
+            ok = false;
         }
         // forward
 #pragma unroll 1
-        for (int l = 0; l < kMlpLayers && ok; l++) {
-            cta_sync_for_mma();
-            if (tid == 0)
-                issue_layer(tmem, l == 0 ? xz_a : h_a + (uint32_t)((l - 1) * kTrH), wf_a + umma_off(l) * 2, mlp_in(l),
-                            umma_n(l), bar_a);
-            if (!wait_layer()) break;
-            if (l < kMlpLayers - 1) {
-                unsigned char *ht = h_s + (size_t)l * kTrH;
-                __nv_bfloat16 *hg = M.hcm + (size_t)l * kMlpHid * cap;
+        for (int l = 0; l < kMlpLayers - 1; l++) {
+            if (!ready()) break;
+            if (threadIdx.x == 0) {
+                if (l == 0)
+                    issue_layer<kMlpIn, kMlpHid>(tmem, x_a, wf_a, bar_a);
+                else
+                    issue_layer<kMlpHid, kMlpHid>(tmem, h_a + (uint32_t)((l - 1) * kTrH),
+                                                  wf_a + 2u * (umma_off(1) + (l - 1) * kMlpHid * kMlpHid), bar_a);
+            }
+            wait_layer();
+            float v[16];
+            load_acc(v);
 #pragma unroll
-                for (int q = 0; q < 4; q++) {
-                    float v[16];
-                    tmem_ld16(taddr + q * 16, v);
-                    tmem_wait_ld();
+            for (int e = 0; e < 16; e++) v[e] = fmaxf(v[e], 0.f);
+            put16(h_s + (size_t)l * kTrH, v);
+        }
+        // the output layer, the loss and dL/dy (mean over rows and RGB of
+        // (y - t)^2 / (y^2 + 0.01)): one thread a row
+        if (!ready()) break;
+        if (threadIdx.x == 0)
+            issue_layer<kMlpHid, umma_n(kMlpLayers - 1)>(tmem, h_a + (uint32_t)(4 * kTrH),
+                                                         wf_a + 2u * umma_off(kMlpLayers - 1), bar_a);
+        wait_layer();
+        if (part == 0) {
+            float y[16], d[16];
+            load_acc(y);
 #pragma unroll
-                    for (int e = 0; e < 16; e++) v[e] = fmaxf(v[e], 0.f);
-                    put_chunk(ht, tid, 2 * q, kMlpHid, v);
-                    put_chunk(ht, tid, 2 * q + 1, kMlpHid, v + 8);
-                    if (keep) {
+            for (int e = 0; e < 16; e++) d[e] = 0.f;
 #pragma unroll
-                        for (int e = 0; e < 16; e++) hg[(size_t)(16 * q + e) * cap + row] = __float2bfloat16_rn(v[e]);
-                    }
-                }
-            } else {
-                // loss and dL/dy (mean over rows and RGB of (y - t)^2 / (y^2 + 0.01))
-                float y[16];
-                tmem_ld16(taddr, y);
-                tmem_wait_ld();
-                float d[16];
-#pragma unroll
-                for (int e = 0; e < 16; e++) d[e] = 0.f;
-#pragma unroll
-                for (int c = 0; c < 3; c++) {
-                    if (live) {
-                        const float t = target[(size_t)row * 3 + c];
-                        const float den = y[c] * y[c] + 0.01f;
-                        const float diff = y[c] - t;
-                        loss += diff * diff / den;
-                        d[c] = 2.f * diff / den * inv_count;
-                    }
-                }
-                // dZ_5 as the A tile of the first backward layer (K = 16)
-                put_chunk(xz_s, tid, 0, 16, d);
-                put_chunk(xz_s, tid, 1, 16, d + 8);
-                if (keep) {
-                    __nv_bfloat16 *dz5 = M.dzcm + (size_t)(kMlpLayers - 1) * kMlpHid * cap;
-#pragma unroll
-                    for (int c = 0; c < kMlpOutP; c++) dz5[(size_t)c * cap + row] = __float2bfloat16_rn(d[c]);
+            for (int c = 0; c < 3; c++) {
+                if (live) {
+                    const float t = target[(size_t)row * 3 + c];
+                    const float den = y[c] * y[c] + 0.01f;
+                    const float diff = y[c] - t;
+                    loss += diff * diff / den;
+                    d[c] = 2.f * diff / den * inv_count;
                 }
             }
+            // dZ_5 as the A tile of the first backward layer (K = 16)
+            put_chunk(dz_s + kTrH, tid, 0, 16, d);
+            put_chunk(dz_s + kTrH, tid, 1, 16, d + 8);
         }
-        if (!ok) break;
-        // backward: dZ_{l-1} = (dZ_l W_l^T) * (H_{l-1} > 0)
+        // backward: dZ_{l-1} = (dZ_l W_l^T) * (H_{l-1} > 0), dZ_l in tile l & 1
 #pragma unroll 1
         for (int l = kMlpLayers - 1; l >= 1; l--) {
-            cta_sync_for_mma();
-            if (tid == 0) issue_layer(tmem, xz_a, wb_a + umma_boff(l) * 2, umma_bk(l), mlp_in(l), bar_a);
-            if (!wait_layer()) break;
-            const unsigned char *ht = h_s + (size_t)(l - 1) * kTrH;
-            __nv_bfloat16 *dzg = M.dzcm + (size_t)(l - 1) * kMlpHid * cap;
-#pragma unroll
-            for (int q = 0; q < 4; q++) {
-                float v[16];
-                tmem_ld16(taddr + q * 16, v);
-                tmem_wait_ld();
-#pragma unroll
-                for (int h = 0; h < 2; h++) {
-                    // this row's 8 activations of chunk 2q + h (the K-major tile's 16-byte row piece)
-                    const int c = 2 * q + h;
-                    const uint4 hv = *reinterpret_cast<const uint4 *>(ht + (size_t)(tid / 8) * (kMlpHid / 8) * 128 +
-                                                                      (size_t)c * 128 + (tid % 8) * 16);
-                    const uint32_t w4[4] = {hv.x, hv.y, hv.z, hv.w};
-#pragma unroll
-                    for (int e = 0; e < 4; e++) {
-                        if (!((w4[e] & 0x7fffu) != 0u && !(w4[e] & 0x8000u))) v[8 * h + 2 * e] = 0.f;
-                        if (!((w4[e] >> 16 & 0x7fffu) != 0u && !(w4[e] & 0x80000000u))) v[8 * h + 2 * e + 1] = 0.f;
-                    }
-                }
-                put_chunk(xz_s, tid, 2 * q, kMlpHid, v);
-                put_chunk(xz_s, tid, 2 * q + 1, kMlpHid, v + 8);
-                if (keep) {
-#pragma unroll
-                    for (int e = 0; e < 16; e++) dzg[(size_t)(16 * q + e) * cap + row] = __float2bfloat16_rn(v[e]);
+            if (!ready()) break;
+            if (threadIdx.x == 0) {
+                const uint32_t a = dz_a + (l & 1) * (uint32_t)kTrH, h = h_a + (uint32_t)((l - 1) * kTrH);
+                if (l == kMlpLayers - 1) {
+                    issue_layer<umma_bk(kMlpLayers - 1), kMlpHid>(tmem, a, wb_a + 2u * umma_boff(kMlpLayers - 1), bar_a);
+                    issue_dw<kMlpHid, umma_n(kMlpLayers - 1)>(tmem + dw_col(l), h, a, add);
+                } else {
+                    issue_layer<kMlpHid, kMlpHid>(tmem, a, wb_a + 2u * (uint32_t)((l - 1) * kMlpHid * kMlpHid), bar_a);
+                    issue_dw<kMlpHid, kMlpHid>(tmem + dw_col(l), h, a, add);
                 }
             }
+            wait_layer();
+            const unsigned char *ht = h_s + (size_t)(l - 1) * kTrH;
+            float v[16];
+            load_acc(v);
+#pragma unroll
+            for (int h = 0; h < 2; h++) {
+                // this row's 8 activations of chunk 2 * part + h (the K-major tile's 16-byte row piece)
+                const uint4 hv = *reinterpret_cast<const uint4 *>(ht + (size_t)(tid / 8) * (kMlpHid / 8) * 128 +
+                                                                  (size_t)(2 * part + h) * 128 + (tid % 8) * 16);
+                const uint32_t w4[4] = {hv.x, hv.y, hv.z, hv.w};
+#pragma unroll
+                for (int e = 0; e < 4; e++) {
+                    if (!((w4[e] & 0x7fffu) != 0u && !(w4[e] & 0x8000u))) v[8 * h + 2 * e] = 0.f;
+                    if (!((w4[e] >> 16 & 0x7fffu) != 0u && !(w4[e] & 0x80000000u))) v[8 * h + 2 * e + 1] = 0.f;
+                }
+            }
+            put16(dz_s + ((l - 1) & 1) * kTrH, v);
+            if (l == 1 && live && M.encoding == kEncHashGrid) {
+#pragma unroll
+                for (int e = 0; e < 16; e++) M.dzcm[(size_t)(16 * part + e) * cap + row] = __float2bfloat16_rn(v[e]);
+            }
+        }
+        if (!ready()) break;
+        if (threadIdx.x == 0) {
+            issue_dw<kMlpIn, kMlpHid>(tmem + dw_col(0), x_a, dz_a, add);
+            mma_commit(bar_a);
+        }
+        wait_layer();  // all of the tile's MMAs: its shared memory is free again
+    }
+    ok = __syncthreads_and(ok) != 0;
+    fence_after_sync();
+    if (ok) {
+        // row `tid` of each dW_l, this thread's 16 columns of it
+#pragma unroll 1
+        for (int k = 0; k < kMlpLayers; k++) {  // neighbouring CTAs begin with different layers
+            const int l = (int)((blockIdx.x + k) % kMlpLayers);
+            const int in = mlp_in(l), out = mlp_out(l);
+            if ((warp & 3) * 32 >= in || 16 * part >= out) continue;  // whole warps
+            float v[16];
+            tmem_ld16(taddr + dw_col(l), v);
+            tmem_wait_ld();
+            float *g = M.grad + mlp_off(l) + (size_t)tid * out + 16 * part;
+#pragma unroll
+            for (int e = 0; e < 16; e += 4)  // four columns in one vector atomic (sm_90 and later)
+                if (16 * part + e < out)
+                    atomicAdd(reinterpret_cast<float4 *>(g + e), make_float4(v[e], v[e + 1], v[e + 2], v[e + 3]));
         }
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) loss += __shfl_xor_sync(0xffffffffu, loss, o);
-    if ((tid & 31) == 0 && loss != 0.f) atomicAdd(M.loss, loss / (3.f * (float)n));
-    fence_before_sync();
-    __syncthreads();
-    fence_after_sync();
-    if (warp == 0)
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kTrTmemCols) : "memory");
-}
-
-// the batch rows (K) one CTA sums; measured on a B200 (16,384-row step):
-// 1024 rows 12 % slower, 256 rows 2 % slower
-constexpr uint32_t kDwTcRowsPerCta = 512;
-constexpr int kDwTcK = 64;                  // rows per MMA group
-
-__global__ void __launch_bounds__(128) k_mlp_dw_tc(const MlpDev M, uint32_t n_pad, const TrainRows rows)
-{
-    n_pad = (rows_of(n_pad, rows) + 15u) / 16u * 16u;
-    if (blockIdx.x * kDwTcRowsPerCta >= n_pad) return;
-    // counts the Adam step whose kernel comes next
-    if (rows.count && blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) *M.step += 1u;
-    __shared__ __align__(1024) unsigned char a_s[128 * kDwTcK * 2];  // M = 128 features x K = 64 rows
-    __shared__ __align__(1024) unsigned char b_s[64 * kDwTcK * 2];   // N (<= 64) features x K = 64 rows
-    __shared__ __align__(8) uint64_t bar;
-    __shared__ uint32_t tmem_base_s;
-    const int tid = threadIdx.x, warp = tid >> 5;
-    const int l = blockIdx.y;
-    const int in = mlp_in(l), out = mlp_out(l), N = umma_n(l);
-    const size_t cap = M.cap;
-    const __nv_bfloat16 *A = l == 0 ? M.xcm : M.hcm + (size_t)(l - 1) * kMlpHid * cap;
-    const __nv_bfloat16 *B = M.dzcm + (size_t)l * kMlpHid * cap;
-    // features past the layer's own stay zero in both tiles
-    for (int i = tid; i < (int)(sizeof(a_s) / 16); i += 128) reinterpret_cast<uint4 *>(a_s)[i] = make_uint4(0u, 0u, 0u, 0u);
-    for (int i = tid; i < (int)(sizeof(b_s) / 16); i += 128) reinterpret_cast<uint4 *>(b_s)[i] = make_uint4(0u, 0u, 0u, 0u);
-    if (warp == 0) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_base_s)),
-                     "r"(kTrTmemCols)
-                     : "memory");
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-    }
-    if (tid == 0) {
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&bar)) : "memory");
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    }
-    fence_before_sync();
-    __syncthreads();
-    fence_after_sync();
-    const uint32_t tmem = tmem_base_s;
-    const uint32_t bar_a = smem_u32(&bar), a_a = smem_u32(a_s), b_a = smem_u32(b_s);
-    uint32_t phase = 0;
-    bool ok = true, any = false;
-    const uint32_t k_begin = blockIdx.x * kDwTcRowsPerCta;
-    const uint32_t k_end = min(n_pad, k_begin + kDwTcRowsPerCta);
-    for (uint32_t k0 = k_begin; k0 < k_end && ok; k0 += kDwTcK) {
-        // 16-byte pieces: (feature f, 8-row group g) -> core matrix (f / 8, g), row f % 8
-        for (int u = tid; u < in * (kDwTcK / 8); u += 128) {
-            const int f = u / (kDwTcK / 8), g = u % (kDwTcK / 8);
-            const uint32_t r = k0 + 8u * g;
-            const uint4 v = r < k_end ? *reinterpret_cast<const uint4 *>(A + (size_t)f * cap + r) : make_uint4(0u, 0u, 0u, 0u);
-            *reinterpret_cast<uint4 *>(a_s + (size_t)(f / 8) * (kDwTcK / 8) * 128 + g * 128 + (f % 8) * 16) = v;
-        }
-        for (int u = tid; u < out * (kDwTcK / 8); u += 128) {
-            const int f = u / (kDwTcK / 8), g = u % (kDwTcK / 8);
-            const uint32_t r = k0 + 8u * g;
-            const uint4 v = r < k_end ? *reinterpret_cast<const uint4 *>(B + (size_t)f * cap + r) : make_uint4(0u, 0u, 0u, 0u);
-            *reinterpret_cast<uint4 *>(b_s + (size_t)(f / 8) * (kDwTcK / 8) * 128 + g * 128 + (f % 8) * 16) = v;
-        }
-        cta_sync_for_mma();
-        if (tid == 0) {
-            const uint32_t idesc = umma_idesc(128, N);
-            for (int s = 0; s < kDwTcK / 16; s++) {
-                const uint64_t da = umma_desc(a_a + s * 256, 128, (kDwTcK / 8) * 128);
-                const uint64_t db = umma_desc(b_a + s * 256, 128, (kDwTcK / 8) * 128);
-                mma_bf16(tmem, da, db, idesc, (any || s > 0) ? 1u : 0u);
-            }
-            mma_commit(bar_a);
-        }
-        const bool waited = mbar_wait(bar_a, phase);
-        if (!waited) atomicOr(M.err, kErrWait);
-        ok = __syncthreads_and(waited) != 0;
-        phase ^= 1u;
-        fence_after_sync();
-        any = true;
-    }
-    if (ok && any) {
-        // row `tid` of dW_l: feature tid, the N accumulator columns
-        const uint32_t taddr = tmem + ((uint32_t)(warp * 32) << 16);
-        float *g = M.grad + mlp_off(l);
-        for (int q = 0; q < N / 16; q++) {
-            float v[16];
-            tmem_ld16(taddr + q * 16, v);
-            tmem_wait_ld();
-            if (tid < in) {
-#pragma unroll
-                for (int e = 0; e < 16; e++) {
-                    const int o = 16 * q + e;
-                    if (o < out) atomicAdd(g + (size_t)tid * out + o, v[e]);
-                }
-            }
-        }
-    }
+    if ((threadIdx.x & 31) == 0 && loss != 0.f) atomicAdd(M.loss, loss / (3.f * (float)n));
     fence_before_sync();
     __syncthreads();
     fence_after_sync();
@@ -363,18 +346,7 @@ cudaError_t mlp_train_tc(const MlpDev &M, const float *raw, const float *target,
     if (e != cudaSuccess) return e;
     const uint32_t tiles = (n + kTrRows - 1) / kTrRows;
     const uint32_t sms = (uint32_t)current_sm_count();
-    k_mlp_train_tc<<<tiles < sms ? tiles : sms, kTrRows, kTrSmem, st>>>(M, raw, target, n, rows);
-    return cudaGetLastError();
-}
-
-cudaError_t mlp_dw_tc(const MlpDev &M, uint32_t n_pad, cudaStream_t st, const TrainRows &rows)
-{
-    if (n_pad == 0) return cudaSuccess;
-    if (n_pad > M.cap || (n_pad & 15u) || (M.cap & 15u)) return cudaErrorInvalidValue;
-    const dim3 grid((n_pad + kDwTcRowsPerCta - 1) / kDwTcRowsPerCta, kMlpLayers);
-    // 6 KB of unused dynamic shared memory keep at most 7 CTAs on an SM, so
-    // their 64-column TMEM allocations always fit the SM's 512 columns
-    k_mlp_dw_tc<<<grid, 128, 6 * 1024, st>>>(M, n_pad, rows);
+    k_mlp_train_tc<<<tiles < sms ? tiles : sms, kTrThreads, kTrSmem, st>>>(M, raw, target, n, rows);
     return cudaGetLastError();
 }
 
