@@ -35,7 +35,7 @@ sys.path.insert(0, ROOT)
 METRIC = "Mrays/s closest-hit"
 UNIT = "Mrays/s"
 WORKLOAD = "ray batch: 1,048,576-tri heightfield, 4,194,304 coherent + 4,194,304 incoherent rays, FP32"
-NODE_BYTES, TRI_BYTES, RAY_IN, HIT_OUT = 80, 48, 32, 16
+NODE_BYTES, TRI_BYTES, RAY_IN, HIT_OUT = 96, 64, 32, 16
 
 
 def load_peaks():
@@ -424,7 +424,7 @@ def ic_cpu_baseline(width=64, ic_spp=16):
 def pt_bytes_per_sample(counts, samples):
     """Algorithmic bytes per path sample from a counted render: every
     closest-hit ray reads its 32-byte ray, the node and triangle records its
-    traversal visits (80 and 48 bytes) and moves ~64 bytes of path state
+    traversal visits (96 and 64 bytes) and moves ~64 bytes of path state
     (hit, throughput, next queue entry); every shadow ray reads its 48-byte
     segment and its records and adds a 16-byte contribution."""
     cr, cn, ct, sr, sn, st = counts
