@@ -28,7 +28,8 @@
 // a thread a row, weights copied through registers and the activations written
 // out for a second kernel that summed the weight gradients a K step at a time
 // (53.8 with both of those kernels pipelined but apart); 43.3 us so, of which the
-// encoding is about a third and the gradient's atomics 4.
+// encoding was about a quarter and the weight gradient's atomics 4 (39.5 since,
+// by the grid's kernel and the clears).
 //
 // The arithmetic is the warp-level kernels' (mlp.cu): BF16 operands at the
 // same points, FP32 accumulation. Every mbarrier wait is bounded and raises
