@@ -147,12 +147,13 @@ __global__ void __launch_bounds__(kCoopThreads) k_trace_coop(const Node8 *__rest
         bool miss = true;
         float4 q0 = make_float4(0.f, 0.f, 0.f, 0.f), q1 = q0;
         uint32_t slots = 0;
+        if (visit && !(r.ng_hits & kSlotInner)) {
+            const uint2 e = stack[--r.sp];
+            r.ng_base = e.x;
+            r.ng_hits = e.y;
+        }
+        __syncwarp();  // the ray's lanes have read the entry that the first of them may write again below
         if (visit) {
-            if (!(r.ng_hits & kSlotInner)) {
-                const uint2 e = stack[--r.sp];
-                r.ng_base = e.x;
-                r.ng_hits = e.y;
-            }
             const uint32_t bit = 31u - __clz(r.ng_hits & kSlotInner);
             r.ng_hits &= ~(1u << bit);
             const uint32_t slot4 = (bit & 28u) ^ r.oct4;
