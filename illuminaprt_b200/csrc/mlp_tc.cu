@@ -248,7 +248,7 @@ __global__ void __launch_bounds__(kTcRows * kTcGroups, 1)
             } else {
                 float v[16];
                 tmem_ld16(taddr, v);
-                tmem_wait_ld();
+                tmem_wait_ld(v);
                 if (row < n) {
                     out[(size_t)row * 3] = v[0];
                     out[(size_t)row * 3 + 1] = v[1];

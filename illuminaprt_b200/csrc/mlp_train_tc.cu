@@ -166,7 +166,7 @@ __global__ void __launch_bounds__(kTrThreads, 1) k_mlp_train_tc(const MlpDev M, 
     // this thread's 16 accumulator values
     auto load_acc = [&](float (&v)[16]) {
         tmem_ld16(taddr, v);
-        tmem_wait_ld();
+        tmem_wait_ld(v);
     };
     auto put16 = [&](unsigned char *tile, const float (&v)[16]) {
         put_chunk(tile, tid, 2 * part, kMlpHid, v);
@@ -316,7 +316,7 @@ __global__ void __launch_bounds__(kTrThreads, 1) k_mlp_train_tc(const MlpDev M, 
             if ((warp & 3) * 32 >= in || 16 * part >= out) continue;  // whole warps
             float v[16];
             tmem_ld16(taddr + dw_col(l), v);
-            tmem_wait_ld();
+            tmem_wait_ld(v);
             float *g = M.grad + mlp_off(l) + (size_t)tid * out + 16 * part;
 #pragma unroll
             for (int e = 0; e < 16; e += 4)  // four columns in one vector atomic (sm_90 and later)
