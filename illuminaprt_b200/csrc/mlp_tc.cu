@@ -93,7 +93,7 @@ __global__ void __launch_bounds__(kTcRows * kTcGroups, 1)
 {
     extern __shared__ __align__(1024) unsigned char smem[];
     unsigned char *w_s = smem;  // kUmmaElems bf16
-    __shared__ __align__(8) uint64_t bar[kTcGroups];
+    __shared__ __align__(8) uint64_t bar[kTcGroups], drain[kTcGroups];
     __shared__ uint32_t tmem_base_s;
 
     if (n_dev) n = min(n, *n_dev);
@@ -115,6 +115,7 @@ __global__ void __launch_bounds__(kTcRows * kTcGroups, 1)
     }
     if (tid < kTcGroups) {
         asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&bar[tid])) : "memory");
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&drain[tid])) : "memory");
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     fence_async_smem();
@@ -258,6 +259,7 @@ __global__ void __launch_bounds__(kTcRows * kTcGroups, 1)
         }
         ok = group_and(bar_id, ok);  // after a wait that ran out the group's threads leave together
     }
+    if (!ok && lt == 0) mma_drain(smem_u32(&drain[grp]));
     fence_before_sync();
     __syncthreads();
     fence_after_sync();

@@ -109,7 +109,7 @@ __global__ void __launch_bounds__(kTrThreads, 1) k_mlp_train_tc(const MlpDev M, 
     if (rows.count && blockIdx.x == 0 && threadIdx.x == 0) *M.step += 1u;
     extern __shared__ __align__(1024) unsigned char smem[];
     unsigned char *wf_s = smem, *wb_s = smem + kTrWf, *x_s = wb_s + kTrWb, *h_s = x_s + kTrX, *dz_s = h_s + 5 * kTrH;
-    __shared__ __align__(8) uint64_t bar, wbar;
+    __shared__ __align__(8) uint64_t bar, wbar, drain;
     __shared__ uint32_t tmem_base_s;
 
     const int warp = threadIdx.x >> 5, part = threadIdx.x / kTrRows, tid = threadIdx.x % kTrRows;
@@ -119,6 +119,7 @@ __global__ void __launch_bounds__(kTrThreads, 1) k_mlp_train_tc(const MlpDev M, 
     if (threadIdx.x == 0) {
         asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar_a) : "memory");
         asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(wbar_a) : "memory");
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&drain)) : "memory");
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         // the weights arrive while the first tile is encoded
         asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(wbar_a),
@@ -323,6 +324,9 @@ __global__ void __launch_bounds__(kTrThreads, 1) k_mlp_train_tc(const MlpDev M, 
                 if (16 * part + e < out)
                     atomicAdd(reinterpret_cast<float4 *>(g + e), make_float4(v[e], v[e + 1], v[e + 2], v[e + 3]));
         }
+    } else if (threadIdx.x == 0) {
+        mbar_wait(wbar_a, 0u);  // nothing may arrive in shared memory after the block has gone
+        mma_drain(smem_u32(&drain));
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) loss += __shfl_xor_sync(0xffffffffu, loss, o);

@@ -75,6 +75,15 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity)
     return false;
 }
 
+// After a wait that ran out, before the block gives its tensor and shared
+// memory back: another bounded wait for every MMA this thread has issued.
+// `bar` is an mbarrier of its own, not used before.
+__device__ __forceinline__ void mma_drain(uint32_t bar)
+{
+    mma_commit(bar);
+    mbar_wait(bar, 0u);
+}
+
 // 16 consecutive accumulator columns of this warp's 32 TMEM lanes; not to be
 // read before the tmem_wait_ld of the same registers
 __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float (&v)[16])
