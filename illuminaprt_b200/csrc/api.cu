@@ -1187,12 +1187,14 @@ static int run_render(ilg_ctx *ctx, std::vector<SceneRec> &recs, uint32_t cap_re
     // so a call whose launch configuration equals the previous one replays
     // the instantiated graph; a different one is captured afresh.
     uint32_t launches = 0;
-    unsigned char key[sizeof(RenderDev) + sizeof(MlpDev) + 6 * sizeof(uint64_t)];
+    unsigned char key[sizeof(RenderDev) + sizeof(MlpDev) + 7 * sizeof(uint64_t)];
     {
         uint32_t lr_bits;
         memcpy(&lr_bits, &ctx->mlp_lr, 4);
-        const uint64_t extra[6] = {cap, total, block, cache_depth | (one_launch ? 0x100000000ull : 0ull),
-                                   steps | (uint64_t)train_epochs << 32, train_batch | (uint64_t)lr_bits << 32};
+        // (nl: the layout of the one-launch renderer's pool; R has it only in
+        // sh_capacity = cap * nl, which wraps at 2^30 paths a wave)
+        const uint64_t extra[7] = {cap, total, block, cache_depth | (one_launch ? 0x100000000ull : 0ull),
+                                   steps | (uint64_t)train_epochs << 32, train_batch | (uint64_t)lr_bits << 32, nl};
         memcpy(key, &R, sizeof(RenderDev));
         memcpy(key + sizeof(RenderDev), &mlp, sizeof(MlpDev));
         memcpy(key + sizeof(RenderDev) + sizeof(MlpDev), extra, sizeof(extra));
