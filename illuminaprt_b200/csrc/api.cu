@@ -1005,6 +1005,7 @@ static int prepare_scene(ilg_ctx *runner, ilg_ctx *ctx, const ilg_camera_frame &
     }
     S = SceneRec{};
     S.nodes = ctx->bb.nodes; S.tris = ctx->bb.tris; S.n_nodes = ctx->stats.n_nodes; S.n_tris = ctx->stats.n_tris;
+    S.min_dir = min_direction(ctx->max_abs);
     S.mats = ctx->mats.ptr; S.n_mats = ctx->n_mats;
     S.lights = ctx->lights.ptr; S.n_lights = ctx->n_lights;
     S.sky = make_float3(sky[0], sky[1], sky[2]);
@@ -1094,6 +1095,7 @@ static int run_render(ilg_ctx *ctx, std::vector<SceneRec> &recs, uint32_t cap_re
     // measured on a B200: persistent traversal gains 18-25 % on the 21 M- and
     // 13.8 M-triangle workloads and loses 6 % on the 16-triangle box scene
     for (auto &S : recs) R.persistent |= S.n_tris >= 4096u ? 1u : 0u;
+    for (auto &S : recs) R.min_dir = std::max(R.min_dir, S.min_dir);
     if (count) {
         CK(ctx->render_stats.reserve(6));
         CK(cudaMemsetAsync(ctx->render_stats.ptr, 0, 6 * sizeof(unsigned long long), st));

@@ -119,6 +119,14 @@ inline bool from_file(const FileNode8 &f, Node8 &n)
     return back.q[0].w == f.q[0].w && back.q[1].z == f.q[1].z && back.q[1].w == f.q[1].w;
 }
 
+// The smallest direction component that the box test divides by, for a scene
+// with coordinates up to max_abs: 1e-20, and more in scenes above 8e14 units,
+// where a quantisation step (at most 2^-5.9 max_abs) times 32768 and the
+// reciprocal (see node_misses) would pass FLT_MAX and every box be missed.
+// 2^-116 max_abs keeps that product below 2^126; a ray that it tilts is off by
+// a whole step only at distances of 2^90 steps.
+inline float min_direction(float max_abs) { return max_abs * 0x1p-116f > 1e-20f ? max_abs * 0x1p-116f : 1e-20f; }
+
 // Lower bound of the reference's triangle window, `t < 1e-5` evaluated in
 // double (IndexedTriangle.cpp:115): for a float t this is t < the smallest
 // float >= 1e-5, i.e. 0x3727C5AD.

@@ -149,7 +149,7 @@ struct ilg_ctx {
 
     ilg::SceneView view() const
     {
-        return ilg::SceneView{bb.nodes, bb.tris, stats.n_nodes, stats.n_tris};
+        return ilg::SceneView{bb.nodes, bb.tris, stats.n_nodes, stats.n_tris, ilg::min_direction(max_abs)};
     }
 
     int check_device_error()

@@ -258,7 +258,7 @@ __global__ void __launch_bounds__(256) k_extend(RenderDev R, int cur)
         const SceneRec &S = R.scenes[R.n_scenes > 1u ? R.path_scene[R.q_path[cur][i]] : 0u];
         int best;
         float bt, bu, bv;
-        trace_one<false, kStats>(S.nodes, S.tris, S.n_nodes, S.n_tris, o, d, best, bt, bu, bv, R.err, nn, nt);
+        trace_one<false, kStats>(S.nodes, S.tris, S.n_nodes, S.n_tris, R.min_dir, o, d, best, bt, bu, bv, R.err, nn, nt);
         R.hit_tri[i] = best;
         R.hit_t[i] = bt;
     }
@@ -703,7 +703,7 @@ __global__ void __launch_bounds__(256) k_shadow(RenderDev R)
         const float4 o = R.s_o[i], d = R.s_d[i];
         const SceneRec &S = R.scenes[R.n_scenes > 1u ? R.s_sid[i] : 0u];
         float bt, bu, bv;
-        trace_one<true, kStats>(S.nodes, S.tris, S.n_nodes, S.n_tris, o, d, best, bt, bu, bv, R.err, nn, nt);
+        trace_one<true, kStats>(S.nodes, S.tris, S.n_nodes, S.n_tris, R.min_dir, o, d, best, bt, bu, bv, R.err, nn, nt);
     }
     if (kStats) count_work(R, 3, live, nn, nt);
     if (live && best == -1) shadow_unoccluded(R, i);
@@ -742,8 +742,8 @@ __device__ __forceinline__ void wave_trace_dyn(const RenderDev &R, uint32_t n, u
         [&](uint32_t k, RayState &r, TraceScene &T) {
             id = k;
             if (!kOne) bind_scene(T, R.scenes[kAnyHit ? R.s_sid[id] : R.path_scene[R.q_path[cur][id]]]);
-            if (kAnyHit) ray_init(r, R.s_o[id], R.s_d[id], T.n_nodes);
-            else ray_init(r, R.q_o[cur][id], R.q_d[cur][id], T.n_nodes);
+            if (kAnyHit) ray_init(r, R.s_o[id], R.s_d[id], T.n_nodes, R.min_dir);
+            else ray_init(r, R.q_o[cur][id], R.q_d[cur][id], T.n_nodes, R.min_dir);
         },
         [&](const RayState &r) {
             if (kAnyHit) {
@@ -778,8 +778,8 @@ __global__ void __launch_bounds__(kStackColumns, 7) k_trace_mixed(RenderDev R, i
             const bool shadow = k >= n_ext;
             id = shadow ? k - n_ext : k;
             if (!kOne) bind_scene(T, R.scenes[shadow ? R.s_sid[id] : R.path_scene[R.q_path[cur][id]]]);
-            if (shadow) ray_init(r, R.s_o[id], R.s_d[id], T.n_nodes);
-            else ray_init(r, R.q_o[cur][id], R.q_d[cur][id], T.n_nodes);
+            if (shadow) ray_init(r, R.s_o[id], R.s_d[id], T.n_nodes, R.min_dir);
+            else ray_init(r, R.q_o[cur][id], R.q_d[cur][id], T.n_nodes, R.min_dir);
             r.any = shadow;
         },
         [&](const RayState &r) {
@@ -879,11 +879,11 @@ __device__ __forceinline__ void park(Parked &s, const RayState &r)
 #pragma unroll
     for (int k = 0; k < kParkedWords; k++) s.w[k][threadIdx.x] = v[k];
 }
-__device__ __forceinline__ void unpark(const Parked &s, RayState &r)
+__device__ __forceinline__ void unpark(const Parked &s, RayState &r, float min_dir)
 {
     auto u = [&](int k) { return s.w[k][threadIdx.x]; };
     auto f = [&](int k) { return __uint_as_float(s.w[k][threadIdx.x]); };
-    ray_init(r, make_float4(f(0), f(1), f(2), f(6)), make_float4(f(3), f(4), f(5), f(7)), 0u);
+    ray_init(r, make_float4(f(0), f(1), f(2), f(6)), make_float4(f(3), f(4), f(5), f(7)), 0u, min_dir);
     r.ng_base = u(8);
     r.ng_hits = u(9);
     r.tg_base = u(10);
@@ -923,7 +923,7 @@ __global__ void __launch_bounds__(kPersistThreads, kOne ? 6 : 5)
     TraceScene scene{nullptr, nullptr, 0u, 0u};
     if (kOne) bind_scene(scene, R.scenes[0]);
     RayState r;
-    ray_init(r, make_float4(0.f, 0.f, 0.f, 0.f), make_float4(0.f, 0.f, 1.f, 0.f), 0u);
+    ray_init(r, make_float4(0.f, 0.f, 0.f, 0.f), make_float4(0.f, 0.f, 1.f, 0.f), 0u, 1.f);
     ray_stop(r);
     r.any = false;
     bool has = false;
@@ -1061,7 +1061,7 @@ __global__ void __launch_bounds__(kPersistThreads, kOne ? 6 : 5)
                 __syncwarp();
                 do shade();
                 while (n_rays < want && n_wait > 0u && (n_wait >= 32u || want > 24u));
-                unpark(s_park, r);
+                unpark(s_park, r, R.min_dir);
                 if (!kOne) bind_scene(scene, R.scenes[meta & 0xffffu]);
             }
             const uint32_t rank = __popc(idle & below), take = min(want, n_rays);
@@ -1070,7 +1070,7 @@ __global__ void __launch_bounds__(kPersistThreads, kOne ? 6 : 5)
                 const float4 o = P.ray_o[at], d = P.ray_d[at];
                 meta = P.ray_m[at];
                 if (!kOne) bind_scene(scene, R.scenes[meta & 0xffffu]);
-                ray_init(r, o, d, scene.n_nodes);
+                ray_init(r, o, d, scene.n_nodes, R.min_dir);
                 r.any = (meta >> 31) != 0u;
                 if (r.any) s_shadow[threadIdx.x] = P.ray_c[at];
                 has = true;

@@ -36,6 +36,7 @@ struct SceneRec {
     const Node8 *nodes;
     const Tri *tris;
     uint32_t n_nodes, n_tris;
+    float min_dir;  // min_direction of the scene
     const Mat *mats;
     uint32_t n_mats;
     const Light *lights;
@@ -71,6 +72,7 @@ struct RenderDev {
     const SceneRec *scenes;
     uint32_t n_scenes;
     uint32_t depth_max;    // largest max_depth over the scenes
+    float min_dir;         // largest min_dir over the scenes (a scene's own would take a register a lane)
     uint32_t *path_scene;  // per path of the wave: its scene
     uint32_t *s_sid;       // per shadow segment: its scene
     // wavefront queues (ping-pong) and path state

@@ -11,7 +11,7 @@ namespace {
 
 template <bool kStats, bool kSkip = false>
 __global__ void __launch_bounds__(128) k_closest(const Node8 *__restrict__ nodes, const Tri *__restrict__ tris,
-                                                 uint32_t n_nodes_total, uint32_t n_tris_total,
+                                                 uint32_t n_nodes_total, uint32_t n_tris_total, float min_dir,
                                                  const float4 *__restrict__ ro, const float4 *__restrict__ rd,
                                                  uint32_t n, int32_t *__restrict__ prim, float *__restrict__ tout,
                                                  float *__restrict__ uout, float *__restrict__ vout,
@@ -24,7 +24,7 @@ __global__ void __launch_bounds__(128) k_closest(const Node8 *__restrict__ nodes
     int best;
     float bt, bu, bv;
     unsigned long long nn = 0, nt = 0;
-    trace_one<false, kStats, kSkip>(nodes, tris, n_nodes_total, n_tris_total, o, d, best, bt, bu, bv, err, nn, nt,
+    trace_one<false, kStats, kSkip>(nodes, tris, n_nodes_total, n_tris_total, min_dir, o, d, best, bt, bu, bv, err, nn, nt,
                                     Skip{skip_lo, skip_n});
     __stcs(prim + i, best >= 0 ? (int32_t)__ldg(&tris[best].id.x) : (best == -2 ? -2 : -1));
     __stcs(tout + i, bt);
@@ -38,7 +38,7 @@ __global__ void __launch_bounds__(128) k_closest(const Node8 *__restrict__ nodes
 
 template <bool kSkip = false>
 __global__ void __launch_bounds__(128) k_any(const Node8 *__restrict__ nodes, const Tri *__restrict__ tris,
-                                             uint32_t n_nodes_total, uint32_t n_tris_total,
+                                             uint32_t n_nodes_total, uint32_t n_tris_total, float min_dir,
                                              const float4 *__restrict__ ro, const float4 *__restrict__ rd,
                                              uint32_t n, uint8_t *__restrict__ occ, uint32_t *__restrict__ err,
                                              uint32_t skip_lo = 0, uint32_t skip_n = 0)
@@ -49,7 +49,7 @@ __global__ void __launch_bounds__(128) k_any(const Node8 *__restrict__ nodes, co
     int best;
     float bt, bu, bv;
     unsigned long long nn = 0, nt = 0;
-    trace_one<true, false, kSkip>(nodes, tris, n_nodes_total, n_tris_total, o, d, best, bt, bu, bv, err, nn, nt,
+    trace_one<true, false, kSkip>(nodes, tris, n_nodes_total, n_tris_total, min_dir, o, d, best, bt, bu, bv, err, nn, nt,
                                   Skip{skip_lo, skip_n});
     occ[i] = best >= 0 ? 1 : 0;
 }
@@ -59,7 +59,8 @@ __global__ void __launch_bounds__(128) k_any(const Node8 *__restrict__ nodes, co
 // registers): seven ran 5 % and nine, spilling, 11 % slower.
 template <bool kAnyHit, bool kWT = false>
 __global__ void __launch_bounds__(128, 8) k_trace_dyn(const Node8 *__restrict__ nodes, const Tri *__restrict__ tris,
-                                                   uint32_t n_nodes_total, uint32_t n_tris_total, const float4 *__restrict__ ro,
+                                                   uint32_t n_nodes_total, uint32_t n_tris_total, float min_dir,
+                                                   const float4 *__restrict__ ro,
                                                    const float4 *__restrict__ rd, uint32_t n,
                                                    int32_t *__restrict__ prim, float *__restrict__ tout,
                                                    float *__restrict__ uout, float *__restrict__ vout,
@@ -76,7 +77,7 @@ __global__ void __launch_bounds__(128, 8) k_trace_dyn(const Node8 *__restrict__ 
         stack, scene, n, next, err, raw,
         [&](uint32_t k, RayState &r, TraceScene &) {
             id = k;
-            ray_init<kWT>(r, __ldcs(ro + k), __ldcs(rd + k), n_nodes_total);
+            ray_init<kWT>(r, __ldcs(ro + k), __ldcs(rd + k), n_nodes_total, min_dir);
         },
         [&](const RayState &r) {
             if (kAnyHit) {
@@ -120,7 +121,8 @@ struct SmallOut {
 template <bool kAnyHit, bool kWT>
 __global__ void __launch_bounds__(kCoopThreads) k_trace_coop(const Node8 *__restrict__ nodes,
                                                              const Tri *__restrict__ tris, uint32_t n_nodes_total,
-                                                             uint32_t n_tris_total, const float4 *__restrict__ ro,
+                                                             uint32_t n_tris_total, float min_dir,
+                                                             const float4 *__restrict__ ro,
                                                              const float4 *__restrict__ rd, uint32_t n, SmallOut out,
                                                              uint32_t *__restrict__ err,
                                                              const float4 *__restrict__ raw)
@@ -136,7 +138,7 @@ __global__ void __launch_bounds__(kCoopThreads) k_trace_coop(const Node8 *__rest
     r.ng_hits = 0u;
     r.sp = 0;
     r.best = -1;
-    if (has) ray_init<kWT>(r, ro[id], rd[id], n_nodes_total);
+    if (has) ray_init<kWT>(r, ro[id], rd[id], n_nodes_total, min_dir);
     const uint32_t px = r.ix >= 0.f ? 0u : 8u, py = r.iy >= 0.f ? 0u : 8u, pz = r.iz >= 0.f ? 0u : 8u;
     // (an earlier launch's error is this call's to report too)
     if (out.host_err && id == 0 && l == 0 && *err) *out.host_err = 1u;
@@ -290,7 +292,7 @@ cudaError_t launch_coop(const SceneView &s, const float4 *raw, const float4 *ro,
                         const SmallOut &out, uint32_t *err, cudaStream_t st)
 {
     k_trace_coop<kAnyHit, kWT><<<(n + kCoopThreads / 8 - 1) / (kCoopThreads / 8), kCoopThreads, 0, st>>>(
-        s.nodes, s.tris, s.n_nodes, s.n_tris, ro, rd, n, out, err, raw);
+        s.nodes, s.tris, s.n_nodes, s.n_tris, s.min_dir, ro, rd, n, out, err, raw);
     return cudaGetLastError();
 }
 
@@ -323,7 +325,7 @@ cudaError_t launch_closest_dyn(const SceneView &s, const float4 *ro, const float
     cudaError_t e = cudaMemsetAsync(next, 0, sizeof(uint32_t), st);
     if (e != cudaSuccess) return e;
     const uint32_t blocks = std::min<uint32_t>((n + 127) / 128, (uint32_t)sm_count() * 16u);
-    k_trace_dyn<false><<<blocks, 128, 0, st>>>(s.nodes, s.tris, s.n_nodes, s.n_tris, ro, rd, n, prim, t,
+    k_trace_dyn<false><<<blocks, 128, 0, st>>>(s.nodes, s.tris, s.n_nodes, s.n_tris, s.min_dir, ro, rd, n, prim, t,
                                                u, v, nullptr, next, err);
     return cudaGetLastError();
 }
@@ -337,7 +339,7 @@ cudaError_t launch_any_dyn(const SceneView &s, const float4 *ro, const float4 *r
     cudaError_t e = cudaMemsetAsync(next, 0, sizeof(uint32_t), st);
     if (e != cudaSuccess) return e;
     const uint32_t blocks = std::min<uint32_t>((n + 127) / 128, (uint32_t)sm_count() * 16u);
-    k_trace_dyn<true><<<blocks, 128, 0, st>>>(s.nodes, s.tris, s.n_nodes, s.n_tris, ro, rd, n, nullptr,
+    k_trace_dyn<true><<<blocks, 128, 0, st>>>(s.nodes, s.tris, s.n_nodes, s.n_tris, s.min_dir, ro, rd, n, nullptr,
                                               nullptr, nullptr, nullptr, occ, next, err);
     return cudaGetLastError();
 }
@@ -352,7 +354,7 @@ cudaError_t launch_closest_wt(const SceneView &s, const float4 *raw, const float
     cudaError_t e = cudaMemsetAsync(next, 0, sizeof(uint32_t), st);
     if (e != cudaSuccess) return e;
     const uint32_t blocks = std::min<uint32_t>((n + 127) / 128, (uint32_t)sm_count() * 16u);
-    k_trace_dyn<false, true><<<blocks, 128, 0, st>>>(s.nodes, s.tris, s.n_nodes, s.n_tris, ro, rd, n,
+    k_trace_dyn<false, true><<<blocks, 128, 0, st>>>(s.nodes, s.tris, s.n_nodes, s.n_tris, s.min_dir, ro, rd, n,
                                                      prim, t, u, v, nullptr, next, err, raw);
     return cudaGetLastError();
 }
@@ -366,7 +368,7 @@ cudaError_t launch_any_wt(const SceneView &s, const float4 *raw, const float4 *r
     cudaError_t e = cudaMemsetAsync(next, 0, sizeof(uint32_t), st);
     if (e != cudaSuccess) return e;
     const uint32_t blocks = std::min<uint32_t>((n + 127) / 128, (uint32_t)sm_count() * 16u);
-    k_trace_dyn<true, true><<<blocks, 128, 0, st>>>(s.nodes, s.tris, s.n_nodes, s.n_tris, ro, rd, n,
+    k_trace_dyn<true, true><<<blocks, 128, 0, st>>>(s.nodes, s.tris, s.n_nodes, s.n_tris, s.min_dir, ro, rd, n,
                                                     nullptr, nullptr, nullptr, nullptr, occ, next, err, raw);
     return cudaGetLastError();
 }
@@ -401,9 +403,9 @@ cudaError_t launch_closest(const SceneView &s, const float4 *ro, const float4 *r
     const uint32_t T = 128;
     const uint32_t blocks = (n + T - 1) / T;
     if (stats)
-        k_closest<true><<<blocks, T, 0, st>>>(s.nodes, s.tris, s.n_nodes, s.n_tris, ro, rd, n, prim, t, u, v, err, stats);
+        k_closest<true><<<blocks, T, 0, st>>>(s.nodes, s.tris, s.n_nodes, s.n_tris, s.min_dir, ro, rd, n, prim, t, u, v, err, stats);
     else
-        k_closest<false><<<blocks, T, 0, st>>>(s.nodes, s.tris, s.n_nodes, s.n_tris, ro, rd, n, prim, t, u, v, err, nullptr);
+        k_closest<false><<<blocks, T, 0, st>>>(s.nodes, s.tris, s.n_nodes, s.n_tris, s.min_dir, ro, rd, n, prim, t, u, v, err, nullptr);
     return cudaGetLastError();
 }
 
@@ -412,7 +414,7 @@ cudaError_t launch_any(const SceneView &s, const float4 *ro, const float4 *rd, u
 {
     if (n == 0) return cudaSuccess;
     const uint32_t T = 128;
-    k_any<false><<<(n + T - 1) / T, T, 0, st>>>(s.nodes, s.tris, s.n_nodes, s.n_tris, ro, rd, n, occ, err);
+    k_any<false><<<(n + T - 1) / T, T, 0, st>>>(s.nodes, s.tris, s.n_nodes, s.n_tris, s.min_dir, ro, rd, n, occ, err);
     return cudaGetLastError();
 }
 
@@ -422,7 +424,7 @@ cudaError_t launch_closest_skip(const SceneView &s, const float4 *ro, const floa
 {
     if (n == 0) return cudaSuccess;
     const uint32_t T = 128;
-    k_closest<false, true><<<(n + T - 1) / T, T, 0, st>>>(s.nodes, s.tris, s.n_nodes, s.n_tris, ro, rd, n,
+    k_closest<false, true><<<(n + T - 1) / T, T, 0, st>>>(s.nodes, s.tris, s.n_nodes, s.n_tris, s.min_dir, ro, rd, n,
                                                           prim, t, u, v, err, nullptr, skip_lo, skip_n);
     return cudaGetLastError();
 }
@@ -432,7 +434,7 @@ cudaError_t launch_any_skip(const SceneView &s, const float4 *ro, const float4 *
 {
     if (n == 0) return cudaSuccess;
     const uint32_t T = 128;
-    k_any<true><<<(n + T - 1) / T, T, 0, st>>>(s.nodes, s.tris, s.n_nodes, s.n_tris, ro, rd, n, occ, err,
+    k_any<true><<<(n + T - 1) / T, T, 0, st>>>(s.nodes, s.tris, s.n_nodes, s.n_tris, s.min_dir, ro, rd, n, occ, err,
                                                skip_lo, skip_n);
     return cudaGetLastError();
 }

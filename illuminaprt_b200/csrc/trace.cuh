@@ -84,14 +84,13 @@ struct RayState {
 };
 
 template <bool kWT = false>
-__device__ __forceinline__ void ray_init(RayState &r, float4 o, float4 d, uint32_t n_nodes_total)
+__device__ __forceinline__ void ray_init(RayState &r, float4 o, float4 d, uint32_t n_nodes_total, float min_dir)
 {
     if (kWT) r.sh = shear_of(d.x, d.y, d.z);
-    const float kTiny = 1e-20f;
     r.ox = o.x; r.oy = o.y; r.oz = o.z; r.dx = d.x; r.dy = d.y; r.dz = d.z;
-    r.ix = __frcp_rn(fabsf(d.x) > kTiny ? d.x : copysignf(kTiny, d.x));
-    r.iy = __frcp_rn(fabsf(d.y) > kTiny ? d.y : copysignf(kTiny, d.y));
-    r.iz = __frcp_rn(fabsf(d.z) > kTiny ? d.z : copysignf(kTiny, d.z));
+    r.ix = __frcp_rn(fabsf(d.x) > min_dir ? d.x : copysignf(min_dir, d.x));
+    r.iy = __frcp_rn(fabsf(d.y) > min_dir ? d.y : copysignf(min_dir, d.y));
+    r.iz = __frcp_rn(fabsf(d.z) > min_dir ? d.z : copysignf(min_dir, d.z));
     const uint32_t oct = (d.x < 0.f ? 1u : 0u) | (d.y < 0.f ? 2u : 0u) | (d.z < 0.f ? 4u : 0u);
     r.oct4 = 4u * (7u - oct);
     r.tmin = o.w;
@@ -336,14 +335,14 @@ __device__ __forceinline__ void ray_tri(RayState &r, const Tri *__restrict__ tri
 // Whole traversal of one ray (one ray per thread).
 template <bool kAnyHit, bool kStats, bool kSkip = false>
 __device__ __forceinline__ void trace_one(const Node8 *__restrict__ nodes, const Tri *__restrict__ tris,
-                                          uint32_t n_nodes_total, uint32_t n_tris_total,
+                                          uint32_t n_nodes_total, uint32_t n_tris_total, float min_dir,
                                           float4 o, float4 d, int &best, float &bt, float &bu, float &bv,
                                           uint32_t *__restrict__ err, unsigned long long &n_nodes,
                                           unsigned long long &n_tris, Skip skip = Skip{0u, 0u})
 {
     uint2 stack[kMaxStack];
     RayState r;
-    ray_init(r, o, d, n_nodes_total);
+    ray_init(r, o, d, n_nodes_total, min_dir);
     const uint32_t magic = plane_magic(n_nodes_total);
     while (ray_has_nodes(r)) {
         ray_node<kStats>(r, stack, nodes, n_nodes_total, magic, err, &n_nodes);

@@ -12,6 +12,7 @@ struct SceneView {
     const Node8 *nodes;
     const Tri *tris;
     uint32_t n_nodes, n_tris;
+    float min_dir;  // min_direction of the scene
 };
 
 cudaError_t launch_closest(const SceneView &s, const float4 *ro, const float4 *rd, uint32_t n, int32_t *prim,
