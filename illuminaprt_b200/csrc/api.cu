@@ -1046,6 +1046,7 @@ static int run_render(ilg_ctx *ctx, std::vector<SceneRec> &recs, uint32_t cap_re
     cudaStream_t st = ctx->stream;
     uint64_t total = 0, pixels64 = 0;
     uint32_t pixels = 0, depth_max = 0, nl = 1;
+    bool ordered = false;  // some image has one path a pixel: the one-launch renderer repeats its bits
     for (auto &S : recs) {
         S.path_begin = total;
         S.pixel_base = pixels;
@@ -1054,6 +1055,7 @@ static int run_render(ilg_ctx *ctx, std::vector<SceneRec> &recs, uint32_t cap_re
         pixels = (uint32_t)std::min<uint64_t>(pixels64, 0xffffffffu);
         depth_max = std::max(depth_max, S.max_depth);
         nl = std::max(nl, S.n_lights);
+        ordered |= S.spp == 1u;
     }
     // shadow segments carry the pixel in 31 bits (bit 31 tags Direct)
     if (pixels64 >= 0x80000000u) return fail(ctx, ILG_EINVAL, "render: more than 2^31 pixels in one call");
@@ -1177,7 +1179,7 @@ static int run_render(ilg_ctx *ctx, std::vector<SceneRec> &recs, uint32_t cap_re
 
     if (one_launch) {
         size_t bytes = 0;
-        CK(render_persistent_bytes(R, total, nl, bytes));
+        CK(render_persistent_bytes(R, total, nl, ordered, bytes));
         const size_t had = ctx->persist_pool.cap;
         CK(ctx->persist_next.reserve(1));
         CK(ctx->persist_pool.reserve(bytes));
@@ -1195,7 +1197,8 @@ static int run_render(ilg_ctx *ctx, std::vector<SceneRec> &recs, uint32_t cap_re
         memcpy(&lr_bits, &ctx->mlp_lr, 4);
         // (nl: the layout of the one-launch renderer's pool; R has it only in
         // sh_capacity = cap * nl, which wraps at 2^30 paths a wave)
-        const uint64_t extra[7] = {cap, total, block, cache_depth | (one_launch ? 0x100000000ull : 0ull),
+        const uint64_t extra[7] = {cap, total, block,
+                                   cache_depth | (one_launch ? 0x100000000ull : 0ull) | (ordered ? 0x200000000ull : 0ull),
                                    steps | (uint64_t)train_epochs << 32, train_batch | (uint64_t)lr_bits << 32, nl};
         memcpy(key, &R, sizeof(RenderDev));
         memcpy(key + sizeof(RenderDev), &mlp, sizeof(MlpDev));
@@ -1206,7 +1209,7 @@ static int run_render(ilg_ctx *ctx, std::vector<SceneRec> &recs, uint32_t cap_re
         CK(cudaStreamBeginCapture(st, cudaStreamCaptureModeRelaxed));
         cudaError_t ce = cudaSuccess;
         if (one_launch) {
-            ce = render_persistent(R, total, nl, ctx->persist_next.ptr, ctx->persist_pool.ptr, &launches, st);
+            ce = render_persistent(R, total, nl, ordered, ctx->persist_next.ptr, ctx->persist_pool.ptr, &launches, st);
         } else {
             for (uint64_t g0 = 0; g0 < total && ce == cudaSuccess; g0 += cap) {
                 const uint32_t k = (uint32_t)std::min<uint64_t>(cap, total - g0);

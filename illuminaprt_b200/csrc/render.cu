@@ -829,10 +829,21 @@ __global__ void __launch_bounds__(kStackColumns, 7) k_shadow_dyn(RenderDev R, ui
 // same index and the images agree up to the order of the float additions into
 // each pixel. Plain renders only: no radiance cache, no Direct / Albedo
 // outputs, no work counters.
+//
+// kOrdered, for renders with one sample a pixel: a pixel then has one path, and
+// its sum the path's own order: what vertex d emits, its light samples light
+// by light, what vertex d + 1 emits. So two calls give the same bits, as a
+// wavefront does that adds to a pixel once a launch. A path is shaded when all
+// its rays are back, and adds its light samples then instead of as they
+// arrive. Measured on a B200, added as they arrive / ordered: box scene 64x64
+// at 1 sample 124 / 135 us, 512x512 281 / 327, 5.2 M-triangle field 960x540
+// 1606 / 1899; as a wavefront 227, 348 and 2303. With eight lights the waiting
+// costs more: box 256x256 561 us ordered, 362 as a wavefront.
 // ---------------------------------------------------------------------------
 constexpr int kPersistThreads = 128;
 constexpr uint32_t kPathSlots = 64;
 constexpr int kNewPath = -3;  // hit of a slot that waits for a path
+constexpr int kEndedPath = -4;  // hit of a slot whose path ended with shadow rays under way (kOrdered)
 
 // One warp's part of the pool, in device memory: the paths, then a stack of
 // rays. A shading step runs when fewer than 32 rays are left and appends at
@@ -842,11 +853,12 @@ struct WarpPool {
     uint4 *id;             // sample key (x, y), pixel, scene | depth << 16
     float4 *hit_o, *hit_d; // the finished ray: origin, t; direction, triangle
     float4 *ray_o, *ray_d, *ray_c;  // ray; shadow rays: contribution, pixel
-    uint32_t *ray_m;       // scene | slot << 16; bit 31: a shadow ray
+    uint32_t *ray_m;       // scene | slot << 16; bit 31: a shadow ray (kOrdered: | light << 24)
+    float4 *lit;           // kOrdered: the contributions of a slot's shadow rays, a light each
 };
-__host__ __device__ constexpr size_t pool_bytes(uint32_t lights)
+__host__ __device__ constexpr size_t pool_bytes(uint32_t lights, bool ordered)
 {
-    return kPathSlots * 64u + 32u * (2u + lights) * 52u;
+    return kPathSlots * 64u + 32u * (2u + lights) * 52u + (ordered ? kPathSlots * lights * 16u : 0u);
 }
 __device__ __forceinline__ WarpPool warp_pool(unsigned char *base, uint32_t lights)
 {
@@ -861,6 +873,7 @@ __device__ __forceinline__ WarpPool warp_pool(unsigned char *base, uint32_t ligh
     P.ray_d = P.ray_o + rays;
     P.ray_c = P.ray_d + rays;
     P.ray_m = reinterpret_cast<uint32_t *>(P.ray_c + rays);
+    P.lit = reinterpret_cast<float4 *>(P.ray_m + rays);
     return P;
 }
 
@@ -898,7 +911,7 @@ __device__ __forceinline__ void unpark(const Parked &s, RayState &r, float min_d
     r.any = u(19) != 0u;
 }
 
-template <bool kOne>
+template <bool kOne, bool kOrdered>
 __global__ void __launch_bounds__(kPersistThreads, kOne ? 6 : 5)
     k_render_persistent(RenderDev R, uint64_t total, unsigned long long *next, unsigned char *pool, uint32_t lights)
 {
@@ -907,15 +920,20 @@ __global__ void __launch_bounds__(kPersistThreads, kOne ? 6 : 5)
     __shared__ float4 s_shadow[kPersistThreads];               // the lane's shadow ray: contribution, pixel
     __shared__ uint8_t s_wait[kPersistThreads / 32][kPathSlots];  // slots of the paths to shade
     __shared__ Parked s_park;
+    // kOrdered: a slot's rays under way, and which of its light samples are lit
+    __shared__ uint32_t s_pending[kOrdered ? kPersistThreads / 32 : 1][kPathSlots];
+    __shared__ uint32_t s_lit[kOrdered ? kPersistThreads / 32 : 1][kPathSlots];
     uint2 lstack[kMaxStack - kShortStack];
     const SplitStack stack{sstack + threadIdx.x, lstack};
     const uint32_t lane = threadIdx.x & 31u, below = (1u << lane) - 1u, magic = plane_magic(R.n_scenes);
     uint8_t *wait = s_wait[threadIdx.x >> 5];
+    uint32_t *pending = s_pending[kOrdered ? threadIdx.x >> 5 : 0], *lit_mask = s_lit[kOrdered ? threadIdx.x >> 5 : 0];
     const WarpPool P = warp_pool(
-        pool + (size_t)(blockIdx.x * (kPersistThreads / 32) + (threadIdx.x >> 5)) * pool_bytes(lights), lights);
+        pool + (size_t)(blockIdx.x * (kPersistThreads / 32) + (threadIdx.x >> 5)) * pool_bytes(lights, kOrdered), lights);
     for (uint32_t k = lane; k < kPathSlots; k += 32u) {
         wait[k] = (uint8_t)k;
         P.hit_d[k] = make_float4(0.f, 0.f, 0.f, __int_as_float(kNewPath));
+        if (kOrdered) pending[k] = lit_mask[k] = 0u;
     }
     __syncwarp();
     uint32_t n_wait = kPathSlots, n_rays = 0;  // warp-uniform, as is exhausted
@@ -936,7 +954,7 @@ __global__ void __launch_bounds__(kPersistThreads, kOne ? 6 : 5)
             const uint32_t at = n_rays + __popc(lanes & below);
             P.ray_o[at] = o;
             P.ray_d[at] = d;
-            if (m >> 31) P.ray_c[at] = c;
+            if (!kOrdered && m >> 31) P.ray_c[at] = c;
             P.ray_m[at] = m;
         }
         n_rays += __popc(lanes);
@@ -956,6 +974,7 @@ __global__ void __launch_bounds__(kPersistThreads, kOne ? 6 : 5)
         float3 p, W = make_float3(0.f, 0.f, 1.f), U = W, V = W, wo_l = W;
         bool specular = false;
         int ti = kNewPath;
+        uint32_t rays = 0;  // kOrdered: the slot's new rays
         if (live) {
             const float4 hd = P.hit_d[slot];
             ti = __float_as_int(hd.w);
@@ -969,6 +988,14 @@ __global__ void __launch_bounds__(kPersistThreads, kOne ? 6 : 5)
                 beta = make_float3(b4.x, b4.y, b4.z);
                 const bool after_specular = b4.w != 0.f;
                 const SceneRec &S = R.scenes[sid];
+                if (kOrdered) {  // the vertex before this one
+                    for (uint32_t l = 0, lit_of = lit_mask[slot]; lit_of >> l; l++) {
+                        if (!(lit_of >> l & 1u)) continue;
+                        const float4 c = P.lit[slot * lights + l];
+                        add_pixel(R.accum, pixel, make_float3(c.x, c.y, c.z));
+                    }
+                    lit_mask[slot] = 0u;
+                }
                 float3 add = make_float3(0.f, 0.f, 0.f);
                 if (ti == -1) {
                     add = beta * S.sky;
@@ -1002,21 +1029,29 @@ __global__ void __launch_bounds__(kPersistThreads, kOne ? 6 : 5)
             float3 c = make_float3(0.f, 0.f, 0.f);
             const bool ok = lit && l < n_lights && l != light_id &&
                             light_sample(R.scenes[sid], l, key, depth, p, U, V, W, wo_l, mat, beta, so, sd, c);
-            push(ok, so, sd, make_float4(c.x, c.y, c.z, __uint_as_float(pixel)), 0x80000000u | sid);
+            const float4 cp = make_float4(c.x, c.y, c.z, __uint_as_float(pixel));
+            if (kOrdered && ok) {
+                P.lit[slot * lights + l] = cp;
+                rays++;
+            }
+            push(ok, so, sd, cp, 0x80000000u | sid | (kOrdered ? slot << 16 | l << 24 : 0u));
         }
         if (cont)
             cont = continue_path(R.scenes[sid], key, depth, mat, specular, p, W, U, V, W, wo_l, beta, no, nd);
         float flag = specular ? 1.f : 0.f;
         depth++;
         // ended paths (and slots that had none) take new ones
-        const uint32_t need = __ballot_sync(kFull, live && !cont);
+        // (kOrdered: once their last light samples are added)
+        const bool ended = live && !cont, stay = kOrdered && ended && rays != 0u;
+        if (stay) P.hit_d[slot].w = __int_as_float(kEndedPath);
+        const uint32_t need = __ballot_sync(kFull, ended && !stay);
         if (need && !exhausted) {
             unsigned long long base = 0;
             if (lane == 0u) base = atomicAdd(next, (unsigned long long)__popc(need));
             base = __shfl_sync(kFull, base, 0);
             exhausted = base + __popc(need) >= total;
             const uint64_t g = base + __popc(need & below);
-            if (live && !cont && g < total) {
+            if (ended && !stay && g < total) {
                 sid = kOne ? 0u : scene_of(R, g);
                 const SceneRec &S = R.scenes[sid];
                 first_ray(S, g, pixel, key, no, nd);
@@ -1031,6 +1066,7 @@ __global__ void __launch_bounds__(kPersistThreads, kOne ? 6 : 5)
             P.beta[slot] = make_float4(beta.x, beta.y, beta.z, flag);
             P.id[slot] = make_uint4((uint32_t)key, (uint32_t)(key >> 32), pixel, sid | depth << 16);
         }
+        if (kOrdered && live) pending[slot] = rays + (cont ? 1u : 0u);
         push(cont, no, nd, no, sid | slot << 16);
         __syncwarp();
     };
@@ -1040,16 +1076,22 @@ __global__ void __launch_bounds__(kPersistThreads, kOne ? 6 : 5)
         if (__popc(idle) >= kRefillLanes || idle == kFull) {
             // results of the finished rays
             const bool mine = (idle >> lane) & 1u, done = mine && has, closest = done && !(meta >> 31);
-            const uint32_t hits = __ballot_sync(kFull, closest);
+            const uint32_t slot = meta >> 16 & (kPathSlots - 1u);
             if (closest) {
-                const uint32_t slot = meta >> 16;
                 P.hit_o[slot] = make_float4(r.ox, r.oy, r.oz, r.tcur);
                 P.hit_d[slot] = make_float4(r.dx, r.dy, r.dz, __int_as_float(r.best));
-                wait[n_wait + __popc(hits & below)] = (uint8_t)slot;
             } else if (done && r.best == -1) {
-                const float4 c = s_shadow[threadIdx.x];
-                add_pixel(R.accum, __float_as_uint(c.w), make_float3(c.x, c.y, c.z));
+                if (kOrdered) {
+                    atomicOr(&lit_mask[slot], 1u << (meta >> 24 & 7u));
+                } else {
+                    const float4 c = s_shadow[threadIdx.x];
+                    add_pixel(R.accum, __float_as_uint(c.w), make_float3(c.x, c.y, c.z));
+                }
             }
+            // kOrdered: the last of a slot's rays to finish
+            const bool to_shade = kOrdered ? done && atomicSub(&pending[slot], 1u) == 1u : closest;
+            const uint32_t hits = __ballot_sync(kFull, to_shade);
+            if (to_shade) wait[n_wait + __popc(hits & below)] = (uint8_t)slot;
             if (mine) has = false;
             n_wait += __popc(hits);
             __syncwarp();
@@ -1072,7 +1114,7 @@ __global__ void __launch_bounds__(kPersistThreads, kOne ? 6 : 5)
                 if (!kOne) bind_scene(scene, R.scenes[meta & 0xffffu]);
                 ray_init(r, o, d, scene.n_nodes, R.min_dir);
                 r.any = (meta >> 31) != 0u;
-                if (r.any) s_shadow[threadIdx.x] = P.ray_c[at];
+                if (!kOrdered && r.any) s_shadow[threadIdx.x] = P.ray_c[at];
                 has = true;
             }
             n_rays -= take;
@@ -1322,12 +1364,19 @@ cudaError_t render_wave(const RenderDev &R, uint32_t n_paths, uint64_t wave_begi
     return cudaSuccess;
 }
 
-// Warps of the one-launch renderer on the current device, at most.
-static cudaError_t persistent_grid(uint64_t total, bool one, uint32_t &blocks)
+// The one-launch renderer's form for a render.
+using PersistentKernel = void (*)(RenderDev, uint64_t, unsigned long long *, unsigned char *, uint32_t);
+static PersistentKernel persistent_kernel(bool one, bool ordered)
+{
+    if (ordered) return one ? k_render_persistent<true, true> : k_render_persistent<false, true>;
+    return one ? k_render_persistent<true, false> : k_render_persistent<false, false>;
+}
+
+// Its blocks on the current device, at most.
+static cudaError_t persistent_grid(uint64_t total, PersistentKernel kernel, uint32_t &blocks)
 {
     int per_sm = 0;
-    cudaError_t e = one ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_render_persistent<true>, kPersistThreads, 0)
-                        : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_render_persistent<false>, kPersistThreads, 0);
+    const cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kPersistThreads, 0);
     if (e != cudaSuccess) return e;
     // small renders: a path a lane rather than two, on more SMs
     const uint64_t want = (total + kPersistThreads - 1) / kPersistThreads;
@@ -1336,24 +1385,23 @@ static cudaError_t persistent_grid(uint64_t total, bool one, uint32_t &blocks)
     return cudaSuccess;
 }
 
-cudaError_t render_persistent_bytes(const RenderDev &R, uint64_t total, uint32_t lights, size_t &bytes)
+cudaError_t render_persistent_bytes(const RenderDev &R, uint64_t total, uint32_t lights, bool ordered, size_t &bytes)
 {
     uint32_t blocks = 0;
-    const cudaError_t e = persistent_grid(total, R.n_scenes == 1u, blocks);
-    bytes = (size_t)blocks * (kPersistThreads / 32) * pool_bytes(lights);
+    const cudaError_t e = persistent_grid(total, persistent_kernel(R.n_scenes == 1u, ordered), blocks);
+    bytes = (size_t)blocks * (kPersistThreads / 32) * pool_bytes(lights, ordered);
     return e;
 }
 
-cudaError_t render_persistent(const RenderDev &R, uint64_t total, uint32_t lights, unsigned long long *next,
-                              unsigned char *pool, uint32_t *launches, cudaStream_t st)
+cudaError_t render_persistent(const RenderDev &R, uint64_t total, uint32_t lights, bool ordered,
+                              unsigned long long *next, unsigned char *pool, uint32_t *launches, cudaStream_t st)
 {
     cudaError_t e = cudaMemsetAsync(next, 0, sizeof(unsigned long long), st);
     if (e != cudaSuccess) return e;
-    const bool one = R.n_scenes == 1u;
+    const PersistentKernel kernel = persistent_kernel(R.n_scenes == 1u, ordered);
     uint32_t blocks = 0;
-    if ((e = persistent_grid(total, one, blocks)) != cudaSuccess) return e;
-    (one ? k_render_persistent<true> : k_render_persistent<false>)<<<blocks, kPersistThreads, 0, st>>>(R, total, next,
-                                                                                                   pool, lights);
+    if ((e = persistent_grid(total, kernel, blocks)) != cudaSuccess) return e;
+    kernel<<<blocks, kPersistThreads, 0, st>>>(R, total, next, pool, lights);
     if (launches) *launches += 1;
     return cudaGetLastError();
 }

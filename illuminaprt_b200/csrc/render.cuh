@@ -139,11 +139,11 @@ cudaError_t render_wave(const RenderDev &R, uint32_t n_paths, uint64_t wave_begi
 cudaError_t render_resolve(const float4 *accum, uint32_t wh, float scale, float *out, cudaStream_t st);
 // Every path of the render ([0, total)) in one persistent launch
 // (k_render_persistent); `next` is a device counter, pool memory of
-// render_persistent_bytes bytes, lights the most lights of any scene. Plain
-// renders only.
-cudaError_t render_persistent_bytes(const RenderDev &R, uint64_t total, uint32_t lights, size_t &bytes);
-cudaError_t render_persistent(const RenderDev &R, uint64_t total, uint32_t lights, unsigned long long *next,
-                              unsigned char *pool, uint32_t *launches, cudaStream_t st);
+// render_persistent_bytes bytes, lights the most lights of any scene. ordered:
+// a path adds to its pixel in the path's order. Plain renders only.
+cudaError_t render_persistent_bytes(const RenderDev &R, uint64_t total, uint32_t lights, bool ordered, size_t &bytes);
+cudaError_t render_persistent(const RenderDev &R, uint64_t total, uint32_t lights, bool ordered,
+                              unsigned long long *next, unsigned char *pool, uint32_t *launches, cudaStream_t st);
 
 // Hash-grid radiance cache: the training records of a call (raw features +
 // targets) are added to their cells.

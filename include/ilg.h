@@ -276,7 +276,10 @@ ILG_API int ilg_render(ilg_ctx *ctx, const ilg_camera *cam, const ilg_render_opt
  * carries a pool of paths through all their bounces (closest hit, shading, a
  * shadow ray per light, the next ray) and takes a new path, of any scene of
  * a batch, when one ends. Same paths as the wavefront (same sample sequence
- * and arithmetic): the images agree up to float summation order. Plain
+ * and arithmetic): the images agree up to float summation order. With one
+ * sample a pixel a call repeats bit for bit (a pixel's path adds in its own
+ * order; the wavefront does with at most one light); with more, pixels may
+ * differ in the last bits from call to call, as the wavefront's do. Plain
  * renders of at most 2^21 paths take it without the flag when no wave or
  * block size is given.
  * Plain renders only (no cache options, ILG_RENDER_COUNT, or Direct /
