@@ -88,9 +88,9 @@ __device__ __forceinline__ void ray_init(RayState &r, float4 o, float4 d, uint32
 {
     if (kWT) r.sh = shear_of(d.x, d.y, d.z);
     r.ox = o.x; r.oy = o.y; r.oz = o.z; r.dx = d.x; r.dy = d.y; r.dz = d.z;
-    r.ix = __frcp_rn(fabsf(d.x) > min_dir ? d.x : copysignf(min_dir, d.x));
-    r.iy = __frcp_rn(fabsf(d.y) > min_dir ? d.y : copysignf(min_dir, d.y));
-    r.iz = __frcp_rn(fabsf(d.z) > min_dir ? d.z : copysignf(min_dir, d.z));
+    r.ix = copysignf(__frcp_rn(fmaxf(fabsf(d.x), min_dir)), d.x);
+    r.iy = copysignf(__frcp_rn(fmaxf(fabsf(d.y), min_dir)), d.y);
+    r.iz = copysignf(__frcp_rn(fmaxf(fabsf(d.z), min_dir)), d.z);
     const uint32_t oct = (d.x < 0.f ? 1u : 0u) | (d.y < 0.f ? 2u : 0u) | (d.z < 0.f ? 4u : 0u);
     r.oct4 = 4u * (7u - oct);
     r.tmin = o.w;
