@@ -1021,13 +1021,30 @@ static int prepare_scene(ilg_ctx *runner, ilg_ctx *ctx, const ilg_camera_frame &
     return ILG_OK;
 }
 
-// Plain renders of at most this many paths go in one persistent launch when
-// the caller set no wave or block size. Measured on a B200, wavefront / one
-// launch: box scene 64x64 at 1 sample 246 / 138 us, 256x256x16 (1.0 M paths)
-// 923 / 855 us, 400x400x16 (2.6 M) 1931 / 1901 us; field of 3x3 spheres 320x180
-// at 1 sample 607 / 319 us; 5.2 M-triangle field at 8.3 M paths, one call after
-// another, 15.3 / 15.4 ms.
-constexpr uint64_t kOneLaunchPaths = 1u << 21;
+// Whether a plain render whose caller set no wave or block size goes in one
+// persistent launch. A wavefront's fixed cost is some 30 to 50 us a bounce
+// (launches that a small render leaves mostly empty), so the line rises with
+// the depth; in its larger launches it traces more rays a second. Measured on a
+// B200, wavefront / one launch over 4 K to 2 M paths, depths 2 to 32, box scene
+// with 0 to 8 lights, fields of 5 K to 5.2 M triangles, batches of 2 to 16 scenes.
+// Several samples a pixel: depth 2 breaks even between 64 K and 256 K paths
+// (with eight lights nowhere: 0.89 to 1.00), depth 4 between 256 K and 1 M, depth 6
+// gains to the end of the range (2 M paths: 1.00 to 1.16), depth 12 1.05 to 1.29 there.
+// One sample (the ordered form): one light breaks even at 16 K to 64 K paths at
+// depth 2, at 256 K to 512 K at depth 6, at 2 M at depth 12; four lights at 16 K to 64 K,
+// at depth 6 and 1 M at depth 12, eight at 64 K at depth 12 and below depth 8 nowhere:
+// each light more costs about what a bounce less saves.
+bool one_launch_pays(uint64_t paths, uint64_t depth, uint64_t lights, bool ordered)
+{
+    uint64_t line;
+    if (ordered) {
+        const uint64_t d = depth + 1u > lights ? depth + 1u - lights : 0u;
+        line = 2048u * d * d * d;
+    } else {
+        line = depth > 2u || lights <= 4u ? 10240u * depth * depth * depth : 0u;
+    }
+    return paths <= std::min<uint64_t>(line, 1u << 21);
+}
 
 // Renders the scenes of `recs` (path ranges and pixel bases filled here) on
 // the runner's buffers and stream: as one persistent launch (one_launch), or
@@ -1060,7 +1077,8 @@ static int run_render(ilg_ctx *ctx, std::vector<SceneRec> &recs, uint32_t cap_re
     // shadow segments carry the pixel in 31 bits (bit 31 tags Direct)
     if (pixels64 >= 0x80000000u) return fail(ctx, ILG_EINVAL, "render: more than 2^31 pixels in one call");
     if (total_paths_out) *total_paths_out = total;
-    one_launch = one_launch || (automatic && !cache_depth && !aux && !count && total <= kOneLaunchPaths);
+    one_launch = one_launch ||
+                 (automatic && !cache_depth && !aux && !count && one_launch_pays(total, depth_max, nl, ordered));
     // wave size: whole samples for a single scene (so a wave never splits a pixel's sample)
     uint32_t cap = cap_req ? cap_req : (1u << 22);
     if (recs.size() == 1) {

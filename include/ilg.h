@@ -280,8 +280,10 @@ ILG_API int ilg_render(ilg_ctx *ctx, const ilg_camera *cam, const ilg_render_opt
  * sample a pixel a call repeats bit for bit (a pixel's path adds in its own
  * order; the wavefront does with at most one light); with more, pixels may
  * differ in the last bits from call to call, as the wavefront's do. Plain
- * renders of at most 2^21 paths take it without the flag when no wave or
- * block size is given.
+ * renders that gain by it take it without the flag when no wave or block
+ * size is given: at most 10240 depth^3 paths (depth 2: and at most four
+ * lights), with one sample a pixel 2048 (depth + 1 - lights)^3, and 2^21 in
+ * any case.
  * Plain renders only (no cache options, ILG_RENDER_COUNT, or Direct /
  * Albedo outputs). */
 #define ILG_RENDER_PERSISTENT 0x20u
