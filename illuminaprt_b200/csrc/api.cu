@@ -1046,6 +1046,14 @@ bool one_launch_pays(uint64_t paths, uint64_t depth, uint64_t lights, bool order
     return paths <= std::min<uint64_t>(line, 1u << 21);
 }
 
+// Up to this many training steps are launched with a cached frame, before the
+// number of its records is known; for more the host waits for the frame and
+// launches those that have records. A step without any costs 4.5 us (its
+// three kernels look and return), the wait 15 to 25: a frame of 960x540 with records
+// for one step of 4 / 8 / 16 / 64 allowed takes 790 / 809 / 852 / 1086 us with all of
+// them launched and 794 to 806 with the wait.
+constexpr uint64_t kTrainInFrame = 4u;
+
 // Renders the scenes of `recs` (path ranges and pixel bases filled here) on
 // the runner's buffers and stream: as one persistent launch (one_launch), or
 // in waves of at most `cap_req` paths (0 = automatic) with `block` threads a
@@ -1181,19 +1189,19 @@ static int run_render(ilg_ctx *ctx, std::vector<SceneRec> &recs, uint32_t cap_re
         mlp = ctx->mlp_view();
     }
     // Online training on the call's records (the next call renders with the
-    // update). The device knows how many there are: steps beyond them do
-    // nothing, and the host waits for none.
+    // update). The device knows how many there are: steps beyond `records` do
+    // nothing, and are not launched where the host knows the count.
     const uint32_t steps = hash_cache || !cache_depth ? 0u : train_steps;
-    auto train = [&]() {
+    auto train = [&](uint64_t records) {
         cudaError_t e = cudaSuccess;
         for (uint32_t ep = 0; ep < train_epochs; ep++)
-            for (uint32_t s = 0; s < steps && e == cudaSuccess; s++)
+            for (uint32_t s = 0; s < steps && (uint64_t)s * train_batch < records && e == cudaSuccess; s++)
                 e = mlp_train_rows(mlp, R.rec_feat + (size_t)s * train_batch * kMlpRaw,
                                    R.rec_tgt + (size_t)s * train_batch * 3, train_batch,
                                    TrainRows{R.rec_count, R.rec_cap, s * train_batch}, ctx->mlp_lr, st);
         return e;
     };
-    const bool train_in_graph = (uint64_t)steps * train_epochs <= 64u;
+    const bool train_in_graph = (uint64_t)steps * train_epochs <= kTrainInFrame;
 
     if (one_launch) {
         size_t bytes = 0;
@@ -1234,7 +1242,7 @@ static int run_render(ilg_ctx *ctx, std::vector<SceneRec> &recs, uint32_t cap_re
                 ce = render_wave(R, k, g0, st, &launches, cache_depth ? &mlp : nullptr, block);
             }
         }
-        if (ce == cudaSuccess && train_in_graph) ce = train();
+        if (ce == cudaSuccess && train_in_graph) ce = train(UINT64_MAX);
         cudaGraph_t graph = nullptr;
         const cudaError_t ee = cudaStreamEndCapture(st, &graph);
         if (ce == cudaSuccess) ce = ee;
@@ -1262,7 +1270,10 @@ static int run_render(ilg_ctx *ctx, std::vector<SceneRec> &recs, uint32_t cap_re
             CK(hash_cache_update(R, st));
             launches += 1;
         } else if (!train_in_graph) {
-            CK(train());
+            uint32_t records = 0;
+            CK(cudaMemcpyAsync(&records, R.rec_count, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
+            CK(cudaStreamSynchronize(st));
+            CK(train(records));
         }
         launches += steps * train_epochs * 4;
     }
