@@ -468,12 +468,15 @@ int ilg_build(ilg_ctx *ctx)
     CK(cudaEventRecord(ctx->ev0, ctx->stream));
     int rc = bvh_build(ctx->bb, ctx->pos.ptr, ctx->n_verts, ctx->idx.ptr, ctx->n_tris, ctx->stream, res, ctx->err,
                        sizeof(ctx->err));
-    if (rc) return rc;
+    if (rc) {
+        ctx->bb.release_scratch(false);
+        return rc;
+    }
     CK(cudaEventRecord(ctx->ev1, ctx->stream));
     CK(cudaEventSynchronize(ctx->ev1));
     float ms = 0.f;
     cudaEventElapsedTime(&ms, ctx->ev0, ctx->ev1);
-    ctx->bb.release_scratch();
+    ctx->bb.release_scratch(true);
     ctx->stats.n_tris = ctx->n_tris;
     ctx->stats.n_nodes = res.n_nodes;
     ctx->stats.n_leaf_tris = res.n_tris;

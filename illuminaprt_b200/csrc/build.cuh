@@ -43,6 +43,7 @@ struct BuildBuffers {
     // build made of 25 of them spent three quarters of its time in cudaMalloc
     // and cudaFree (262 K triangles: 12.0 ms, of which 3.1 ms on the device)
     DevBuf<unsigned char> scratch_b;
+    int builds = 0;  // builds of the context so far (2: more)
     // outputs (the built scene)
     DevBuf<Node8> nodes_b;
     DevBuf<Tri> tris_b;
@@ -95,11 +96,14 @@ struct BuildBuffers {
         return cudaSuccess;
     }
 
-    // After a build: scratch up to 256 MB (1.4 M triangles) stays for the
-    // context's next build, more is given back at once.
-    void release_scratch()
+    // After a build: a context that builds again and again keeps scratch of up
+    // to 256 MB (1.4 M triangles, 180 bytes each) for its next build; its first
+    // build, which may be its only one, a failed one and larger ones give it
+    // back at once.
+    void release_scratch(bool built)
     {
-        if (scratch_b.cap > ((size_t)256 << 20)) scratch_b.release();
+        if (!built || builds == 0 || scratch_b.cap > ((size_t)256 << 20)) scratch_b.release();
+        if (built && builds < 2) builds++;
     }
 
     void release_all()
