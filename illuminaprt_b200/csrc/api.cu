@@ -75,6 +75,17 @@ bool pageable(const void *p)
     return a.type == cudaMemoryTypeUnregistered;
 }
 
+// Whether p is memory that the host cannot touch.
+bool device_only(const void *p)
+{
+    cudaPointerAttributes a;
+    if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    return a.type == cudaMemoryTypeDevice;
+}
+
 // host copies of pageable queries: up to 16 parts (the calling thread and
 // the context's pool), 1 MB a part at least
 constexpr unsigned kCopyParts = 16u;
@@ -267,7 +278,11 @@ int query_host(ilg_ctx *ctx, const float *o4, const float *d4, uint32_t n, int32
                float *v, uint8_t *occ, bool wt)
 {
     const bool any = occ != nullptr;
-    if (n <= kSmallHostBatch) return query_host_small(ctx, o4, d4, n, prim, t, u, v, occ, wt);
+    // (the small route touches the arrays itself; a device array passed by
+    // mistake goes on to the copies, which refuse it)
+    if (n <= kSmallHostBatch && !device_only(o4) && !device_only(d4) &&
+        (any ? !device_only(occ) : !device_only(prim) && !device_only(t) && !device_only(u) && !device_only(v)))
+        return query_host_small(ctx, o4, d4, n, prim, t, u, v, occ, wt);
     if (n >= (1u << 16) && (pageable(o4) || pageable(d4) || (any ? pageable(occ) : pageable(prim) || pageable(t) ||
                                                                    pageable(u) || pageable(v))))
         return query_host_pageable(ctx, o4, d4, n, prim, t, u, v, occ, wt);
