@@ -247,12 +247,12 @@ __device__ __forceinline__ void shadow_unoccluded(const RenderDev &R, uint32_t i
 }
 
 template <bool kStats>
-__global__ void __launch_bounds__(256) k_extend(RenderDev R, int cur)
+__global__ void __launch_bounds__(256, 4) k_extend(RenderDev R, int cur)
 {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     const bool live = i < R.count[cur];
     if (!kStats && !live) return;
-    unsigned long long nn = 0, nt = 0;
+    uint32_t nn = 0, nt = 0;
     if (live) {
         const float4 o = R.q_o[cur][i], d = R.q_d[cur][i];
         const SceneRec &S = R.scenes[R.n_scenes > 1u ? R.path_scene[R.q_path[cur][i]] : 0u];
@@ -692,12 +692,12 @@ __global__ void k_cache_apply(RenderDev R)
 }
 
 template <bool kStats>
-__global__ void __launch_bounds__(256) k_shadow(RenderDev R)
+__global__ void __launch_bounds__(256, 4) k_shadow(RenderDev R)
 {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     const bool live = i < *R.sh_count;
     if (!kStats && !live) return;
-    unsigned long long nn = 0, nt = 0;
+    uint32_t nn = 0, nt = 0;
     int best = -2;
     if (live) {
         const float4 o = R.s_o[i], d = R.s_d[i];

@@ -9,8 +9,10 @@ namespace ilg {
 
 namespace {
 
+// One ray a thread: the excluding and the counted queries. Eight blocks an SM
+// (64 registers; 70 without the bound: 1 M excluding rays 2 to 3 % slower).
 template <bool kStats, bool kSkip = false>
-__global__ void __launch_bounds__(128) k_closest(const Node8 *__restrict__ nodes, const Tri *__restrict__ tris,
+__global__ void __launch_bounds__(128, 8) k_closest(const Node8 *__restrict__ nodes, const Tri *__restrict__ tris,
                                                  uint32_t n_nodes_total, uint32_t n_tris_total, float min_dir,
                                                  const float4 *__restrict__ ro, const float4 *__restrict__ rd,
                                                  uint32_t n, int32_t *__restrict__ prim, float *__restrict__ tout,
@@ -23,7 +25,7 @@ __global__ void __launch_bounds__(128) k_closest(const Node8 *__restrict__ nodes
     const float4 o = __ldcs(ro + i), d = __ldcs(rd + i);
     int best;
     float bt, bu, bv;
-    unsigned long long nn = 0, nt = 0;
+    uint32_t nn = 0, nt = 0;
     trace_one<false, kStats, kSkip>(nodes, tris, n_nodes_total, n_tris_total, min_dir, o, d, best, bt, bu, bv, err, nn, nt,
                                     Skip{skip_lo, skip_n});
     __stcs(prim + i, best >= 0 ? (int32_t)__ldg(&tris[best].id.x) : (best == -2 ? -2 : -1));
@@ -48,7 +50,7 @@ __global__ void __launch_bounds__(128) k_any(const Node8 *__restrict__ nodes, co
     const float4 o = __ldcs(ro + i), d = __ldcs(rd + i);
     int best;
     float bt, bu, bv;
-    unsigned long long nn = 0, nt = 0;
+    uint32_t nn = 0, nt = 0;
     trace_one<true, false, kSkip>(nodes, tris, n_nodes_total, n_tris_total, min_dir, o, d, best, bt, bu, bv, err, nn, nt,
                                   Skip{skip_lo, skip_n});
     occ[i] = best >= 0 ? 1 : 0;

@@ -235,11 +235,11 @@ __device__ __forceinline__ bool ray_has_nodes(const RayState &r) { return (r.ng_
 
 // Visits the next node in the ray's order (there is one: ray_has_nodes) and
 // queues its hit triangles behind those still to test. At most one group of
-// triangles may be pending (r.tq_hits == 0).
-template <bool kStats = false, class Stack = uint2 *>
+// triangles may be pending (r.tq_hits == 0), without kQueue none (r.tg_hits == 0).
+template <bool kStats = false, bool kQueue = true, class Stack = uint2 *>
 __device__ __forceinline__ void ray_node(RayState &r, Stack stack, const Node8 *__restrict__ nodes,
                                          uint32_t n_nodes_total, uint32_t magic, uint32_t *__restrict__ err,
-                                         unsigned long long *n_nodes = nullptr)
+                                         uint32_t *n_nodes = nullptr)
 {
     if (!(r.ng_hits & kSlotInner)) {
         const uint2 e = stack_get(stack, --r.sp);
@@ -270,7 +270,7 @@ __device__ __forceinline__ void ray_node(RayState &r, Stack stack, const Node8 *
     r.ng_base = q0.w;
     r.ng_hits = octant_order(inner & ~miss, r.oct4) | (inner >> 3);
     const uint32_t hit = ~(miss - (miss >> 3));  // bits 0..2 of a hit slot's nibble
-    if (r.tg_hits == 0u) {
+    if (!kQueue || r.tg_hits == 0u) {
         r.tg_base = q1.w;
         r.tg_slots = slots;
         r.tg_hits = hit & slots;
@@ -287,15 +287,16 @@ __device__ __forceinline__ void ray_node(RayState &r, Stack stack, const Node8 *
 // kWT selects the watertight triangle test over `raw` (three float4
 // vertices per triangle record) instead of the reference's Shirley test.
 // kMixed: closest- and any-hit rays share one instance (r.any chooses per ray).
-template <bool kAnyHit, bool kStats = false, bool kSkip = false, bool kWT = false, bool kMixed = false>
+template <bool kAnyHit, bool kStats = false, bool kSkip = false, bool kWT = false, bool kMixed = false,
+          bool kQueue = true>
 __device__ __forceinline__ void ray_tri(RayState &r, const Tri *__restrict__ tris, uint32_t n_tris_total,
-                                        uint32_t *__restrict__ err, unsigned long long *n_tris = nullptr,
+                                        uint32_t *__restrict__ err, uint32_t *n_tris = nullptr,
                                         Skip skip = Skip{0u, 0u}, const float4 *__restrict__ raw = nullptr)
 {
     const uint32_t b = r.tg_hits & (0u - r.tg_hits);
     const uint32_t ti = r.tg_base + __popc(r.tg_slots & (b - 1u));
     r.tg_hits ^= b;
-    if (r.tg_hits == 0u) {
+    if (kQueue && r.tg_hits == 0u) {
         r.tg_base = r.tq_base;
         r.tg_slots = r.tq_slots;
         r.tg_hits = r.tq_hits;
@@ -307,7 +308,6 @@ __device__ __forceinline__ void ray_tri(RayState &r, const Tri *__restrict__ tri
         ray_stop(r);
         return;
     }
-    if (kSkip && __ldg(&tris[ti].id.x) - skip.lo < skip.n) return;
     if (kStats) (*n_tris)++;
     float th, bh, gh;
     bool hit;
@@ -315,9 +315,15 @@ __device__ __forceinline__ void ray_tri(RayState &r, const Tri *__restrict__ tri
         const float4 *vp = raw + 3ull * ti;
         hit = watertight(__ldg(vp), __ldg(vp + 1), __ldg(vp + 2), r.ox, r.oy, r.oz, r.sh, r.whi, th, bh, gh);
     } else {
-        float4 ta, tb;
+        float4 ta, tb, tc, id;
         load32(&tris[ti].a, ta, tb);
-        hit = shirley(ta, tb, __ldg(&tris[ti].c), r.ox, r.oy, r.oz, r.dx, r.dy, r.dz, r.whi, th, bh, gh);
+        if (kSkip) {  // (the id's sector is the third edge's: both halves of the record are under way before it is looked at)
+            load32(&tris[ti].c, tc, id);
+            if (__float_as_uint(id.x) - skip.lo < skip.n) return;
+        } else {
+            tc = __ldg(&tris[ti].c);
+        }
+        hit = shirley(ta, tb, tc, r.ox, r.oy, r.oz, r.dx, r.dy, r.dz, r.whi, th, bh, gh);
     }
     if (hit) {
         r.best = (int)ti;
@@ -332,21 +338,23 @@ __device__ __forceinline__ void ray_tri(RayState &r, const Tri *__restrict__ tri
     }
 }
 
-// Whole traversal of one ray (one ray per thread).
+// Whole traversal of one ray (one ray per thread), a node's triangles right
+// after the node. Its counters stay below the records there are (< 2^31).
 template <bool kAnyHit, bool kStats, bool kSkip = false>
 __device__ __forceinline__ void trace_one(const Node8 *__restrict__ nodes, const Tri *__restrict__ tris,
                                           uint32_t n_nodes_total, uint32_t n_tris_total, float min_dir,
                                           float4 o, float4 d, int &best, float &bt, float &bu, float &bv,
-                                          uint32_t *__restrict__ err, unsigned long long &n_nodes,
-                                          unsigned long long &n_tris, Skip skip = Skip{0u, 0u})
+                                          uint32_t *__restrict__ err, uint32_t &n_nodes, uint32_t &n_tris,
+                                          Skip skip = Skip{0u, 0u})
 {
     uint2 stack[kMaxStack];
     RayState r;
     ray_init(r, o, d, n_nodes_total, min_dir);
     const uint32_t magic = plane_magic(n_nodes_total);
     while (ray_has_nodes(r)) {
-        ray_node<kStats>(r, stack, nodes, n_nodes_total, magic, err, &n_nodes);
-        while (r.tg_hits) ray_tri<kAnyHit, kStats, kSkip>(r, tris, n_tris_total, err, &n_tris, skip);
+        ray_node<kStats, false>(r, stack, nodes, n_nodes_total, magic, err, &n_nodes);
+        while (r.tg_hits)
+            ray_tri<kAnyHit, kStats, kSkip, false, false, false>(r, tris, n_tris_total, err, &n_tris, skip);
     }
     best = r.best;
     bt = r.best >= 0 ? r.tcur : __int_as_float(0x7f800000);
