@@ -935,7 +935,62 @@ __global__ void k_root(Work *q, int n, uint32_t *counters)
 
 inline uint32_t div_up(uint64_t a, uint32_t b) { return (uint32_t)((a + b - 1) / b); }
 
+__global__ void k_nodes_to_file(const Node8 *__restrict__ in, uint32_t n, FileNode8 *__restrict__ out)
+{
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n) out[i] = to_file(in[i]);
+}
+
+__global__ void k_nodes_from_file(const FileNode8 *__restrict__ in, uint32_t n, Node8 *__restrict__ out)
+{
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n) out[i] = from_file(in[i]);
+}
+
+__global__ void k_tris_to_file(const Tri *__restrict__ in, uint32_t n, FileTri *__restrict__ out,
+                               uint32_t *__restrict__ prim)
+{
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const Tri t = in[i];
+    out[i] = FileTri{t.a, t.b, t.c};
+    prim[i] = t.id.x;
+}
+
+__global__ void k_tris_from_file(const FileTri *__restrict__ in, const uint32_t *__restrict__ prim, uint32_t n,
+                                 Tri *__restrict__ out)
+{
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const FileTri t = in[i];
+    out[i] = Tri{t.a, t.b, t.c, make_uint4(prim[i], 0u, 0u, 0u)};
+}
+
 }  // namespace
+
+cudaError_t records_to_file(const Node8 *nodes, uint32_t n, FileNode8 *out, cudaStream_t st)
+{
+    k_nodes_to_file<<<div_up(n, 128), 128, 0, st>>>(nodes, n, out);
+    return cudaGetLastError();
+}
+
+cudaError_t records_to_file(const Tri *tris, uint32_t n, FileTri *out, uint32_t *prim, cudaStream_t st)
+{
+    k_tris_to_file<<<div_up(n, 128), 128, 0, st>>>(tris, n, out, prim);
+    return cudaGetLastError();
+}
+
+cudaError_t records_from_file(const FileNode8 *in, uint32_t n, Node8 *nodes, cudaStream_t st)
+{
+    k_nodes_from_file<<<div_up(n, 128), 128, 0, st>>>(in, n, nodes);
+    return cudaGetLastError();
+}
+
+cudaError_t records_from_file(const FileTri *in, const uint32_t *prim, uint32_t n, Tri *tris, cudaStream_t st)
+{
+    k_tris_from_file<<<div_up(n, 128), 128, 0, st>>>(in, prim, n, tris);
+    return cudaGetLastError();
+}
 
 // ---------------------------------------------------------------------------
 #define ILG_CK(call)                                                                       \

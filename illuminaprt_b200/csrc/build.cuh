@@ -121,6 +121,12 @@ struct BuildResult {
     uint32_t depth = 0;     // out
 };
 
+// Records of a built scene to those of a scene file and back, on the device.
+cudaError_t records_to_file(const Node8 *nodes, uint32_t n, FileNode8 *out, cudaStream_t st);
+cudaError_t records_to_file(const Tri *tris, uint32_t n, FileTri *out, uint32_t *prim, cudaStream_t st);
+cudaError_t records_from_file(const FileNode8 *in, uint32_t n, Node8 *nodes, cudaStream_t st);
+cudaError_t records_from_file(const FileTri *in, const uint32_t *prim, uint32_t n, Tri *tris, cudaStream_t st);
+
 // Returns 0 on success, else an ilg_status code with `err` filled in.
 int bvh_build(BuildBuffers &B, const float *d_pos, uint32_t n_verts, const uint32_t *d_idx, uint32_t n,
               cudaStream_t st, BuildResult &res, char *err, size_t err_len);

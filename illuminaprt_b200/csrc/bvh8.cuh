@@ -78,7 +78,7 @@ constexpr int kLeafMax = 2;
 constexpr uint32_t kSlotInner = 0x88888888u, kSlotTris = 0x77777777u;
 constexpr uint32_t kMetaInternal = 0x80u;  // scene file
 
-inline FileNode8 to_file(const Node8 &n)
+__host__ __device__ inline FileNode8 to_file(const Node8 &n)
 {
     FileNode8 f;
     uint32_t imask = 0, off = 0;
@@ -101,9 +101,23 @@ inline FileNode8 to_file(const Node8 &n)
     return f;
 }
 
-// False when the record is not one that to_file writes (triangle offsets that
-// do not follow from the counts, or an imask that the slots contradict).
-inline bool from_file(const FileNode8 &f, Node8 &n)
+// Whether a file's record is one that to_file writes: triangle offsets that
+// follow from the counts, an imask that agrees with the slots.
+inline bool canonical(const FileNode8 &f)
+{
+    uint32_t off = 0;
+    for (int s = 0; s < 8; s++) {
+        const uint32_t m = ((s < 4 ? f.q[1].z : f.q[1].w) >> (8 * (s & 3))) & 0xffu, count = m >> 5 & 3u;
+        const bool inner = m == kMetaInternal;
+        if (inner != ((f.q[0].w >> (24 + s) & 1u) != 0u)) return false;
+        if (inner || m == 0u) continue;
+        if (count == 0u || m != (count << 5 | off)) return false;
+        off += count;
+    }
+    return true;
+}
+
+__host__ __device__ inline Node8 from_file(const FileNode8 &f)
 {
     uint32_t slots = 0;
     for (int s = 0; s < 8; s++) {
@@ -111,12 +125,12 @@ inline bool from_file(const FileNode8 &f, Node8 &n)
         slots |= (m == kMetaInternal ? 8u : (1u << ((m >> 5) & 3u)) - 1u) << (4 * s);
     }
     const uint32_t e = f.q[0].w;
+    Node8 n;
     n.q[0] = uint4{f.q[0].x, f.q[0].y, f.q[0].z, f.q[1].x};
     n.q[1] = uint4{(e & 0xffu) << 23, (e >> 8 & 0xffu) << 23, (e >> 16 & 0xffu) << 23, f.q[1].y};
     for (int a = 0; a < 3; a++) n.q[2 + a] = f.q[2 + a];
     n.q[5] = uint4{slots, 0u, 0u, 0u};
-    const FileNode8 back = to_file(n);
-    return back.q[0].w == f.q[0].w && back.q[1].z == f.q[1].z && back.q[1].w == f.q[1].w;
+    return n;
 }
 
 // The smallest direction component that the box test divides by, for a scene
