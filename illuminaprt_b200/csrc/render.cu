@@ -746,7 +746,7 @@ __device__ __forceinline__ void wave_trace_dyn(const RenderDev &R, uint32_t n, u
     if (kOne) bind_scene(scene, R.scenes[0]);
     uint32_t id = 0;
     trace_persistent<kAnyHit, false, false, kRefillLanes>(
-        stack, scene, n, next, R.err, nullptr,
+        stack, scene, n, plane_magic(n), next, R.err, nullptr,
         [&](uint32_t k, RayState &r, TraceScene &T) {
             id = k;
             if (!kOne) bind_scene(T, R.scenes[kAnyHit ? R.s_sid[id] : R.path_scene[R.q_path[cur][id]]]);
@@ -781,7 +781,7 @@ __global__ void __launch_bounds__(kStackColumns, 7) k_trace_mixed(RenderDev R, i
     if (kOne) bind_scene(scene, R.scenes[0]);
     uint32_t id = 0;
     trace_persistent<false, false, true, kRefillLanes>(
-        stack, scene, n_ext + n_sh, next, R.err, nullptr,
+        stack, scene, n_ext + n_sh, plane_magic(n_ext), next, R.err, nullptr,
         [&](uint32_t k, RayState &r, TraceScene &T) {
             const bool shadow = k >= n_ext;
             id = shadow ? k - n_ext : k;

@@ -76,7 +76,7 @@ __global__ void __launch_bounds__(128, 8) k_trace_dyn(const Node8 *__restrict__ 
     TraceScene scene{nodes, tris, n_nodes_total, n_tris_total};
     uint32_t id = 0;
     trace_persistent<kAnyHit, kWT, false, kRefillLanesQuery>(
-        stack, scene, n, next, err, raw,
+        stack, scene, n, plane_magic(n_nodes_total), next, err, raw,
         [&](uint32_t k, RayState &r, TraceScene &) {
             id = k;
             ray_init<kWT>(r, __ldcs(ro + k), __ldcs(rd + k), n_nodes_total, min_dir);

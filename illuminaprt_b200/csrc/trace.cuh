@@ -220,8 +220,10 @@ __device__ __forceinline__ uint32_t octant_order(uint32_t x, uint32_t oct4)
     return (oct4 & 4u) ? y : x;
 }
 
-// The byte permute's constant (see node_misses); a tree has < 2^31 nodes.
-__device__ __forceinline__ uint32_t plane_magic(uint32_t n_nodes_total) { return 0x47000000u | (n_nodes_total >> 31); }
+// The byte permute's constant (see node_misses), made from a number below 2^31
+// that the compiler does not know: a tree's nodes, a render's scenes, the rays of
+// a wave's queue (their buffers of 80 bytes a ray bound them).
+__device__ __forceinline__ uint32_t plane_magic(uint32_t count) { return 0x47000000u | (count >> 31); }
 
 // Ends the ray's traversal with r.best as it stands (-2 after an error).
 __device__ __forceinline__ void ray_stop(RayState &r)
@@ -391,7 +393,8 @@ __device__ __forceinline__ void trace_one(const Node8 *__restrict__ nodes, const
 //
 // `fetch(k, r, S)` starts ray k < n in r (and its scene in S), `done(r)` takes
 // the result of the lane's ray; both run for several lanes at a time, when
-// kRefill lanes are idle. `next` is a device counter, zero at the launch.
+// kRefill lanes are idle. `next` is a device counter, zero at the launch;
+// magic: plane_magic.
 // ---------------------------------------------------------------------------
 constexpr int kTriLanes = 12;
 constexpr int kNodeLanes = 12;
@@ -405,11 +408,12 @@ struct TraceScene {
 };
 
 template <bool kAnyHit, bool kWT, bool kMixed, int kRefill, class Stack, class Fetch, class Done>
-__device__ __forceinline__ void trace_persistent(Stack stack, TraceScene &S, uint32_t n, uint32_t *__restrict__ next,
+__device__ __forceinline__ void trace_persistent(Stack stack, TraceScene &S, uint32_t n, uint32_t magic,
+                                                 uint32_t *__restrict__ next,
                                                  uint32_t *__restrict__ err, const float4 *__restrict__ raw,
                                                  Fetch fetch, Done done)
 {
-    const uint32_t lane = threadIdx.x & 31u, magic = plane_magic(n);
+    const uint32_t lane = threadIdx.x & 31u;
     bool exhausted = n == 0u;  // warp-uniform
     RayState r;
     r.ng_hits = r.tg_hits = r.tq_hits = 0u;
