@@ -1265,7 +1265,6 @@ static int run_render(ilg_ctx *ctx, std::vector<SceneRec> &recs, uint32_t cap_re
     // depends on the host between launches (queue counts stay on the device),
     // so a call whose launch configuration equals the previous one replays
     // the instantiated graph; a different one is captured afresh.
-    uint32_t launches = 0;
     unsigned char key[sizeof(RenderDev) + sizeof(MlpDev) + 7 * sizeof(uint64_t)];
     {
         uint32_t lr_bits;
@@ -1284,11 +1283,11 @@ static int run_render(ilg_ctx *ctx, std::vector<SceneRec> &recs, uint32_t cap_re
         CK(cudaStreamBeginCapture(st, cudaStreamCaptureModeRelaxed));
         cudaError_t ce = cudaSuccess;
         if (one_launch) {
-            ce = render_persistent(R, total, nl, ordered, ctx->persist_next.ptr, ctx->persist_pool.ptr, &launches, st);
+            ce = render_persistent(R, total, nl, ordered, ctx->persist_next.ptr, ctx->persist_pool.ptr, st);
         } else {
             for (uint64_t g0 = 0; g0 < total && ce == cudaSuccess; g0 += cap) {
                 const uint32_t k = (uint32_t)std::min<uint64_t>(cap, total - g0);
-                ce = render_wave(R, k, g0, st, &launches, cache_depth ? &mlp : nullptr, block);
+                ce = render_wave(R, k, g0, st, cache_depth ? &mlp : nullptr, block);
             }
         }
         if (ce == cudaSuccess && train_in_graph) ce = train(UINT64_MAX);
@@ -1302,9 +1301,6 @@ static int run_render(ilg_ctx *ctx, std::vector<SceneRec> &recs, uint32_t cap_re
             CK(ce);
         }
         ctx->graph_key.assign(key, key + sizeof(key));
-        ctx->graph_kernels = launches;
-    } else {
-        launches = ctx->graph_kernels;
     }
     if (steps && !ctx->mlp_grads_clear) {
         CK(mlp_clear_grads(mlp, st));
@@ -1317,16 +1313,13 @@ static int run_render(ilg_ctx *ctx, std::vector<SceneRec> &recs, uint32_t cap_re
         if (hash_cache) {
             CK(cudaMemsetAsync(R.hc_dropped, 0, sizeof(uint32_t), st));
             CK(hash_cache_update(R, st));
-            launches += 1;
         } else if (!train_in_graph) {
             uint32_t records = 0;
             CK(cudaMemcpyAsync(&records, R.rec_count, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
             CK(cudaStreamSynchronize(st));
             CK(train(records));
         }
-        launches += steps * train_epochs * 4;
     }
-    ctx->last_render_launches = launches;
     return ILG_OK;
 }
 
@@ -1377,7 +1370,6 @@ int render_one(ilg_ctx *ctx, const ilg_camera_frame &frame, const ilg_render_opt
         if (!outs[k]) continue;
         float *dst = dev ? outs[k] : ctx->out_dev.ptr;
         CK(render_resolve(sums[k], wh, 1.f / opts->spp, dst, st));
-        ctx->last_render_launches += 1;
         if (!dev) {
             CK(cudaMemcpyAsync(outs[k], dst, 12ull * wh, cudaMemcpyDeviceToHost, st));
             CK(cudaStreamSynchronize(st));  // out_dev is reused for the next output
@@ -1529,7 +1521,6 @@ int ilg_render_batch(ilg_ctx *runner, const ilg_batch_item *items, uint32_t n, u
             CK2(runner, cudaMemcpyAsync(items[i].out_rgb, dst, 12ull * S.wh, cudaMemcpyDeviceToHost, st));
         if (!(flags & ILG_DEVICE_PTRS)) CK2(runner, cudaStreamSynchronize(st));  // runner->out_dev is reused per item
     }
-    runner->last_render_launches += n;
     if (!(flags & ILG_DEVICE_PTRS)) return runner->check_device_error();
     return ILG_OK;
 }

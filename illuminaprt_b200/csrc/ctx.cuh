@@ -100,8 +100,6 @@ struct ilg_ctx {
     ilg::DevBuf<float4> rec_beta, qry_beta;
     uint32_t last_rec_cap = 0;      // the last cached render stored at most this many training records
     bool last_hash_update = false;  // the last cached render updated the hash-grid cache
-    float last_train_loss = 0.f;
-    uint32_t last_render_launches = 0;
     // work counters of the last render made with ILG_RENDER_COUNT
     ilg::DevBuf<unsigned long long> render_stats;
     // path counter of the one-launch renderer (ILG_RENDER_PERSISTENT)
@@ -111,7 +109,6 @@ struct ilg_ctx {
     // the last frame's instantiated CUDA graph and the launch configuration it was captured for
     cudaGraphExec_t graph_exec = nullptr;
     std::vector<unsigned char> graph_key;
-    uint32_t graph_kernels = 0;
     void drop_graph()
     {
         if (graph_exec) cudaGraphExecDestroy(graph_exec);

@@ -1293,7 +1293,7 @@ cudaError_t hash_cache_update(const RenderDev &R, cudaStream_t st)
 }
 
 cudaError_t render_wave(const RenderDev &R, uint32_t n_paths, uint64_t wave_begin, cudaStream_t st,
-                        uint32_t *launches, const MlpDev *cache, uint32_t block)
+                        const MlpDev *cache, uint32_t block)
 {
     const uint32_t T = block;
     cudaError_t e;
@@ -1306,7 +1306,6 @@ cudaError_t render_wave(const RenderDev &R, uint32_t n_paths, uint64_t wave_begi
             return e;
     }
     k_camera<<<blocks_for(n_paths, 128), 128, 0, st>>>(R, n_paths, wave_begin);  // also sets count[0]
-    uint32_t n_launch = 1;
     int cur = 0;
     // with short training tails every path has stopped by the tail vertex
     const uint32_t tail = R.cache_depth + R.train_tail;
@@ -1328,13 +1327,11 @@ cudaError_t render_wave(const RenderDev &R, uint32_t n_paths, uint64_t wave_begi
                 (one ? k_extend_dyn<true> : k_extend_dyn<false>)<<<persistent_blocks(n_paths), kStackColumns, 0, st>>>(
                     R, cur, R.count + 6);
             }
-            n_launch++;
         }
         traced = false;
         (R.cache_depth ? (one ? k_shade<true, true> : k_shade<true, false>)
                        : (one ? k_shade<false, true> : k_shade<false, false>))<<<blocks_for(n_paths, T), T, 0, st>>>(
             R, cur, depth, wave_begin);
-        n_launch++;
         if (R.cache_depth && cache && (depth == R.cache_depth || (R.train_tail && depth == tail))) {
             if (R.hc_keys)
                 k_hc_query<<<blocks_for(n_paths, 256), 256, 0, st>>>(R, R.capacity);
@@ -1342,7 +1339,6 @@ cudaError_t render_wave(const RenderDev &R, uint32_t n_paths, uint64_t wave_begi
                 return e;
             k_cache_apply<<<blocks_for(n_paths, 128), 128, 0, st>>>(R);
             if ((e = cudaMemsetAsync(R.qry_count, 0, sizeof(uint32_t), st)) != cudaSuccess) return e;
-            n_launch += 2;
         }
         if (depth < last && merge) {
             if ((e = cudaMemsetAsync(R.count + 6, 0, sizeof(uint32_t), st)) != cudaSuccess) return e;
@@ -1351,7 +1347,6 @@ cudaError_t render_wave(const RenderDev &R, uint32_t n_paths, uint64_t wave_begi
             // the queues the next k_shade appends to, now that they are consumed
             if ((e = cudaMemsetAsync(R.count + cur, 0, sizeof(uint32_t), st)) != cudaSuccess) return e;
             if ((e = cudaMemsetAsync(R.sh_count, 0, sizeof(uint32_t), st)) != cudaSuccess) return e;
-            n_launch++;
             traced = true;
         } else if (depth < last) {
             if (R.stats) {
@@ -1363,12 +1358,10 @@ cudaError_t render_wave(const RenderDev &R, uint32_t n_paths, uint64_t wave_begi
                 (one ? k_shadow_dyn<true> : k_shadow_dyn<false>)<<<persistent_blocks(R.sh_capacity), kStackColumns, 0,
                                                                    st>>>(R, R.count + 7);
             }
-            n_launch++;
         }
         if ((e = cudaGetLastError()) != cudaSuccess) return e;
         cur ^= 1;
     }
-    if (launches) *launches += n_launch;
     return cudaSuccess;
 }
 
@@ -1402,7 +1395,7 @@ cudaError_t render_persistent_bytes(const RenderDev &R, uint64_t total, uint32_t
 }
 
 cudaError_t render_persistent(const RenderDev &R, uint64_t total, uint32_t lights, bool ordered,
-                              unsigned long long *next, unsigned char *pool, uint32_t *launches, cudaStream_t st)
+                              unsigned long long *next, unsigned char *pool, cudaStream_t st)
 {
     cudaError_t e = cudaMemsetAsync(next, 0, sizeof(unsigned long long), st);
     if (e != cudaSuccess) return e;
@@ -1410,7 +1403,6 @@ cudaError_t render_persistent(const RenderDev &R, uint64_t total, uint32_t light
     uint32_t blocks = 0;
     if ((e = persistent_grid(total, kernel, blocks)) != cudaSuccess) return e;
     kernel<<<blocks, kPersistThreads, 0, st>>>(R, total, next, pool, lights);
-    if (launches) *launches += 1;
     return cudaGetLastError();
 }
 

@@ -135,7 +135,7 @@ cudaError_t triangle_areas(const float *pos, const uint32_t *idx, uint32_t first
 struct MlpDev;
 // One wave: global paths [wave_begin, wave_begin + n_paths).
 cudaError_t render_wave(const RenderDev &R, uint32_t n_paths, uint64_t wave_begin, cudaStream_t st,
-                        uint32_t *launches, const MlpDev *cache, uint32_t block = 128);
+                        const MlpDev *cache, uint32_t block = 128);
 cudaError_t render_resolve(const float4 *accum, uint32_t wh, float scale, float *out, cudaStream_t st);
 // Every path of the render ([0, total)) in one persistent launch
 // (k_render_persistent); `next` is a device counter, pool memory of
@@ -143,7 +143,7 @@ cudaError_t render_resolve(const float4 *accum, uint32_t wh, float scale, float 
 // a path adds to its pixel in the path's order. Plain renders only.
 cudaError_t render_persistent_bytes(const RenderDev &R, uint64_t total, uint32_t lights, bool ordered, size_t &bytes);
 cudaError_t render_persistent(const RenderDev &R, uint64_t total, uint32_t lights, bool ordered,
-                              unsigned long long *next, unsigned char *pool, uint32_t *launches, cudaStream_t st);
+                              unsigned long long *next, unsigned char *pool, cudaStream_t st);
 
 // Hash-grid radiance cache: the training records of a call (raw features +
 // targets) are added to their cells.
