@@ -401,9 +401,9 @@ __device__ __forceinline__ float adam_update(float w, float g, float &m, float &
     return w - lr * (m / bc.x) / (sqrtf(v / bc.y) + eps);
 }
 
-// One Adam step of the weights and, after them, the grid features (kGrid4
-// groups of four). // kClear: the gradients are left zero for the next step. Bound by the grid's
-// four arrays of 4 MB.
+// One Adam step of the weights and, behind them, of the grid features in groups
+// of four. kClear: the gradients and the loss are left zero for the next step.
+// Bound by the grid's four arrays of 4 MB.
 constexpr int kAdamThreads = 256;
 constexpr int kWeightBlocks = (kMlpParams + kAdamThreads - 1) / kAdamThreads;
 constexpr int kGridBlocks = (int)(kGridParams / 4 + kAdamThreads - 1) / kAdamThreads;
@@ -413,6 +413,7 @@ __global__ void __launch_bounds__(kAdamThreads) k_adam(MlpDev M, float lr, uint3
 {
     if (rows_of(n, rows) == 0u) return;
     const float2 bc = M.bias[min(*M.step, (uint32_t)kAdamSteps - 1u)];
+    if (kClear && blockIdx.x == 0 && threadIdx.x == 0) *M.loss = 0.f;
     if (blockIdx.x < kWeightBlocks) {
         const int i = blockIdx.x * kAdamThreads + threadIdx.x;
         if (i >= kMlpParams) return;

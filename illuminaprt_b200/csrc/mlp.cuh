@@ -291,7 +291,7 @@ cudaError_t mlp_infer_tc(const MlpDev &M, const float *raw, uint32_t n, float *o
 cudaError_t mlp_grads(const MlpDev &M, const float *raw, const float *target, uint32_t n, cudaStream_t st,
                       bool warp_mma = false);
 // One Adam step on the rows that `rows` says (at most n), with the gradients
-// cleared before (mlp_clear_grads) and left cleared; nothing when there are
+// and the loss cleared before (mlp_clear_grads) and left cleared; nothing when there are
 // none. raw, target: the rows from rows.first on. Never waits for the host.
 cudaError_t mlp_train_rows(const MlpDev &M, const float *raw, const float *target, uint32_t n, const TrainRows &rows,
                            float lr, cudaStream_t st);
