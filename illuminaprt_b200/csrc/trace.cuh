@@ -5,7 +5,7 @@
 //
 // One ray per thread. The stack holds node groups (first child node index,
 // remaining children and internal-child bits), one entry per level at most; the
-// children of a node are intersected together from one 80-byte record and
+// children of a node are intersected together from one 96-byte record and
 // visited in octant order. A hit shrinks the ray's Max exactly as the
 // reference does, so the triangle window `t > Max - 1e-5` and the result are
 // the reference's, up to which of two hits less than 1e-5 apart is visited
@@ -15,16 +15,6 @@
 #include "bvh8.cuh"
 
 namespace ilg {
-
-struct TraceOut {
-    int32_t *prim;   // closest hit: triangle index or -1
-    float *t, *u, *v;
-    uint8_t *occ;    // any hit: 0/1
-};
-
-struct TraceStats {
-    unsigned long long nodes, tris;
-};
 
 // Input triangles [lo, lo + n) that a query ignores (the reference's
 // `p_pExclude` primitive after its triangles were flattened into one range).
@@ -176,7 +166,7 @@ __device__ __forceinline__ float min3(float a, float b, float c)
 // so an undefined axis never culls). The near plane is pulled in by a factor
 // 1 - 2e-6 against rounding of large plane distances; what the offset costs
 // in rounding is below 1/128 of a quantisation step, of which every box has a
-// whole one to spare on each side.
+// whole one to spare on each side; min_direction keeps it finite.
 // `magic` is 0x47000000, as a value the compiler does not know: with the
 // constant in sight it replaces each permute by two logic operations.
 __device__ __forceinline__ uint32_t node_misses(const RayState &r, uint4 q0, uint4 q1, uint4 q2, uint4 q3, uint4 q4,
