@@ -395,7 +395,8 @@ ILG_API int ilg_mlp_get_params(ilg_ctx *ctx, float *params /* ILG_MLP_PARAMS */)
 ILG_API int ilg_mlp_set_params(ilg_ctx *ctx, const float *params);
 ILG_API int ilg_mlp_get_grid(ilg_ctx *ctx, float *grid /* ILG_MLP_GRID_PARAMS */);
 ILG_API int ilg_mlp_set_grid(ilg_ctx *ctx, const float *grid);
-/* The grid part of the gradient the last ilg_mlp_grads computed. */
+/* The grid part of the gradient the last ilg_mlp_grads or ilg_mlp_train_step
+ * computed, if no cached render has trained since (its steps leave it zero). */
 ILG_API int ilg_mlp_get_grid_grads(ilg_ctx *ctx, float *grad /* ILG_MLP_GRID_PARAMS */);
 /* out: n x 3 radiance. Host pointers unless ILG_DEVICE_PTRS (device query
  * rows must start 16-byte aligned). Runs on the
